@@ -29,6 +29,7 @@
 #include "chol_dev.cuh"
 #include "detmath.h"
 #include "internal.cuh"
+#include "loop_f64_kernels.cuh"
 #include "loop_simt_kernels.cuh"
 
 namespace {
@@ -184,34 +185,31 @@ __global__ void k_finalize_batch(const double *partials, const int64_t *part_off
   reps[g] = fma(0.0, 0.0, s * inv_tot);
 }
 
-template <typename T, int GEN>
-int launch_batch_loop(dbgz_ctx *ctx, const SimtParams<T> *d_params, const BatchItem *d_items, int64_t n_items,
-                      unsigned long long *d_counter, T *yws, int64_t Dp, int64_t grid) {
-  using Pol = pol::Forward<T, GEN, false>;
-  const size_t smem = sizeof(simt::SimtSmem<T>);
-  auto kern = simt::k_genz_simt_batch<T, Pol>;
-  DBGZ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), ctx->stream));
-  kern<<<(unsigned)grid, simt::NT, smem, ctx->stream>>>(d_params, d_items, n_items, d_counter, yws, Dp);
-  dbgz_count_launch(ctx);
-  DBGZ_CUDA_TRY(ctx, cudaGetLastError());
-  return DBGZ_OK;
-}
+// The persistent CUDA-core loop over the work queue: the FP64 loop
+// (loop_f64_kernels.cuh) or the FP32 SIMT loop.
+template <typename T>
+struct BatchLoop {
+  using Kern = void (*)(const SimtParams<T> *, const BatchItem *, int64_t, unsigned long long *, T *, int64_t);
+  static constexpr int kThreads = sizeof(T) == 8 ? f64::NT : simt::NT;
+  static constexpr int kSmem = (int)(sizeof(T) == 8 ? sizeof(f64::Smem) : sizeof(simt::SimtSmem<T>));
+  template <int GEN>
+  static Kern kern() {
+    using Pol = pol::Forward<T, GEN, false>;
+    if constexpr (sizeof(T) == 8)
+      return f64::k_genz_f64_batch<Pol>;
+    else
+      return simt::k_genz_simt_batch<T, Pol>;
+  }
+  static Kern pick(int gen) { return gen == DBGZ_QMC_SOBOL ? kern<DBGZ_QMC_SOBOL>() : kern<DBGZ_QMC_RICHTMYER>(); }
+};
 
 template <typename T>
 int batch_grid(dbgz_ctx *ctx, int GEN, int64_t *grid) {
-  const size_t smem = sizeof(simt::SimtSmem<T>);
+  using BL = BatchLoop<T>;
+  const typename BL::Kern k = BL::pick(GEN);
   int per_sm = 0;
-  cudaError_t e;
-  if (GEN == DBGZ_QMC_SOBOL) {
-    auto k = simt::k_genz_simt_batch<T, pol::Forward<T, DBGZ_QMC_SOBOL, false>>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, simt::NT, smem);
-  } else {
-    auto k = simt::k_genz_simt_batch<T, pol::Forward<T, DBGZ_QMC_RICHTMYER, false>>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, simt::NT, smem);
-  }
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, BL::kSmem);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, BL::kThreads, BL::kSmem);
   if (e != cudaSuccess || per_sm < 1) return dbgz_fail(ctx, DBGZ_ERR_CUDA, "pnorm_batch: loop kernel does not fit");
   *grid = (int64_t)per_sm * ctx->num_sms;
   return DBGZ_OK;
@@ -524,11 +522,9 @@ int plan_enqueue(dbgz_batch_plan *P, const double *Sigma, const double *a, const
     launches += 2;
   }
   if (P->n_items) {
-    using PolS = pol::Forward<T, DBGZ_QMC_SOBOL, false>;
-    using PolR = pol::Forward<T, DBGZ_QMC_RICHTMYER, false>;
-    auto kern = P->qmc_type == DBGZ_QMC_SOBOL ? simt::k_genz_simt_batch<T, PolS> : simt::k_genz_simt_batch<T, PolR>;
+    using BL = BatchLoop<T>;
     DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(P->dcounter, 0, sizeof(unsigned long long), st));
-    kern<<<(unsigned)P->grid, simt::NT, sizeof(simt::SimtSmem<T>), st>>>(
+    BL::pick(P->qmc_type)<<<(unsigned)P->grid, BL::kThreads, BL::kSmem, st>>>(
         (const SimtParams<T> *)P->dparams, P->ditems, P->n_items, P->dcounter, (T *)P->dY, P->Dp);
     ++launches;
   }

@@ -1,0 +1,273 @@
+// loop_f64_kernels.cuh -- device code of the FP64 integration loop (launched
+// by loop_f64.cu, batch.cu and noalloc.cu).
+//
+// The FP64 units bound this loop: one warp-wide FMA takes 2 cycles of a
+// scheduler, as scalar DFMAs or inside mma.m8n8k4.f64 (16 cycles for 8 of
+// them; measured, both share one pipe).  The mma form is used for every
+// contraction because it needs an eighth of the issue slots and a twelfth of
+// the shared-memory reads, which leaves both to the special functions.
+//
+// One CTA = one tile of 128 samples = four warps of 32 samples, every thread
+// one sample.  y-indices run in groups of G = 64 (their targets are the
+// indices + 1):
+//   * S[32 x 64] of a warp = Y[:, 0 .. g0) U[0 .. g0, targets]: 4 x 8 mma
+//     tiles in registers (64 doubles a lane), Y and U staged in chunks of 8
+//     y-indices through a four-stage cp.async ring that lies in the S buffer,
+//     idle during this phase.  64 targets per sweep over Y keep the Y traffic
+//     at d / 128 reads of the workspace (it exceeds L2 from d of about 300).
+//   * in the group, sub-blocks of 8 targets: the sums get the contributions
+//     of the group's earlier y's by mma (the y's take the places of the sums
+//     they consumed, so the same buffer is the A operand), then 8 sequential
+//     steps, one thread per sample, with the sub-block's triangle as FMAs on
+//     8 registers that shift by one a step (static indices in a rolled loop:
+//     an unrolled one would not fit the instruction cache).
+// Warps only meet where they share staged data: per chunk of the sweep and
+// per 32 dimensions.
+#pragma once
+#include "internal.cuh"
+#include "genz_step.cuh"
+#include "policies.cuh"
+#include "loop_simt_kernels.cuh"
+
+namespace f64 {
+
+constexpr int TS = 128;  // samples per tile
+constexpr int NT = 128;  // threads per CTA
+constexpr int G = 64;    // y-indices per group
+constexpr int SB = 32;   // y-indices per staged block
+constexpr int KC = 8;    // y-indices per chunk of the sweep
+constexpr int NST = 4;   // stages of the sweep's ring
+
+using Params = simt::SimtParams<double>;
+
+struct Smem {
+  union {
+    double S[4][G][32];  // [warp][target, later y-index][sample ^ swizzle]
+    struct {
+      double Y[NST][4][KC][32];
+      double U[NST][G][KC + 4];  // row stride 12: conflict-free B fragments
+    } ring;
+  } u;
+  pol::Staged<double> sg;
+  double tri[SB / 8][8][8];  // [sub-block][k][j] = U[l0 + k, target of step k + j]
+  uint32_t sob[SB][dbgz::kSobolRow];
+  double red[NT / 32];
+};
+
+__device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+// sample `row` of row t of a [t][32] buffer: rows 4 apart in the low bits of
+// t, so that an A fragment (8 samples x 4 rows) touches every bank once
+__device__ __forceinline__ int swz(int t, int row) { return t * 32 + (row ^ ((t & 3) << 2)); }
+
+// One tile of 128 samples of the problem P (all NT threads; Yw is the CTA's
+// slot of the Y workspace, [y-index][sample], of which only indices that a
+// later group reads are written).
+template <typename Policy>
+__device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int64_t tile_id) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int fr = lane >> 2, fk = lane & 3;  // fragment row (or column) and k
+  const int64_t d = P.d, nY = d - 1;
+  const int64_t k_shift = tile_id / P.tiles_per_shift;
+  const int64_t j = (tile_id - k_shift * P.tiles_per_shift) * TS + tid;
+  double *S = &sm.u.S[warp][0][0];
+  Policy pl;
+  pl.tile_begin(P.gen, d, tile_id, P.tiles_per_shift, tid, P.c1, P.dc1, P.up1, P.cdf_form, P.io);
+  const uint64_t base0 = (uint64_t)(P.gen.sobol_first + pl.gen.gen_base + (j - tid));
+  const dbgz::SobolLane sob_lane(tid, base0);
+  pl.state_begin();
+
+  for (int64_t g0 = 0; g0 < nY; g0 += G) {
+    const int ng = (int)(nY - g0 < (int64_t)G ? nY - g0 : (int64_t)G);
+    const int nt = (ng + 7) >> 3;
+    const bool keep = g0 + G < nY;  // a later group reads this group's y's
+    if (g0 > 0) {
+      // ---- S = Y[:, 0 .. g0) U[0 .. g0, the group's targets] ----
+      double acc[4][8][2];
+#pragma unroll
+      for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 8; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+      const int nch = (int)(g0 / KC);
+      auto issue = [&](int ch) {
+        if (ch < nch) {
+          const int st = ch & (NST - 1);
+          const int64_t l0 = (int64_t)ch * KC;
+#pragma unroll
+          for (int e = 0; e < KC * 16 / 32; ++e) {
+            const int pc = lane + 32 * e, kk = pc >> 4, row = 2 * (pc & 15);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.u.ring.Y[st][warp][0][0] + swz(kk, row));
+            const double *src = Yw + (l0 + kk) * TS + 32 * warp + row;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+          }
+#pragma unroll
+          for (int e = 0; e < G * KC / NT; ++e) {
+            const int el = tid + NT * e, t = el >> 3, kk = el & 7;
+            if (t < 8 * nt) {
+              const bool v = g0 + 1 + t < d;
+              pol::cp_async_or_zero<8>(&sm.u.ring.U[st][t][kk], v ? P.U + (g0 + 1 + t) * d + l0 + kk : P.U, v);
+            }
+          }
+        }
+        pol::cp_async_commit();
+      };
+      __syncthreads();  // the ring lies in the S buffer: every warp is done with the last group
+#pragma unroll
+      for (int ch = 0; ch < NST - 1; ++ch) issue(ch);
+      for (int ch = 0; ch < nch; ++ch) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
+        __syncthreads();  // chunk ch has landed for all; the stage of chunk ch - 1 is free
+        issue(ch + NST - 1);
+        const double *Ys = &sm.u.ring.Y[ch & (NST - 1)][warp][0][0];
+        const double(*Us)[KC + 4] = sm.u.ring.U[ch & (NST - 1)];
+#pragma unroll
+        for (int k4 = 0; k4 < KC / 4; ++k4) {
+          double av[4];
+#pragma unroll
+          for (int mi = 0; mi < 4; ++mi) av[mi] = Ys[swz(4 * k4 + fk, 8 * mi + fr)];
+#pragma unroll
+          for (int ni = 0; ni < 8; ++ni)
+            if (ni < nt) {
+              const double bv = Us[8 * ni + fr][4 * k4 + fk];
+#pragma unroll
+              for (int mi = 0; mi < 4; ++mi) dmma(acc[mi][ni][0], acc[mi][ni][1], av[mi], bv);
+            }
+        }
+      }
+      __syncthreads();  // the ring is read: S may be written
+#pragma unroll
+      for (int ni = 0; ni < 8; ++ni)
+        if (ni < nt) {
+#pragma unroll
+          for (int mi = 0; mi < 4; ++mi) {
+            S[swz(8 * ni + 2 * fk, 8 * mi + fr)] = acc[mi][ni][0];
+            S[swz(8 * ni + 2 * fk + 1, 8 * mi + fr)] = acc[mi][ni][1];
+          }
+        }
+      __syncwarp();
+    }
+    // ---- sequential steps, 32 dimensions staged at a time ----
+    for (int b0 = 0; b0 < ng; b0 += SB) {
+      const int nb = ng - b0 < SB ? ng - b0 : SB;
+      const int64_t lb = g0 + b0;
+      __syncthreads();  // the last block's staging is read
+      pl.stage(sm.sg, P.tgt, tid, lb, nb);
+#pragma unroll
+      for (int e = tid; e < SB * 8; e += NT) {
+        const int li = e >> 3, jj = e & 7, kk = li & 7;
+        const bool v = kk + jj < 8 && li + jj < nb;
+        (&sm.tri[0][0][0])[e] = v ? P.U[(lb + li + jj + 1) * d + lb + li] : 0.0;
+      }
+      if constexpr (Policy::kSobolTable)
+        if (pl.gen.sobol_staged)
+          dbgz::sobol_stage_block(sm.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), base0, pl.sobol_l0(lb),
+                                  Policy::kSobolDir, d - 2, nb, tid);
+      __syncthreads();
+      for (int i0 = 0; i0 < nb; i0 += 8) {
+        const int q8 = b0 + i0;  // the sub-block's first target in the group
+        const int nv = nb - i0 < 8 ? nb - i0 : 8;
+        if (q8 > 0) {
+          double c[4][2];
+#pragma unroll
+          for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) c[mi][e] = g0 > 0 ? S[swz(q8 + 2 * fk + e, 8 * mi + fr)] : 0.0;
+          const bool v = g0 + q8 + 1 + fr < d;
+          const double *Ut = v ? P.U + (g0 + q8 + 1 + fr) * d + g0 + fk : P.U;
+          // 8 y's (two k steps) a round; the next round's coefficients are
+          // loaded while this one's products run
+          double b0v = v ? __ldg(Ut) : 0.0, b1v = v ? __ldg(Ut + 4) : 0.0;
+          for (int kk = 0; kk < q8; kk += 8) {
+            const double c0v = b0v, c1v = b1v;
+            if (kk + 8 < q8 && v) {
+              b0v = __ldg(Ut + kk + 8);
+              b1v = __ldg(Ut + kk + 12);
+            }
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi) dmma(c[mi][0], c[mi][1], S[swz(kk + fk, 8 * mi + fr)], c0v);
+#pragma unroll
+            for (int mi = 0; mi < 4; ++mi) dmma(c[mi][0], c[mi][1], S[swz(kk + 4 + fk, 8 * mi + fr)], c1v);
+          }
+#pragma unroll
+          for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) S[swz(q8 + 2 * fk + e, 8 * mi + fr)] = c[mi][e];
+          __syncwarp();
+        }
+        double s[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) s[t] = (g0 > 0 || q8 > 0) ? S[swz(q8 + t, lane)] : 0.0;
+#pragma unroll 1
+        for (int k = 0; k < nv; ++k) {
+          const int li = i0 + k;
+          const int64_t l = lb + li;
+          uint32_t xs = 0u;
+          if constexpr (Policy::kSobolTable)
+            if (pl.gen.sobol_staged) xs = sob_lane.at(sm.sob, li);
+          const double y = pl.emit_next(sm.sg, li, l, xs);
+          S[swz(q8 + k, lane)] = y;
+          if (keep) Yw[l * TS + tid] = y;
+          const double2 *tr = reinterpret_cast<const double2 *>(&sm.tri[i0 >> 3][k][0]);
+          const double2 t0 = tr[0], t1 = tr[1], t2 = tr[2], t3 = tr[3];
+          const double s0 = fma(y, t0.x, s[0]);
+          s[0] = fma(y, t0.y, s[1]);
+          s[1] = fma(y, t1.x, s[2]);
+          s[2] = fma(y, t1.y, s[3]);
+          s[3] = fma(y, t2.x, s[4]);
+          s[4] = fma(y, t2.y, s[5]);
+          s[5] = fma(y, t3.x, s[6]);
+          s[6] = fma(y, t3.y, s[7]);
+          pl.consume(sm.sg, s0, li, l);
+        }
+        // a partial sub-block (the problem's last) leaves unused rows: no later mma reads them
+        __syncwarp();
+      }
+    }
+  }
+  // ---- per-tile end and sum of p (fixed order) ----
+  pl.tile_end(P.tgt, tid, 0, tile_id, j < P.m);
+  double pv = pl.tile_value(j < P.m);
+  for (int o = 16; o > 0; o >>= 1) pv += __shfl_down_sync(0xffffffffu, pv, o);
+  if (lane == 0) sm.red[warp] = pv;
+  __syncthreads();
+  if (tid == 0) P.partials[tile_id] = ((sm.red[0] + sm.red[1]) + sm.red[2]) + sm.red[3];
+  __syncthreads();
+}
+
+template <typename Policy>
+__global__ void __launch_bounds__(NT, 3) k_genz_f64(const __grid_constant__ Params P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+  double *Yw = P.yws + (int64_t)blockIdx.x * P.Dp * TS;
+  for (int64_t t = P.tile0 + blockIdx.x; t < P.n_tiles; t += gridDim.x) tile<Policy>(P, sm, Yw, t);
+}
+
+// Many problems in one launch, work items from a global counter (as
+// simt::k_genz_simt_batch).
+template <typename Policy>
+__global__ void __launch_bounds__(NT, 3)
+    k_genz_f64_batch(const Params *params, const simt::BatchItem *items, int64_t n_items, unsigned long long *counter,
+                     double *yws, int64_t Dp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+  __shared__ Params Ps;
+  __shared__ long long cur;
+  double *Yw = yws + (int64_t)blockIdx.x * Dp * TS;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      cur = (long long)atomicAdd(counter, 1ull);
+      if (cur < n_items) Ps = params[items[cur].prob];
+    }
+    __syncthreads();
+    const long long it = cur;
+    if (it >= n_items) break;
+    const simt::BatchItem bi = items[it];
+    for (int64_t t = bi.tile0; t < (int64_t)bi.tile0 + bi.ntiles; ++t) tile<Policy>(Ps, sm, Yw, t);
+    __syncthreads();
+  }
+}
+
+}  // namespace f64

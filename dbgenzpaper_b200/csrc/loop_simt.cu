@@ -21,6 +21,7 @@
 //     sub-block 1 (128 x 32 x 32 GEMM from shared memory).
 //   * p is FP64; per-tile sums go to partials[tile] and a finalize kernel
 //     reduces them per shift in a fixed order (deterministic results).
+#include "loop_f64_kernels.cuh"
 #include "loop_simt_kernels.cuh"
 #include <algorithm>
 
@@ -77,17 +78,27 @@ int launch_simt(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   P.io.gu = pa.grad.gu;
   P.io.dc1 = pa.grad.dc1;
   P.io.tile0 = pa.tile0;
-  const size_t smem = sizeof(SimtSmem<T>);
-  auto kern = k_genz_simt<T, Policy>;
+  size_t smem;
+  int nt;
+  void (*kern)(SimtParams<T>);
+  if constexpr (sizeof(T) == 8) {
+    smem = sizeof(f64::Smem);
+    nt = f64::NT;
+    kern = f64::k_genz_f64<Policy>;
+  } else {
+    smem = sizeof(SimtSmem<T>);
+    nt = NT;
+    kern = k_genz_simt<T, Policy>;
+  }
   DBGZ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  DBGZ_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
+  DBGZ_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem));
   if (per_sm < 1) return dbgz_fail(ctx, DBGZ_ERR_CUDA, "simt loop: kernel does not fit on an SM");
   int64_t grid = std::min<int64_t>(n_tiles - pa.tile0, (int64_t)per_sm * ctx->num_sms);
   DBGZ_TRY(dbgz_ensure(ctx, p->yws, sizeof(T) * (size_t)P.Dp * TS * grid));
   P.yws = (T *)p->yws.p;
   if (pa.setup_only) return DBGZ_OK;
-  kern<<<(unsigned)grid, NT, smem, ctx->stream>>>(P);
+  kern<<<(unsigned)grid, nt, smem, ctx->stream>>>(P);
   dbgz_count_launch(ctx);
   DBGZ_CUDA_TRY(ctx, cudaGetLastError());
   return DBGZ_OK;

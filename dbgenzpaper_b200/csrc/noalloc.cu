@@ -10,10 +10,10 @@
 // lives in one file-scope __device__ array of fixed size compiled into the
 // library.  Every GPU that loads the library holds that array until exit.
 //
-// The kernels are the SIMT loop's own templates (loop_simt_kernels.cuh);
+// The kernels are the FP64 loop's own templates (loop_f64_kernels.cuh);
 // only the source of the first dimension's (c, dc) differs: it is computed
 // on the device into the array instead of on the host.
-#include "loop_simt_kernels.cuh"
+#include "loop_f64_kernels.cuh"
 #include <cuda.h>
 #include <algorithm>
 #include <mutex>
@@ -120,10 +120,10 @@ int setup_device(int dev, DeviceSlot &slot) {
     return DBGZ_ERR_CUDA;
   }
   s.ptr = (unsigned char *)p;
-  auto kern = k_genz_simt<double, NoallocPolicy>;
-  const int smem = (int)sizeof(SimtSmem<double>);
+  auto kern = f64::k_genz_f64<NoallocPolicy>;
+  const int smem = (int)sizeof(f64::Smem);
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s.per_sm, kern, NT, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s.per_sm, kern, f64::NT, smem) != cudaSuccess ||
       cudaDeviceGetAttribute(&s.num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       s.per_sm < 1) {
     cudaGetLastError();
@@ -189,7 +189,7 @@ extern "C" int dbgz_pnorm_pass_noalloc(int64_t d, const double *U, const double 
   P.cdf_form = DBGZ_CDF_ERF;
   P.yws = yws;
   P.partials = partials;
-  k_genz_simt<double, NoallocPolicy><<<(unsigned)grid, NT, sizeof(SimtSmem<double>), st>>>(P);
+  f64::k_genz_f64<NoallocPolicy><<<(unsigned)grid, f64::NT, sizeof(f64::Smem), st>>>(P);
   // the output accumulates a running mean with weight 0 for a first pass:
   // clear it so that stale or uninitialised contents cannot leak in
   if (cudaMemsetAsync(qmc_reps, 0, sizeof(double) * n_reps, st) != cudaSuccess) {

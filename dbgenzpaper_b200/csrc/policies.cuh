@@ -208,6 +208,12 @@ struct Forward {
     if (STORE) __stcs(io.y + ga0 + l * io.stride(), y);
     return y;
   }
+  // rolled form (FP64 loop): a policy that reads stored state keeps the next
+  // step's in registers
+  __device__ __forceinline__ void state_begin() {}
+  __device__ __forceinline__ T emit_next(const Staged<T> &sg, int li, int64_t l, uint32_t xs) {
+    return emit(sg, li, l, xs);
+  }
   // chunked form (8 steps whose per-sample inputs may be loaded up front)
   __device__ __forceinline__ void chunk_begin(int64_t, int) {}
   __device__ __forceinline__ void chunk_end(int64_t, int) {}
@@ -559,6 +565,19 @@ struct Adjoint {
     const int64_t t = d - 1 - l;
     const T y = t <= d - 2 ? io.y[ga0 + t * io.stride()] : T(0);
     return emit_from(sg, li, l, y, io.s[ga0 + t * io.stride()], io.dc[ga0 + t * io.stride()], xs);
+  }
+  // rolled form: the stored state of step l + 1 is loaded before step l runs
+  T nx_y, nx_s, nx_dc;
+  __device__ __forceinline__ void state_load(int64_t t) {
+    nx_y = t <= d - 2 ? io.y[ga0 + t * io.stride()] : T(0);
+    nx_s = io.s[ga0 + t * io.stride()];
+    nx_dc = io.dc[ga0 + t * io.stride()];
+  }
+  __device__ __forceinline__ void state_begin() { state_load(d - 1); }
+  __device__ __forceinline__ T emit_next(const Staged<T> &sg, int li, int64_t l, uint32_t xs) {
+    const T y = nx_y, s = nx_s, dc = nx_dc;
+    if (l + 1 < d - 1) state_load(d - 2 - l);
+    return emit_from(sg, li, l, y, s, dc, xs);
   }
   // chunked form: the stored state of the chunk's 8 steps (steps l0 .. l0+7,
   // n of them valid) is loaded before the first, so the loads overlap; in
