@@ -15,7 +15,8 @@
 //
 // Two numerics are provided:
 //  * StepFp64: the reference's Float64 arithmetic (erf form or erfc form of
-//    the CDF, the clamp to [-9, 9] in erf units, the same fma pattern).
+//    the CDF, the clamp to [-9, 9] in erf units, the same fma pattern), with
+//    the table-based erf and inverse erf of normal64.cuh.
 //  * StepFp32: FP32 arithmetic kept close to the FP64 result where the
 //    reference's Float32 loop loses digits (tail masses from normal32.cuh,
 //    relative error < 3e-6 where they are above 1e-10; Phi^-1 of the smaller
@@ -33,6 +34,7 @@
 //    u is clamped to [eps64, 1 - eps64] like the Float64 reference.
 #pragma once
 #include "normal32.cuh"
+#include "normal64.cuh"
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cfloat>
@@ -207,6 +209,7 @@ __device__ __forceinline__ uint32_t sobol_int(const uint32_t *Vl, uint64_t idx) 
 struct StepFp64 {
   double c, dc;
   double p;
+  const NormTab *tab;  // the CTA's table (set before init)
   __device__ __forceinline__ void init(double c1, double dc1, double /*up1*/) {
     c = c1;
     dc = dc1;
@@ -234,8 +237,7 @@ struct StepFp64 {
     u = fabs(fma(u, 2.0, -1.0));
     u = fma(u, dc, c);
     u = fmin(fmax(u, DBL_EPSILON), 1.0 - DBL_EPSILON);
-    double v = fma(2.0, u, -1.0);
-    return kSqrt2 * erfinv(v);
+    return sqrt2_erfinv_tab(*tab, fma(2.0, u, -1.0));
   }
   __device__ __forceinline__ void set_form(int) {}
   // the state between two steps, as four doubles (checkpoints)
@@ -253,12 +255,13 @@ struct StepFp64 {
   __device__ __forceinline__ void cdf(double s, double a, double b, double inv_u, int erfc_form) {
     double cv = (a - s) * inv_u;
     double dv = (b - s) * inv_u;
-    cv = fmax(fmin(cv, 9.0), -9.0);
-    dv = fmax(fmin(dv, 9.0), -9.0);
     if (!erfc_form) {
-      cv = 0.5 * (1.0 + erf(cv));
-      dv = 0.5 * (1.0 + erf(dv)) - cv;
+      // (erf is 1 to the last bit from 6 on, so the clamp to 9 has no effect)
+      cv = 0.5 * (1.0 + erf_tab(*tab, cv));
+      dv = 0.5 * (1.0 + erf_tab(*tab, dv)) - cv;
     } else {
+      cv = fmax(fmin(cv, 9.0), -9.0);
+      dv = fmax(fmin(dv, 9.0), -9.0);
       double c_val = 0.5 * erfc(-cv);
       dv = 0.5 * erfc(-dv) - c_val;
       cv = c_val;
@@ -279,16 +282,16 @@ struct StepFp64LowerInf : StepFp64 {
   __device__ __forceinline__ void set_form(int erfc_form) {
     double m9 = -9.0;
     asm volatile("" : "+d"(m9));
-    cinf = erfc_form ? 0.5 * erfc(-m9) : 0.5 * (1.0 + erf(m9));
+    cinf = erfc_form ? 0.5 * erfc(-m9) : 0.5 * (1.0 + erf_tab(*tab, m9));
   }
   __device__ __forceinline__ void cdf(double s, double /*a*/, double b, double inv_u, int erfc_form) {
     double dv = (b - s) * inv_u;
-    dv = fmax(fmin(dv, 9.0), -9.0);
     double cv;
     if (!erfc_form) {
       cv = cinf;
-      dv = 0.5 * (1.0 + erf(dv)) - cv;
+      dv = 0.5 * (1.0 + erf_tab(*tab, dv)) - cv;
     } else {
+      dv = fmax(fmin(dv, 9.0), -9.0);
       const double c_val = cinf;
       dv = 0.5 * erfc(-dv) - c_val;
       cv = c_val;

@@ -52,6 +52,7 @@ struct Smem {
   double tri[SB / 8][8][8];  // [sub-block][k][j] = U[l0 + k, target of step k + j]
   uint32_t sob[SB][dbgz::kSobolRow];
   double red[NT / 32];
+  dbgz::NormTab tab;
 };
 
 __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
@@ -75,6 +76,7 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
   const int64_t j = (tile_id - k_shift * P.tiles_per_shift) * TS + tid;
   double *S = &sm.u.S[warp][0][0];
   Policy pl;
+  pl.set_tab(&sm.tab);
   pl.tile_begin(P.gen, d, tile_id, P.tiles_per_shift, tid, P.c1, P.dc1, P.up1, P.cdf_form, P.io);
   const uint64_t base0 = (uint64_t)(P.gen.sobol_first + pl.gen.gen_base + (j - tid));
   const dbgz::SobolLane sob_lane(tid, base0);
@@ -241,6 +243,8 @@ template <typename Policy>
 __global__ void __launch_bounds__(NT, 3) k_genz_f64(const __grid_constant__ Params P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+  dbgz::norm_tab_load(sm.tab, threadIdx.x, NT);
+  __syncthreads();
   double *Yw = P.yws + (int64_t)blockIdx.x * P.Dp * TS;
   for (int64_t t = P.tile0 + blockIdx.x; t < P.n_tiles; t += gridDim.x) tile<Policy>(P, sm, Yw, t);
 }
@@ -253,6 +257,8 @@ __global__ void __launch_bounds__(NT, 3)
                      double *yws, int64_t Dp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+  dbgz::norm_tab_load(sm.tab, threadIdx.x, NT);
+  __syncthreads();
   __shared__ Params Ps;
   __shared__ long long cur;
   double *Yw = yws + (int64_t)blockIdx.x * Dp * TS;

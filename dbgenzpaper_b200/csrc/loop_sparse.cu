@@ -95,7 +95,12 @@ __global__ void __launch_bounds__(TS) k_genz_sparse(const SparseParams<T> P) {
   __shared__ pol::Staged<T> sg;
   __shared__ uint32_t sob[Policy::kSobolTable ? CB : 1][dbgz::kSobolRow];  // Sobol integers of the block (dbgz::sobol_stage_block)
   __shared__ double red[TS / 32];
+  __shared__ std::conditional_t<sizeof(T) == 8, dbgz::NormTab, int> tab;  // FP64 step
   const int r = threadIdx.x;
+  if constexpr (sizeof(T) == 8) {
+    dbgz::norm_tab_load(tab, r, TS);
+    __syncthreads();
+  }
   const int W = P.W;
   T *yr = P.ring_in_smem ? ring : P.yglob + (int64_t)blockIdx.x * P.W * TS;
 
@@ -103,6 +108,7 @@ __global__ void __launch_bounds__(TS) k_genz_sparse(const SparseParams<T> P) {
     const int64_t k = tile / P.tiles_per_shift;
     const int64_t j = (tile - k * P.tiles_per_shift) * TS + r;
     Policy pl;
+    if constexpr (sizeof(T) == 8) pl.set_tab(&tab);
     pl.tile_begin(P.gen, P.d, tile, P.tiles_per_shift, r, P.c1, P.dc1, P.up1, 0, P.io);
     // this row's terms of the staged Sobol integers of the tile
     const dbgz::SobolLane sob_lane(r, (uint64_t)(P.gen.sobol_first + pl.gen.gen_base + (j - r)));

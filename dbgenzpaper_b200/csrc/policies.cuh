@@ -160,6 +160,10 @@ struct Forward {
   int cdf_form;
   GradIO<T> io;
 
+  // the FP64 step's table, before tile_begin
+  __device__ __forceinline__ void set_tab(const dbgz::NormTab *tab) {
+    if constexpr (std::is_same<T, double>::value) st.tab = tab;
+  }
   __device__ __forceinline__ void tile_begin(const dbgz::GenParams &gp, int64_t d_, int64_t tile,
                                              int64_t tiles_per_shift, int r, double c1, double dc1,
                                              double up1, int cdf_form_, const GradIO<T> &io_) {
@@ -319,6 +323,7 @@ struct Adjoint {
   float wrel;
   int warp, lane;
 
+  __device__ __forceinline__ void set_tab(const dbgz::NormTab *) {}
   __device__ __forceinline__ void tile_begin(const dbgz::GenParams &gp, int64_t d_, int64_t tile_,
                                              int64_t tiles_per_shift, int r, double, double, double, int,
                                              const GradIO<T> &io_) {
