@@ -215,11 +215,11 @@ struct StepFp64 {
     dc = dc1;
     p = dc1;
   }
-  // Returns y_l for QMC dimension l of sample (point index j in the pass,
-  // 0-based; shift k).
-  template <bool kIntTent = true>  // (no effect in FP64)
-  __device__ __forceinline__ double quantile(const GenParams &g, int64_t d, int64_t j, int64_t k,
-                                             int64_t l, double qv, double shiftv, uint32_t x0) const {
+  // w = |2u - 1| of QMC dimension l of the sample (point index j in the pass,
+  // 0-based; shift k): independent of the recursion, so that a loop can form
+  // the next step's early.
+  static __device__ __forceinline__ double tent(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l,
+                                                double qv, double shiftv, uint32_t x0) {
     double u;
     if (g.qmc_type == 0) {
       double x = __dmul_rn((double)(g.gen_base + j + 1), qv);
@@ -234,10 +234,18 @@ struct StepFp64 {
       uint64_t sh = g.sobol_staged ? 0ull : g.ushift[k * (d - 1) + l] & mask;
       u = (double)((xi ^ sh) & mask) * ldexp(1.0, -L);
     }
-    u = fabs(fma(u, 2.0, -1.0));
-    u = fma(u, dc, c);
+    return fabs(fma(u, 2.0, -1.0));
+  }
+  // y_l from w
+  __device__ __forceinline__ double quantile_w(double w) const {
+    double u = fma(w, dc, c);
     u = fmin(fmax(u, DBL_EPSILON), 1.0 - DBL_EPSILON);
     return sqrt2_erfinv_tab(*tab, fma(2.0, u, -1.0));
+  }
+  template <bool kIntTent = true>  // (no effect in FP64)
+  __device__ __forceinline__ double quantile(const GenParams &g, int64_t d, int64_t j, int64_t k,
+                                             int64_t l, double qv, double shiftv, uint32_t x0) const {
+    return quantile_w(tent(g, d, j, k, l, qv, shiftv, x0));
   }
   __device__ __forceinline__ void set_form(int) {}
   // the state between two steps, as four doubles (checkpoints)

@@ -33,7 +33,11 @@ namespace f64 {
 
 constexpr int TS = 128;  // samples per tile
 constexpr int NT = 128;  // threads per CTA
-constexpr int G = 64;    // y-indices per group
+#ifndef F64_G
+#define F64_G 64
+#define F64_C 3
+#endif
+constexpr int G = F64_G;    // y-indices per group
 constexpr int SB = 32;   // y-indices per staged block
 constexpr int KC = 8;    // y-indices per chunk of the sweep
 constexpr int NST = 4;   // stages of the sweep's ring
@@ -88,11 +92,11 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
     const bool keep = g0 + G < nY;  // a later group reads this group's y's
     if (g0 > 0) {
       // ---- S = Y[:, 0 .. g0) U[0 .. g0, the group's targets] ----
-      double acc[4][8][2];
+      double acc[4][G / 8][2];
 #pragma unroll
       for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 8; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+        for (int ni = 0; ni < G / 8; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
       const int nch = (int)(g0 / KC);
       auto issue = [&](int ch) {
         if (ch < nch) {
@@ -131,7 +135,7 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
 #pragma unroll
           for (int mi = 0; mi < 4; ++mi) av[mi] = Ys[swz(4 * k4 + fk, 8 * mi + fr)];
 #pragma unroll
-          for (int ni = 0; ni < 8; ++ni)
+          for (int ni = 0; ni < G / 8; ++ni)
             if (ni < nt) {
               const double bv = Us[8 * ni + fr][4 * k4 + fk];
 #pragma unroll
@@ -141,7 +145,7 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
       }
       __syncthreads();  // the ring is read: S may be written
 #pragma unroll
-      for (int ni = 0; ni < 8; ++ni)
+      for (int ni = 0; ni < G / 8; ++ni)
         if (ni < nt) {
 #pragma unroll
           for (int mi = 0; mi < 4; ++mi) {
@@ -168,6 +172,14 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
           dbgz::sobol_stage_block(sm.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), base0, pl.sobol_l0(lb),
                                   Policy::kSobolDir, d - 2, nb, tid);
       __syncthreads();
+      // the tent-transformed point of step li, formed one step ahead
+      auto point = [&](int li) -> double {
+        uint32_t xs = 0u;
+        if constexpr (Policy::kSobolTable)
+          if (pl.gen.sobol_staged) xs = sob_lane.at(sm.sob, li);
+        return pl.point(sm.sg, li, lb + li, xs);
+      };
+      double w = point(0);
       for (int i0 = 0; i0 < nb; i0 += 8) {
         const int q8 = b0 + i0;  // the sub-block's first target in the group
         const int nv = nb - i0 < 8 ? nb - i0 : 8;
@@ -206,14 +218,13 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
         for (int k = 0; k < nv; ++k) {
           const int li = i0 + k;
           const int64_t l = lb + li;
-          uint32_t xs = 0u;
-          if constexpr (Policy::kSobolTable)
-            if (pl.gen.sobol_staged) xs = sob_lane.at(sm.sob, li);
-          const double y = pl.emit_next(sm.sg, li, l, xs);
-          S[swz(q8 + k, lane)] = y;
-          if (keep) Yw[l * TS + tid] = y;
           const double2 *tr = reinterpret_cast<const double2 *>(&sm.tri[i0 >> 3][k][0]);
           const double2 t0 = tr[0], t1 = tr[1], t2 = tr[2], t3 = tr[3];
+          const double wn = point(li + 1 < nb ? li + 1 : li);
+          const double y = pl.emit_next(sm.sg, li, l, w);
+          w = wn;
+          S[swz(q8 + k, lane)] = y;
+          if (keep) Yw[l * TS + tid] = y;
           const double s0 = fma(y, t0.x, s[0]);
           s[0] = fma(y, t0.y, s[1]);
           s[1] = fma(y, t1.x, s[2]);
@@ -240,7 +251,7 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
 }
 
 template <typename Policy>
-__global__ void __launch_bounds__(NT, 3) k_genz_f64(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(NT, F64_C) k_genz_f64(const __grid_constant__ Params P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   dbgz::norm_tab_load(sm.tab, threadIdx.x, NT);
@@ -252,7 +263,7 @@ __global__ void __launch_bounds__(NT, 3) k_genz_f64(const __grid_constant__ Para
 // Many problems in one launch, work items from a global counter (as
 // simt::k_genz_simt_batch).
 template <typename Policy>
-__global__ void __launch_bounds__(NT, 3)
+__global__ void __launch_bounds__(NT, F64_C)
     k_genz_f64_batch(const Params *params, const simt::BatchItem *items, int64_t n_items, unsigned long long *counter,
                      double *yws, int64_t Dp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];

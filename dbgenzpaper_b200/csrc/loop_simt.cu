@@ -46,8 +46,8 @@ int launch_simt(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   P.gen.gen_base = pa.gen_base;
   P.gen.gen_base_dev = pa.gen_base_dev;
   P.gen.sobol_first = pa.sobol_first;
-  // staged Sobol integers (not in the adjoint pass)
-  P.gen.sobol_staged = pa.qmc_type == DBGZ_QMC_SOBOL && pa.kind != kLoopAdjoint;
+  // staged Sobol integers (not in the FP32 adjoint pass)
+  P.gen.sobol_staged = pa.qmc_type == DBGZ_QMC_SOBOL && (sizeof(T) == 8 || pa.kind != kLoopAdjoint);
   P.gen.q = (const double *)p->q.p;
   P.gen.shift64 = (const double *)p->shifts.p;
   P.gen.shift32 = (const float *)p->shifts32.p;

@@ -142,11 +142,11 @@ struct Forward {
   // consume_deferred + tail_repair available (the FP32 steps): the loop may
   // run a chunk of steps without the same-tail branch
   static constexpr bool kDeferTail = std::is_same<T, float>::value;
-  // takes staged Sobol integers (GenParams::sobol_staged); not in the pass
+  // takes staged Sobol integers (GenParams::sobol_staged); not in the FP32 pass
   // that keeps the state for the adjoint (measured on the banded d = 10^4,
   // bandwidth 64 workload at 2^14 x 10 Sobol points:
   // the gradient call 125.1 ms without, 136.9 ms with them)
-  static constexpr bool kSobolTable = GEN == DBGZ_QMC_SOBOL && !STORE;
+  static constexpr bool kSobolTable = GEN == DBGZ_QMC_SOBOL && (!STORE || std::is_same<T, double>::value);
   // the QMC dimension of step li of a block: lbase + li
   static constexpr int kSobolDir = 1;
   __device__ __forceinline__ int64_t sobol_l0(int64_t lbase) const { return lbase; }
@@ -212,11 +212,17 @@ struct Forward {
     if (STORE) __stcs(io.y + ga0 + l * io.stride(), y);
     return y;
   }
-  // rolled form (FP64 loop): a policy that reads stored state keeps the next
-  // step's in registers
+  // rolled form (FP64 loop): point() gives a step's tent-transformed point,
+  // formed one step early, emit_next the step's value from it; a policy that
+  // reads stored state keeps the next step's in registers
   __device__ __forceinline__ void state_begin() {}
-  __device__ __forceinline__ T emit_next(const Staged<T> &sg, int li, int64_t l, uint32_t xs) {
-    return emit(sg, li, l, xs);
+  __device__ __forceinline__ T point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
+    return Step::tent(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs);
+  }
+  __device__ __forceinline__ T emit_next(const Staged<T> &, int, int64_t l, T w) {
+    const T y = st.quantile_w(w);
+    if (STORE) __stcs(io.y + ga0 + l * io.stride(), y);
+    return y;
   }
   // chunked form (8 steps whose per-sample inputs may be loaded up front)
   __device__ __forceinline__ void chunk_begin(int64_t, int) {}
@@ -548,8 +554,11 @@ struct Adjoint {
   }
   __device__ __forceinline__ T emit_from(const Staged<T> &sg, int li, int64_t l, T y, T s, T dc, uint32_t xs) {
     const int64_t t = d - 1 - l;
+    return emit_at(sg, li, l, y, s, dc, t <= d - 2 ? point_w(sg, li, t, xs, gen.sobol_staged != 0) : 0.0);
+  }
+  __device__ __forceinline__ T emit_at(const Staged<T> &sg, int li, int64_t l, T y, T s, T dc, double w) {
+    const int64_t t = d - 1 - l;
     const bool has_u = t <= d - 2;
-    const double w = has_u ? point_w(sg, li, t, xs, gen.sobol_staged != 0) : 0.0;
     if (sizeof(T) == 4) {
       float fa, fb, fu;
       const float sb = variable32(sg.tg[li], (float)w, has_u, (float)y, (float)s, (float)dc, true, fa, fb, fu);
@@ -579,10 +588,14 @@ struct Adjoint {
     nx_dc = io.dc[ga0 + t * io.stride()];
   }
   __device__ __forceinline__ void state_begin() { state_load(d - 1); }
-  __device__ __forceinline__ T emit_next(const Staged<T> &sg, int li, int64_t l, uint32_t xs) {
+  __device__ __forceinline__ T point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
+    const int64_t t = d - 1 - l;
+    return t <= d - 2 ? (T)point_w(sg, li, t, xs, gen.sobol_staged != 0) : T(0);
+  }
+  __device__ __forceinline__ T emit_next(const Staged<T> &sg, int li, int64_t l, T w) {
     const T y = nx_y, s = nx_s, dc = nx_dc;
     if (l + 1 < d - 1) state_load(d - 2 - l);
-    return emit_from(sg, li, l, y, s, dc, xs);
+    return emit_at(sg, li, l, y, s, dc, (double)w);
   }
   // chunked form: the stored state of the chunk's 8 steps (steps l0 .. l0+7,
   // n of them valid) is loaded before the first, so the loads overlap; in
