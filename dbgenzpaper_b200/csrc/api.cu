@@ -465,7 +465,8 @@ int dbgz_problem_free(dbgz_problem *p) {
                     &p->shifts32, &p->V,   &p->ushifts, &p->tgt64,      &p->tgt32,   &p->U32,       &p->Uhi,
                     &p->Ulo,   &p->Utf,     &p->Ub,      &p->Ub32,       &p->Ubhi,    &p->Ublo,      &p->Ubtf,
                     &p->grad_buf, &p->yws, &p->partials, &p->reps,      &p->csc_colptr, &p->csc_row, &p->csc_val64,
-                    &p->csc_val32, &p->cscb_colptr, &p->cscb_row, &p->cscb_val64, &p->cscb_val32};
+                    &p->csc_val32, &p->cscb_colptr, &p->cscb_row, &p->cscb_val64, &p->cscb_val32,
+                    &p->w32_ops, &p->w32b_ops};
   for (DevBuf *b : bufs) dbgz_release(*b);
   dbgz_drop_graphs(p);
   dbgz_release(p->drv_state);
@@ -494,7 +495,7 @@ int dbgz_problem_truncate_band(dbgz_problem *p, int64_t bandwidth) {
   DBGZ_TRY(dbgz_band_dev(ctx, p->d, (double *)p->U.p, bandwidth));
   DevBuf *derived[] = {&p->U32, &p->Uhi,  &p->Ulo,  &p->Utf,  &p->Ub,         &p->Ub32,    &p->Ubhi,
                        &p->Ublo, &p->Ubtf, &p->csc_colptr, &p->csc_row, &p->csc_val64, &p->csc_val32,
-                       &p->cscb_colptr, &p->cscb_row, &p->cscb_val64, &p->cscb_val32};
+                       &p->cscb_colptr, &p->cscb_row, &p->cscb_val64, &p->cscb_val32, &p->w32_ops, &p->w32b_ops};
   for (DevBuf *b : derived) dbgz_release(*b);
   dbgz_drop_graphs(p);
   p->ldU = 0;

@@ -272,7 +272,8 @@ struct dbgz_batch_plan {
   uint64_t *dush = nullptr;
   int *dflags = nullptr;  // np + 1 words: per-problem input checks, then the shift check
   unsigned long long *dcounter = nullptr;
-  UmmaBatchPlan *tb = nullptr;
+  UmmaBatchPlan *tb = nullptr;  // TF32
+  W32BatchPlan *wb = nullptr;   // split BF16
   // pinned host block (graph mode): inputs, then outputs
   void *hblock = nullptr;
   double *hSigma = nullptr, *ha = nullptr, *hb = nullptr, *hreps = nullptr;
@@ -292,6 +293,7 @@ int plan_free(dbgz_batch_plan *P) {
   if (P->graph) cudaGraphDestroy(P->graph);
   if (P->ctx) cudaStreamSynchronize(P->ctx->stream);
   dbgz_umma_batch_free(P->tb);
+  dbgz_w32_batch_free(P->wb);
   dbgz_release(P->buf);
   if (P->hblock) cudaFreeHost(P->hblock);
   if (P->ctx) --P->ctx->live_problems;
@@ -415,7 +417,7 @@ int plan_setup(dbgz_batch_plan *P, const dbgz_opts &o, const uint32_t *dirnums, 
     S.n_reps = R;
     S.tiles_per_shift = tps;
     S.n_tiles = tps * R;
-    S.Dp = Dp;
+    S.Dp = S.ring = Dp;
     S.gen.qmc_type = P->qmc_type;
     S.gen.n_bits = P->n_bits;
     S.gen.gen_base = 0;
@@ -478,7 +480,10 @@ int plan_setup(dbgz_batch_plan *P, const dbgz_opts &o, const uint32_t *dirnums, 
     A.dV = P->qmc_type == DBGZ_QMC_SOBOL ? P->dV : nullptr;
     A.dush = P->qmc_type == DBGZ_QMC_SOBOL ? P->dush : nullptr;
     A.dpart = P->dpart;
-    DBGZ_TRY(dbgz_umma_batch_setup(ctx, P->precision, A, &P->tb));
+    if (P->precision == DBGZ_PREC_FP32_SPLIT_BF16)
+      DBGZ_TRY(dbgz_w32_batch_setup(ctx, A, &P->wb));
+    else
+      DBGZ_TRY(dbgz_umma_batch_setup(ctx, P->precision, A, &P->tb));
   }
   return DBGZ_OK;
 }
@@ -519,6 +524,10 @@ int plan_enqueue(dbgz_batch_plan *P, const double *Sigma, const double *a, const
   plan_event(P, 3, capturing);
   if (P->tb) {
     DBGZ_TRY(dbgz_umma_batch_enqueue(P->tb));
+    launches += 2;
+  }
+  if (P->wb) {
+    DBGZ_TRY(dbgz_w32_batch_enqueue(P->wb));
     launches += 2;
   }
   if (P->n_items) {

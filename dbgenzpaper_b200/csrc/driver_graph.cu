@@ -107,7 +107,7 @@ std::vector<uint64_t> signature(const dbgz_problem *p, int precision, const Pass
   const DevBuf *bufs[] = {&p->U,      &p->U32,    &p->Uhi,        &p->Ulo,        &p->Utf,         &p->yws,
                           &p->partials, &p->reps, &p->drv_state, &p->q,          &p->shifts,      &p->shifts32,
                           &p->V,      &p->ushifts, &p->tgt32,     &p->tgt64,      &p->csc_colptr,  &p->csc_row,
-                          &p->csc_val64, &p->csc_val32};
+                          &p->csc_val64, &p->csc_val32, &p->w32_ops};
   for (const DevBuf *b : bufs) {
     addp(b->p);
     s.push_back((uint64_t)b->bytes);

@@ -207,6 +207,7 @@ __device__ __forceinline__ uint32_t sobol_int(const uint32_t *Vl, uint64_t idx) 
 
 // ---------------------------------------------------------------- FP64 ---
 struct StepFp64 {
+  using Tent = double;
   double c, dc;
   double p;
   const NormTab *tab;  // the CTA's table (set before init)
@@ -218,11 +219,12 @@ struct StepFp64 {
   // w = |2u - 1| of QMC dimension l of the sample (point index j in the pass,
   // 0-based; shift k): independent of the recursion, so that a loop can form
   // the next step's early.
+  template <bool kIntTent = true>  // (no effect in FP64)
   static __device__ __forceinline__ double tent(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l,
-                                                double qv, double shiftv, uint32_t x0) {
+                                                double qv, double shiftv, uint32_t x0, double jd) {
     double u;
     if (g.qmc_type == 0) {
-      double x = __dmul_rn((double)(g.gen_base + j + 1), qv);
+      double x = __dmul_rn(jd, qv);
       x = x - floor(x);
       u = shiftv + x;
       u = u > 1.0 ? u - 1.0 : u;
@@ -244,8 +246,8 @@ struct StepFp64 {
   }
   template <bool kIntTent = true>  // (no effect in FP64)
   __device__ __forceinline__ double quantile(const GenParams &g, int64_t d, int64_t j, int64_t k,
-                                             int64_t l, double qv, double shiftv, uint32_t x0) const {
-    return quantile_w(tent(g, d, j, k, l, qv, shiftv, x0));
+                                             int64_t l, double qv, double shiftv, uint32_t x0, double jd) const {
+    return quantile_w(tent(g, d, j, k, l, qv, shiftv, x0, jd));
   }
   __device__ __forceinline__ void set_form(int) {}
   // the state between two steps, as four doubles (checkpoints)
@@ -332,24 +334,30 @@ struct StepFp32 {
   // the adjoint keeps the FP64 form (measured on the banded d = 10^4,
   // bandwidth 64 workload at 2^14 x 10 Sobol points: its
   // gradient call 125.1 ms against 146.4 ms with the integer form)
-  template <bool kIntTent = true>
-  __device__ __forceinline__ float quantile(const GenParams &g, int64_t d, int64_t j, int64_t k,
-                                            int64_t l, double qv, float shiftv, uint32_t x0) const {
+  // The tent-transformed point of QMC dimension l, w = |2u - 1| and w1 = 1 - w
+  // (jd: the lattice multiplier gen_base + j + 1): independent of the
+  // recursion, so that a loop can form it early.
+  struct Tent {
     float w, w1;
+  };
+  template <bool kIntTent = true>
+  static __device__ __forceinline__ Tent tent(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l, double qv,
+                                              float shiftv, uint32_t x0, double jd) {
+    Tent r;
     if (g.qmc_type == 0) {
-      double x = __dmul_rn((double)(g.gen_base + j + 1), qv);
+      double x = __dmul_rn(jd, qv);
       x = x - floor(x);
       float u = shiftv + (float)x;
       u = u > 1.0f ? u - 1.0f : u;
-      w = fabsf(fmaf(u, 2.0f, -1.0f));
-      w1 = 2.0f * fminf(u, 1.0f - u);  // 1 - |2u - 1|
+      r.w = fabsf(fmaf(u, 2.0f, -1.0f));
+      r.w1 = 2.0f * fminf(u, 1.0f - u);  // 1 - |2u - 1|
     } else if (kIntTent) {
       // n_bits <= 32: the shifted integer has at most 32 bits
       const int L = g.n_bits;
       const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
       const uint32_t xw = g.sobol_staged ? x0 : sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j));
       const uint32_t sh = g.sobol_staged ? 0u : (uint32_t)g.ushift[k * (d - 1) + l];
-      sobol_tent_f32((xw ^ sh) & mask, L, w, w1);
+      sobol_tent_f32((xw ^ sh) & mask, L, r.w, r.w1);
     } else {
       const int L = g.n_bits;
       const uint64_t mask = (L >= 64) ? ~0ull : ((1ull << L) - 1);
@@ -357,17 +365,26 @@ struct StepFp32 {
       const uint64_t xi = (uint64_t)xw & mask;
       const uint64_t sh = g.sobol_staged ? 0ull : g.ushift[k * (d - 1) + l] & mask;
       const double u = (double)((xi ^ sh) & mask) * ldexp(1.0, -L);
-      w = (float)fabs(fma(u, 2.0, -1.0));
-      w1 = (float)(2.0 * fmin(u, 1.0 - u));
+      r.w = (float)fabs(fma(u, 2.0, -1.0));
+      r.w1 = (float)(2.0 * fmin(u, 1.0 - u));
     }
+    return r;
+  }
+  // y_l from the point
+  __device__ __forceinline__ float quantile_w(const Tent &q) const {
     const float kEps = (float)DBL_EPSILON;
     // u = lo + w dc when that is <= 1/2, else 1 - u = up + (1 - w) dc;
     // Phi^-1 is taken of the smaller one (one call site keeps the code small)
-    const float t = fmaf(w, dc, lo);
+    const float t = fmaf(q.w, dc, lo);
     const bool lower = t <= 0.5f;
-    const float arg = lower ? t : fmaf(w1, dc, up);
+    const float arg = lower ? t : fmaf(q.w1, dc, up);
     const float y = phi_inv_lower_f32(fmaxf(arg, kEps));
     return lower ? y : -y;
+  }
+  template <bool kIntTent = true>
+  __device__ __forceinline__ float quantile(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l, double qv,
+                                            float shiftv, uint32_t x0, double jd) const {
+    return quantile_w(tent<kIntTent>(g, d, j, k, l, qv, shiftv, x0, jd));
   }
   __device__ __forceinline__ void set_form(int) {}
   // the state between two steps, as four doubles (checkpoints; the floats

@@ -106,7 +106,12 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   // to the next segment.  The same kernels and arithmetic as storing
   // everything: the same bits, with the stored state of K = ceil((d-1)/seg)
   // checkpoints instead of d rows.
-  const int64_t seg = sparse ? ctx->grad_ckpt_seg : 0;
+  // Problems that run in the loops that treat the band as dense
+  // (dbgz_band_loop) store the state of every variable and bound it by chunks of
+  // samples alone, whatever the checkpoint setting: no recomputation (the
+  // setting applies to the CSC loop).
+  if (sparse && !p->csc_colptr.p) DBGZ_TRY(dbgz_build_csc(p));
+  const int64_t seg = sparse && !dbgz_band_loop(p, precision) ? ctx->grad_ckpt_seg : 0;
   const int64_t nY = d - 1, K = seg > 0 ? (nY + seg - 1) / seg : 0;
   const bool ckpt = seg > 0 && K >= 1;
   int64_t Wf = 0, Wb = 0;  // ring sizes of the forward and adjoint banded loops

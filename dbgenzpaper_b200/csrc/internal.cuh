@@ -113,6 +113,7 @@ struct dbgz_problem {
   // (coefficients of the adjoint recurrence, policies.cuh)
   DevBuf Ub, Ub32, Ubhi, Ublo, Ubtf;
   int64_t ldUb = 0;
+  DevBuf w32_ops, w32b_ops;  // warp-level FP32 loop: panels and triangles of U and Ub (loop_w32_impl.cuh)
   DevBuf grad_buf;       // forward state and partial gradients of dbgz_pnorm_grad
   // sparse (banded) structure: CSC of the strict upper factor
   DevBuf csc_colptr, csc_row, csc_val64, csc_val32;
@@ -200,6 +201,9 @@ int dbgz_loop_simt(dbgz_problem *p, const PassArgs &pa, int precision, double *p
                    int64_t n_tiles);
 int dbgz_loop_umma(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,
                    int64_t n_tiles);
+// The warp-level FP32 loop: dense split-BF16, and banded (p->bandwidth).
+int dbgz_loop_w32(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n_tiles);
+int dbgz_loop_w32_band(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n_tiles);
 // Forward tensor-core loop over many problems of at most two halves (d - 1 <= 256) in
 // one launch (batch.cu).  Host tables cover all problems of the batch;
 // `probs` lists the ones to run here, largest first.  Device pointers: FP64
@@ -233,12 +237,27 @@ struct UmmaBatchPlan {
   int32_t *d_iprob = nullptr, *d_itile = nullptr;
   const double *dM = nullptr;
 };
+// The split-BF16 batch's tensor part: the warp-level loop over (problem, tile)
+// items from a counter (loop_w32.cu); the same interface.
+struct W32BatchPlan {
+  dbgz_ctx *ctx = nullptr;
+  int qmc_type = 0, smem = 0;
+  DevBuf buf;
+  char *d_ops = nullptr, *d_probs = nullptr;
+  unsigned long long *d_counter = nullptr;
+  unsigned char *yws = nullptr;
+  int64_t nsel = 0, nt = 0, n_items = 0, grid = 0, slot = 0;
+};
+int dbgz_w32_batch_setup(dbgz_ctx *ctx, const UmmaBatchArgs &A, W32BatchPlan **out);
+int dbgz_w32_batch_enqueue(W32BatchPlan *B);
+void dbgz_w32_batch_free(W32BatchPlan *B);
 int dbgz_umma_batch_setup(dbgz_ctx *ctx, int precision, const UmmaBatchArgs &A, UmmaBatchPlan **out);
 int dbgz_umma_batch_enqueue(UmmaBatchPlan *B);
 void dbgz_umma_batch_free(UmmaBatchPlan *B);
 int dbgz_loop_sparse(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,
                      int64_t n_tiles);
 int dbgz_build_csc(dbgz_problem *p);
+bool dbgz_band_loop(dbgz_problem *p, int precision);  // after dbgz_build_csc
 void dbgz_drop_graphs(dbgz_problem *p);
 // dU[t*d + l] (+)= sum_n Y(l, n) S(t, n) over the nc samples, for l < t only,
 // Y and S tile-major ([tile][row < d][128 samples], the FP32 layout of

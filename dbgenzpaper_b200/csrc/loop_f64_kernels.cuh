@@ -8,13 +8,14 @@
 // the shared-memory reads, which leaves both to the special functions.
 //
 // One CTA = one tile of 128 samples = four warps of 32 samples, every thread
-// one sample.  y-indices run in groups of G = 64 (their targets are the
-// indices + 1):
-//   * S[32 x 64] of a warp = Y[:, 0 .. g0) U[0 .. g0, targets]: 4 x 8 mma
-//     tiles in registers (64 doubles a lane), Y and U staged in chunks of 8
-//     y-indices through a four-stage cp.async ring that lies in the S buffer,
-//     idle during this phase.  64 targets per sweep over Y keep the Y traffic
-//     at d / 128 reads of the workspace (it exceeds L2 from d of about 300).
+// one sample.  y-indices run in groups of G (their targets are the indices + 1):
+//   * S[32 x G] of a warp = Y[:, k0 .. g0) U[k0 .. g0, targets]: 4 x G/8 mma
+//     tiles in registers, Y and U staged in chunks of 8 y-indices through a
+//     cp.async ring that lies in the S buffer, idle during this phase.  Banded
+//     factors: k0 is the first y-index within the band of the group, else 0.
+//     G = 32 with 16 warps an SM measured faster than G = 64 with 12 (d = 500:
+//     3.60 against 3.84 ms; equal at d = 1000, where its sweeps read Y twice
+//     as often; gradient at d = 150 1.82 against 2.00 ms);
 //   * in the group, sub-blocks of 8 targets: the sums get the contributions
 //     of the group's earlier y's by mma (the y's take the places of the sums
 //     they consumed, so the same buffer is the A operand), then 8 sequential
@@ -22,7 +23,7 @@
 //     8 registers that shift by one a step (static indices in a rolled loop:
 //     an unrolled one would not fit the instruction cache).
 // Warps only meet where they share staged data: per chunk of the sweep and
-// per 32 dimensions.
+// per 32 dimensions (whose constants are copied one block ahead).
 #pragma once
 #include "internal.cuh"
 #include "genz_step.cuh"
@@ -33,17 +34,18 @@ namespace f64 {
 
 constexpr int TS = 128;  // samples per tile
 constexpr int NT = 128;  // threads per CTA
-#ifndef F64_G
-#define F64_G 64
-#define F64_C 3
-#endif
-constexpr int G = F64_G;    // y-indices per group
+constexpr int G = 32;    // y-indices per group
 constexpr int SB = 32;   // y-indices per staged block
 constexpr int KC = 8;    // y-indices per chunk of the sweep
-constexpr int NST = 4;   // stages of the sweep's ring
+constexpr int NST = 3;   // stages of the sweep's ring
 
 using Params = simt::SimtParams<double>;
 
+struct Stage {
+  pol::Staged<double> sg;
+  double tri[SB / 8][8][8];  // [sub-block][k][j] = U[l0 + k, target of step k + j]
+  uint32_t sob[SB][dbgz::kSobolRow];
+};
 struct Smem {
   union {
     double S[4][G][32];  // [warp][target, later y-index][sample ^ swizzle]
@@ -52,9 +54,7 @@ struct Smem {
       double U[NST][G][KC + 4];  // row stride 12: conflict-free B fragments
     } ring;
   } u;
-  pol::Staged<double> sg;
-  double tri[SB / 8][8][8];  // [sub-block][k][j] = U[l0 + k, target of step k + j]
-  uint32_t sob[SB][dbgz::kSobolRow];
+  Stage stg[2];
   double red[NT / 32];
   dbgz::NormTab tab;
 };
@@ -85,6 +85,32 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
   const uint64_t base0 = (uint64_t)(P.gen.sobol_first + pl.gen.gen_base + (j - tid));
   const dbgz::SobolLane sob_lane(tid, base0);
   pl.state_begin();
+  // copies of the constants of the block at lb into buffer b (visible after a
+  // wait and a barrier)
+  auto stage = [&](int b, int64_t lb) {
+    Stage &st = sm.stg[b];
+    const int nb = (int)(nY - lb < SB ? nY - lb : SB);
+    pl.stage_async(st.sg, P.tgt, tid, lb, nb);
+#pragma unroll
+    for (int e = tid; e < SB * 8; e += NT) {
+      const int li = e >> 3, jj = e & 7, kk = li & 7;
+      const bool v = kk + jj < 8 && li + jj < nb;
+      pol::cp_async_or_zero<8>(&st.tri[0][0][0] + e, v ? P.U + (lb + li + jj + 1) * d + lb + li : P.U, v);
+    }
+    pol::cp_async_commit();
+    if constexpr (Policy::kSobolTable)
+      if (pl.gen.sobol_staged)
+        dbgz::sobol_stage_block(st.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), base0, pl.sobol_l0(lb),
+                                Policy::kSobolDir, d - 2, nb, tid);
+  };
+  // this sample's place in the workspace row of the next y (a ring of P.ring
+  // rows for banded factors, a multiple of 8)
+  double *yout = Yw + tid;
+  const double *yend = yout + P.ring * TS;
+  stage(0, 0);
+  pol::cp_async_wait_all();
+  __syncthreads();
+  int buf = 0;
 
   for (int64_t g0 = 0; g0 < nY; g0 += G) {
     const int ng = (int)(nY - g0 < (int64_t)G ? nY - g0 : (int64_t)G);
@@ -97,16 +123,19 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
       for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
         for (int ni = 0; ni < G / 8; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
-      const int nch = (int)(g0 / KC);
-      auto issue = [&](int ch) {
-        if (ch < nch) {
-          const int st = ch & (NST - 1);
-          const int64_t l0 = (int64_t)ch * KC;
+      const int64_t k0 = P.band > 0 && g0 + 1 > P.band ? (g0 + 1 - P.band) / KC * KC : 0;
+      const int nch = (int)((g0 - k0) / KC);
+      int64_t yrow = P.band > 0 ? k0 % P.ring : 0;
+      int is = 0, ich = 0;  // stage and number of the next chunk to issue
+      auto issue = [&]() {
+        if (ich < nch) {
+          const int st = is;
+          const int64_t l0 = k0 + (int64_t)ich * KC;
 #pragma unroll
           for (int e = 0; e < KC * 16 / 32; ++e) {
             const int pc = lane + 32 * e, kk = pc >> 4, row = 2 * (pc & 15);
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.u.ring.Y[st][warp][0][0] + swz(kk, row));
-            const double *src = Yw + (l0 + kk) * TS + 32 * warp + row;
+            const double *src = Yw + (yrow + kk) * TS + 32 * warp + row;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
           }
 #pragma unroll
@@ -117,18 +146,23 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
               pol::cp_async_or_zero<8>(&sm.u.ring.U[st][t][kk], v ? P.U + (g0 + 1 + t) * d + l0 + kk : P.U, v);
             }
           }
+          yrow = yrow + KC == P.ring ? 0 : yrow + KC;
         }
         pol::cp_async_commit();
+        ++ich;
+        is = is + 1 == NST ? 0 : is + 1;
       };
-      __syncthreads();  // the ring lies in the S buffer: every warp is done with the last group
+      // (the ring lies in the S buffer: every warp has passed the block
+      // barrier of the last group)
 #pragma unroll
-      for (int ch = 0; ch < NST - 1; ++ch) issue(ch);
+      for (int ch = 0; ch < NST - 1; ++ch) issue();
+      int rs = 0;
       for (int ch = 0; ch < nch; ++ch) {
         asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
         __syncthreads();  // chunk ch has landed for all; the stage of chunk ch - 1 is free
-        issue(ch + NST - 1);
-        const double *Ys = &sm.u.ring.Y[ch & (NST - 1)][warp][0][0];
-        const double(*Us)[KC + 4] = sm.u.ring.U[ch & (NST - 1)];
+        issue();
+        const double *Ys = &sm.u.ring.Y[rs][warp][0][0];
+        const double(*Us)[KC + 4] = sm.u.ring.U[rs];
 #pragma unroll
         for (int k4 = 0; k4 < KC / 4; ++k4) {
           double av[4];
@@ -142,6 +176,7 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
               for (int mi = 0; mi < 4; ++mi) dmma(acc[mi][ni][0], acc[mi][ni][1], av[mi], bv);
             }
         }
+        rs = rs + 1 == NST ? 0 : rs + 1;
       }
       __syncthreads();  // the ring is read: S may be written
 #pragma unroll
@@ -159,25 +194,14 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
     for (int b0 = 0; b0 < ng; b0 += SB) {
       const int nb = ng - b0 < SB ? ng - b0 : SB;
       const int64_t lb = g0 + b0;
-      __syncthreads();  // the last block's staging is read
-      pl.stage(sm.sg, P.tgt, tid, lb, nb);
-#pragma unroll
-      for (int e = tid; e < SB * 8; e += NT) {
-        const int li = e >> 3, jj = e & 7, kk = li & 7;
-        const bool v = kk + jj < 8 && li + jj < nb;
-        (&sm.tri[0][0][0])[e] = v ? P.U[(lb + li + jj + 1) * d + lb + li] : 0.0;
-      }
-      if constexpr (Policy::kSobolTable)
-        if (pl.gen.sobol_staged)
-          dbgz::sobol_stage_block(sm.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), base0, pl.sobol_l0(lb),
-                                  Policy::kSobolDir, d - 2, nb, tid);
-      __syncthreads();
+      if (lb + SB < nY) stage(buf ^ 1, lb + SB);
+      const Stage &st = sm.stg[buf];
       // the tent-transformed point of step li, formed one step ahead
       auto point = [&](int li) -> double {
         uint32_t xs = 0u;
         if constexpr (Policy::kSobolTable)
-          if (pl.gen.sobol_staged) xs = sob_lane.at(sm.sob, li);
-        return pl.point(sm.sg, li, lb + li, xs);
+          if (pl.gen.sobol_staged) xs = sob_lane.at(st.sob, li);
+        return pl.point(st.sg, li, lb + li, xs);
       };
       double w = point(0);
       for (int i0 = 0; i0 < nb; i0 += 8) {
@@ -218,13 +242,13 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
         for (int k = 0; k < nv; ++k) {
           const int li = i0 + k;
           const int64_t l = lb + li;
-          const double2 *tr = reinterpret_cast<const double2 *>(&sm.tri[i0 >> 3][k][0]);
+          const double2 *tr = reinterpret_cast<const double2 *>(&st.tri[i0 >> 3][k][0]);
           const double2 t0 = tr[0], t1 = tr[1], t2 = tr[2], t3 = tr[3];
           const double wn = point(li + 1 < nb ? li + 1 : li);
-          const double y = pl.emit_next(sm.sg, li, l, w);
+          const double y = pl.emit_next(st.sg, li, l, w);
           w = wn;
           S[swz(q8 + k, lane)] = y;
-          if (keep) Yw[l * TS + tid] = y;
+          if (keep) yout[k * TS] = y;
           const double s0 = fma(y, t0.x, s[0]);
           s[0] = fma(y, t0.y, s[1]);
           s[1] = fma(y, t1.x, s[2]);
@@ -233,11 +257,17 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
           s[4] = fma(y, t2.y, s[5]);
           s[5] = fma(y, t3.x, s[6]);
           s[6] = fma(y, t3.y, s[7]);
-          pl.consume(sm.sg, s0, li, l);
+          pl.consume(st.sg, s0, li, l);
         }
         // a partial sub-block (the problem's last) leaves unused rows: no later mma reads them
+        yout += 8 * TS;
+        if (yout == yend) yout -= P.ring * TS;
         __syncwarp();
       }
+      // the next block's constants have landed, and this block's are read
+      pol::cp_async_wait_all();
+      __syncthreads();
+      buf ^= 1;
     }
   }
   // ---- per-tile end and sum of p (fixed order) ----
@@ -251,7 +281,7 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
 }
 
 template <typename Policy>
-__global__ void __launch_bounds__(NT, F64_C) k_genz_f64(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(NT, 4) k_genz_f64(const __grid_constant__ Params P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
   dbgz::norm_tab_load(sm.tab, threadIdx.x, NT);
@@ -263,7 +293,7 @@ __global__ void __launch_bounds__(NT, F64_C) k_genz_f64(const __grid_constant__ 
 // Many problems in one launch, work items from a global counter (as
 // simt::k_genz_simt_batch).
 template <typename Policy>
-__global__ void __launch_bounds__(NT, F64_C)
+__global__ void __launch_bounds__(NT, 4)
     k_genz_f64_batch(const Params *params, const simt::BatchItem *items, int64_t n_items, unsigned long long *counter,
                      double *yws, int64_t Dp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -41,6 +41,12 @@ int launch_simt(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   P.n_tiles = n_tiles;
   P.tile0 = pa.tile0;
   P.Dp = ((d - 1 + G - 1) / G) * G;
+  if (sizeof(T) == 8 && p->structure == DBGZ_STRUCTURE_SPARSE) {
+    // banded: a ring of the y's that the targets of a group reach
+    P.band = p->bandwidth;
+    P.Dp = (P.band + 7) / 8 * 8 + 8 + f64::G;
+  }
+  P.ring = P.Dp;
   P.gen.qmc_type = pa.qmc_type;
   P.gen.n_bits = pa.n_bits;
   P.gen.gen_base = pa.gen_base;
@@ -56,9 +62,10 @@ int launch_simt(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   P.c1 = pa.c1;
   P.dc1 = pa.dc1;
   P.up1 = 1.0 - pa.c1 - pa.dc1;
-  P.cdf_form = pa.cdf_form;
+  P.cdf_form = p->structure == DBGZ_STRUCTURE_SPARSE ? DBGZ_CDF_ERF : pa.cdf_form;  // (src/qmc.jl:618-718)
   P.partials = partials;
   const bool adj = pa.kind == kLoopAdjoint;
+  if (adj && !p->Ub.p) DBGZ_TRY(dbgz_make_Ub(p));
   if (sizeof(T) == 8) {
     P.U = (const T *)(adj ? p->Ub.p : p->U.p);
     P.tgt = (const typename TgtOf<T>::type *)p->tgt64.p;

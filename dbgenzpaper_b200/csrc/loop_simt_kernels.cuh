@@ -28,6 +28,9 @@ struct TgtOf<float> {
 template <typename T>
 struct SimtParams {
   int64_t d, m, n_reps, tiles_per_shift, n_tiles, Dp;
+  // FP64 loop: band > 0: U[l, t] = 0 for t - l > band; ring: rows of a
+  // workspace slot that hold y's (Dp, or a ring for a band; a multiple of 8)
+  int64_t band, ring;
   int64_t tile0;  // tiles [tile0, n_tiles) of the pass
   dbgz::GenParams gen;
   const T *U;  // d x d col-major coefficient array (policies.cuh)

@@ -315,8 +315,11 @@ static int launch_sparse(dbgz_problem *p, const PassArgs &pa, double *partials, 
   P.gen.gen_base = pa.gen_base;
   P.gen.gen_base_dev = pa.gen_base_dev;
   P.gen.sobol_first = pa.sobol_first;
-  // staged Sobol integers
-  P.gen.sobol_staged = pa.qmc_type == DBGZ_QMC_SOBOL;
+  // staged Sobol integers; not in the FP32 pass that keeps its state (measured
+  // on the banded d = 10^4, bandwidth 64 workload at 2^14 x 10 Sobol points: the
+  // gradient call 125.1 ms without, 136.9 ms with them)
+  P.gen.sobol_staged =
+      pa.qmc_type == DBGZ_QMC_SOBOL && !(sizeof(T) == 4 && pa.kind == kLoopForwardStore);
   P.gen.q = (const double *)p->q.p;
   P.gen.shift64 = (const double *)p->shifts.p;
   P.gen.shift32 = (const float *)p->shifts32.p;
@@ -409,8 +412,19 @@ static int launch_sparse_gen(dbgz_problem *p, const PassArgs &pa, double *partia
   return launch_sparse_kind<T, DBGZ_QMC_RICHTMYER>(p, pa, partials, n_tiles);
 }
 
+// Whether the problem runs in the loops that treat the band as dense
+// (loop_f64_kernels.cuh, loop_w32_kernels.cuh) rather than in the CSC loop.
+bool dbgz_band_loop(dbgz_problem *p, int precision) {
+  static const char *e = getenv("W32_BAND");
+  return p->bandwidth <= (e ? atoi(e) : 100000);
+}
+
 int dbgz_loop_sparse(dbgz_problem *p, const PassArgs &pa, int precision, double *partials, int64_t n_tiles) {
   if (!p->csc_colptr.p) DBGZ_TRY(dbgz_build_csc(p));
+  const bool segments = pa.i_begin != 0 || pa.i_end >= 0 || pa.ck_save || pa.ck_load || pa.store_p;
+  if (!segments && dbgz_band_loop(p, precision))
+    return precision == DBGZ_PREC_FP64 ? dbgz_loop_simt(p, pa, precision, partials, n_tiles)
+                                       : dbgz_loop_w32_band(p, pa, partials, n_tiles);
   if (pa.kind == kLoopAdjoint && !p->cscb_colptr.p) {
     if (!p->Ub.p) DBGZ_TRY(dbgz_make_Ub(p));
     int64_t nnz = 0, bw = 1;

@@ -178,7 +178,7 @@ extern "C" int dbgz_pnorm_pass_noalloc(int64_t d, const double *U, const double 
   P.n_reps = n_reps;
   P.tiles_per_shift = tps;
   P.n_tiles = n_tiles;
-  P.Dp = Dp;
+  P.Dp = P.ring = Dp;
   P.gen.qmc_type = DBGZ_QMC_RICHTMYER;
   P.gen.n_bits = 32;
   P.gen.gen_base = n_base;

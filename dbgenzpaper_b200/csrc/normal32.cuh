@@ -25,8 +25,28 @@ __device__ __forceinline__ float exp2_sfu(float z) {
   return e;
 }
 
+// The SFU's reciprocal, base-2 logarithm and reciprocal square root in the
+// forms that flush subnormals: their arguments here are normal (or 0 where
+// the result is not used), and the plain forms (__fdividef, __logf, rsqrtf)
+// spend two to five instructions each on scaling subnormal arguments.
+__device__ __forceinline__ float rcp_sfu(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float log2_sfu(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_sfu(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 __device__ __forceinline__ float tail_mass_f32(float x) {
-  const float t = __fdividef(1.0f, fmaf(0.5f, x, 1.0f));
+  const float t = rcp_sfu(fmaf(0.5f, x, 1.0f));
   float p = 1.6112529716e-01f;
   p = fmaf(p, t, -7.6098558876e-01f);
   p = fmaf(p, t, 1.3262850294e+00f);
@@ -52,7 +72,7 @@ __device__ __forceinline__ float tail_mass_f32(float x) {
 // (maximum 9.4e-8 and 5.8e-8); both are evaluated and the region selected, so
 // the code has no branch.  Relative error in FP32 below 4e-7 for p >= 2.2e-16.
 __device__ __forceinline__ float phi_inv_lower_f32(float p) {
-  const float w = -__logf(4.0f * p * (1.0f - p));
+  const float w = log2_sfu(4.0f * p * (1.0f - p)) * -0.69314718056f;
   const float x = fmaf(-2.0f, p, 1.0f);
   const float tc = w - 2.5f;
   float pc = 2.854775242e-08f;
@@ -64,7 +84,7 @@ __device__ __forceinline__ float phi_inv_lower_f32(float p) {
   pc = fmaf(pc, tc, -4.177708101e-03f);
   pc = fmaf(pc, tc, 2.466407258e-01f);
   pc = fmaf(pc, tc, 1.501409422e+00f);
-  const float ts = w * rsqrtf(w) - 4.0f;
+  const float ts = w * rsqrt_sfu(w) - 4.0f;
   float pt = 8.193106379e-07f;
   pt = fmaf(pt, ts, -1.490730122e-06f);
   pt = fmaf(pt, ts, -6.624017282e-06f);

@@ -110,6 +110,17 @@ __device__ __forceinline__ void cp_async_or_zero(void *dst_smem, const void *src
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// a target's constants (16 bytes in FP32, three doubles in FP64)
+__device__ __forceinline__ void copy_target(TargetParams32 &dst, const TargetParams32 &src) {
+  static_assert(sizeof(TargetParams32) == 16, "one 16-byte copy");
+  cp_async_or_zero<16>(&dst, &src, true);
+}
+__device__ __forceinline__ void copy_target(TargetParams64 &dst, const TargetParams64 &src) {
+  cp_async_or_zero<8>(&dst.a, &src.a, true);
+  cp_async_or_zero<8>(&dst.b, &src.b, true);
+  cp_async_or_zero<8>(&dst.inv_u, &src.inv_u, true);
+}
+
 template <typename T>
 __device__ __forceinline__ T shift_at(const dbgz::GenParams &g, int64_t idx);
 template <>
@@ -142,11 +153,8 @@ struct Forward {
   // consume_deferred + tail_repair available (the FP32 steps): the loop may
   // run a chunk of steps without the same-tail branch
   static constexpr bool kDeferTail = std::is_same<T, float>::value;
-  // takes staged Sobol integers (GenParams::sobol_staged); not in the FP32 pass
-  // that keeps the state for the adjoint (measured on the banded d = 10^4,
-  // bandwidth 64 workload at 2^14 x 10 Sobol points:
-  // the gradient call 125.1 ms without, 136.9 ms with them)
-  static constexpr bool kSobolTable = GEN == DBGZ_QMC_SOBOL && (!STORE || std::is_same<T, double>::value);
+  // takes staged Sobol integers (GenParams::sobol_staged)
+  static constexpr bool kSobolTable = GEN == DBGZ_QMC_SOBOL;
   // the QMC dimension of step li of a block: lbase + li
   static constexpr int kSobolDir = 1;
   __device__ __forceinline__ int64_t sobol_l0(int64_t lbase) const { return lbase; }
@@ -157,6 +165,7 @@ struct Forward {
   int64_t j, k, g;  // point index in the pass, shift, global sample index
   int64_t ga0;      // io.at0(g)
   int64_t d;
+  double jd;        // gen.gen_base + j + 1: the lattice point's multiplier
   int cdf_form;
   GradIO<T> io;
 
@@ -174,6 +183,7 @@ struct Forward {
     d = d_;
     k = tile / tiles_per_shift;
     j = (tile - k * tiles_per_shift) * 128 + r;
+    jd = (double)(gen.gen_base + j + 1);
     g = (tile - io_.tile0) * 128 + r;
     cdf_form = cdf_form_;
     io = io_;
@@ -192,37 +202,46 @@ struct Forward {
       sg.shv[r] = shift_at<T>(gen, k * (d - 1) + lbase + r);
     }
   }
-  // stage() by asynchronous copies (FP32 staging only): the caller commits
-  // and waits
+  // stage() by asynchronous copies: the caller commits and waits
   __device__ __forceinline__ void stage_async(Staged<T> &sg, const typename TgtT<T>::type *tgt, int r,
                                               int64_t lbase, int nval) const {
-    static_assert(sizeof(typename TgtT<T>::type) == 16 && sizeof(T) == 4, "FP32 staging");
     if (r < nval) {
       const int64_t si = k * (d - 1) + lbase + r;
-      cp_async_or_zero<16>(&sg.tg[r], &tgt[lbase + r + 1], true);
+      copy_target(sg.tg[r], tgt[lbase + r + 1]);
       cp_async_or_zero<8>(&sg.qv[r], gen.q ? (const void *)(gen.q + lbase + r) : (const void *)tgt, gen.q != nullptr);
-      cp_async_or_zero<4>(&sg.shv[r], gen.shift32 ? (const void *)(gen.shift32 + si) : (const void *)tgt,
+      if constexpr (sizeof(T) == 8)
+        cp_async_or_zero<8>(&sg.shv[r], gen.shift64 ? (const void *)(gen.shift64 + si) : (const void *)tgt,
+                            gen.shift64 != nullptr);
+      else
+        cp_async_or_zero<4>(&sg.shv[r], gen.shift32 ? (const void *)(gen.shift32 + si) : (const void *)tgt,
                           gen.shift32 != nullptr);
     }
   }
   // xs: the Sobol integer of this point in dimension l when the loop stages
   // them (GenParams::sobol_staged), else unused
   __device__ __forceinline__ T emit(const Staged<T> &sg, int li, int64_t l, uint32_t xs = 0u) {
-    const T y = st.template quantile<!STORE>(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs);
+    const T y = st.template quantile<!STORE>(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs, jd);
     if (STORE) __stcs(io.y + ga0 + l * io.stride(), y);
     return y;
   }
-  // rolled form (FP64 loop): point() gives a step's tent-transformed point,
-  // formed one step early, emit_next the step's value from it; a policy that
-  // reads stored state keeps the next step's in registers
+  // point() gives a step's tent-transformed point, emit_at its value from it: a
+  // loop forms the points ahead of the steps.  Rolled form (FP64 loop): a
+  // policy that reads stored state keeps the next step's in registers.
+  using Point = typename Step::Tent;
   __device__ __forceinline__ void state_begin() {}
-  __device__ __forceinline__ T point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
-    return Step::tent(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs);
+  __device__ __forceinline__ Point point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
+    return Step::template tent<!STORE>(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs, jd);
   }
-  __device__ __forceinline__ T emit_next(const Staged<T> &, int, int64_t l, T w) {
+  __device__ __forceinline__ T emit_next(const Staged<T> &, int, int64_t l, Point w) {
     const T y = st.quantile_w(w);
     if (STORE) __stcs(io.y + ga0 + l * io.stride(), y);
     return y;
+  }
+  __device__ __forceinline__ T emit_k_at(const Staged<T> &sg, int li, int64_t l, int, Point w) {
+    return emit_next(sg, li, l, w);
+  }
+  __device__ __forceinline__ T emit_k_fast_at(const Staged<T> &sg, int li, int64_t l, int, Point w) {
+    return emit_next(sg, li, l, w);
   }
   // chunked form (8 steps whose per-sample inputs may be loaded up front)
   __device__ __forceinline__ void chunk_begin(int64_t, int) {}
@@ -370,15 +389,17 @@ struct Adjoint {
 
   __device__ __forceinline__ void stage_async(Staged<T> &sg, const typename TgtT<T>::type *tgt, int r,
                                               int64_t lbase, int nval) const {
-    static_assert(sizeof(typename TgtT<T>::type) == 16 && sizeof(T) == 4, "FP32 staging");
     if (r < nval) {
       const int64_t t = d - 1 - (lbase + r);
       const bool has_u = t <= d - 2;
       const int64_t si = k * (d - 1) + t;
-      cp_async_or_zero<16>(&sg.tg[r], &tgt[t], true);
-      const bool vq = has_u && gen.q, vs = has_u && gen.shift32;
+      copy_target(sg.tg[r], tgt[t]);
+      const bool vq = has_u && gen.q, vs = has_u && (sizeof(T) == 8 ? gen.shift64 != nullptr : gen.shift32 != nullptr);
       cp_async_or_zero<8>(&sg.qv[r], vq ? (const void *)(gen.q + t) : (const void *)tgt, vq);
-      cp_async_or_zero<4>(&sg.shv[r], vs ? (const void *)(gen.shift32 + si) : (const void *)tgt, vs);
+      if constexpr (sizeof(T) == 8)
+        cp_async_or_zero<8>(&sg.shv[r], vs ? (const void *)(gen.shift64 + si) : (const void *)tgt, vs);
+      else
+        cp_async_or_zero<4>(&sg.shv[r], vs ? (const void *)(gen.shift32 + si) : (const void *)tgt, vs);
     }
   }
 
@@ -588,9 +609,12 @@ struct Adjoint {
     nx_dc = io.dc[ga0 + t * io.stride()];
   }
   __device__ __forceinline__ void state_begin() { state_load(d - 1); }
-  __device__ __forceinline__ T point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
+  using Point = T;
+  __device__ __forceinline__ Point point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
     const int64_t t = d - 1 - l;
-    return t <= d - 2 ? (T)point_w(sg, li, t, xs, gen.sobol_staged != 0) : T(0);
+    const bool has_u = t <= d - 2;
+    if constexpr (sizeof(T) == 4) return has_u ? point_w32(sg, li, t, xs, gen.sobol_staged != 0) : 0.0f;
+    else return has_u ? point_w(sg, li, t, xs, gen.sobol_staged != 0) : 0.0;
   }
   __device__ __forceinline__ T emit_next(const Staged<T> &sg, int li, int64_t l, T w) {
     const T y = nx_y, s = nx_s, dc = nx_dc;
@@ -635,10 +659,14 @@ struct Adjoint {
   __device__ __forceinline__ T emit_k_fast(const Staged<T> &sg, int li, int64_t l, int kk, uint32_t xs) {
     const int64_t t = d - 1 - l;
     const bool has_u = t <= d - 2;
-    const float w = has_u ? point_w32(sg, li, t, xs, gen.sobol_staged != 0) : 0.0f;
+    return emit_k_fast_at(sg, li, l, kk, has_u ? point_w32(sg, li, t, xs, gen.sobol_staged != 0) : 0.0f);
+  }
+  __device__ __forceinline__ T emit_k_fast_at(const Staged<T> &sg, int li, int64_t l, int kk, Point w) {
+    const int64_t t = d - 1 - l;
+    const bool has_u = t <= d - 2;
     float fa, fb, fu;
-    const float sb = variable32(sg.tg[li], w, has_u, (float)pre_y[kk], (float)pre_s[kk], (float)pre_dc[kk], true, fa,
-                                fb, fu);
+    const float sb = variable32(sg.tg[li], (float)w, has_u, (float)pre_y[kk], (float)pre_s[kk], (float)pre_dc[kk],
+                                true, fa, fb, fu);
     const float wa = wrel * fa, wb = wrel * fb, wu = wrel * fu;
     // one test for the four: an infinite or NaN term makes the sum so (a
     // finite sum that overflows only costs a redo)
