@@ -129,11 +129,12 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
     Wb = p->bandwidth_b + 1;
   }
   const int64_t ck_rows = seg + 2;  // rows of a segment's recomputed state
+  const int64_t ck_slots = K > 1 ? K - 1 : 1;  // checkpoints held (one unused slot when there is one segment)
   // samples per chunk: as many whole tiles as the context's state budget
   // allows (forward-store, adjoint, reduction and the dU GEMM run per chunk;
   // the GEMM accumulates across chunks)
   const size_t state_per_sample =
-      ckpt ? (size_t)(K - 1) * (Wf * esz + 32) + (Wb * esz + 32) + 3 * ck_rows * esz
+      ckpt ? (size_t)ck_slots * (Wf * esz + 32) + (Wb * esz + 32) + 3 * ck_rows * esz
            : (sparse ? 3 : 4) * esz * (size_t)d;
   const size_t tile_bytes = 128 * (state_per_sample + 8) + 3 * 4 * 8 * (size_t)d;
   const int64_t chunk =
@@ -144,7 +145,8 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   // one allocation: y, s, dc (+ p sbar on the dense path; a segment's rows
   // with checkpoints), checkpoints, p, 3 partial arrays, sums, dU
   const size_t arr = esz * (size_t)(ckpt ? ck_rows : d) * N;
-  const size_t ck_bytes = ckpt ? (size_t)(K - 1) * ((size_t)Wf * esz + 32) * N + ((size_t)Wb * esz + 32) * N : 0;
+  const size_t ck_bytes =
+      ckpt ? (size_t)ck_slots * ((size_t)Wf * esz + 32) * N + ((size_t)Wb * esz + 32) * N + 4 * 256 : 0;
   const size_t part = sizeof(double) * (size_t)chunk * 4 * d;
   const size_t total = (sparse ? 3 : 4) * arr + ck_bytes + 8 * 256 + 8 * (size_t)N + 3 * part +
                        3 * 8 * (size_t)d * (kRedChunks + 1) +
@@ -165,8 +167,8 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   ga.sbar = sparse ? nullptr : take(arr);
   // checkpoints: slots 0..K-2 (forward: ring [Wf][N], state [4][N]) and the
   // adjoint's carry (ring [Wb][N], state [4][N])
-  char *ck_ring = ckpt ? take((size_t)(K > 1 ? K - 1 : 1) * Wf * esz * N) : nullptr;
-  double *ck_state = ckpt ? (double *)take((size_t)(K > 1 ? K - 1 : 1) * 32 * N) : nullptr;
+  char *ck_ring = ckpt ? take((size_t)ck_slots * Wf * esz * N) : nullptr;
+  double *ck_state = ckpt ? (double *)take((size_t)ck_slots * 32 * N) : nullptr;
   char *cr_ring = ckpt ? take((size_t)Wb * esz * N) : nullptr;
   double *cr_state = ckpt ? (double *)take((size_t)32 * N) : nullptr;
   ga.p = (double *)take(8 * (size_t)N);
