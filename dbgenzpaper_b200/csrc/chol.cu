@@ -21,6 +21,7 @@
 #include "internal.cuh"
 #include "detmath.h"
 #include "chol_dev.cuh"
+#include <algorithm>
 #include <cfloat>
 
 namespace {
@@ -90,15 +91,55 @@ k_genz_block_smem(double *M, int64_t n, double *a, double *b, double *dvec, doub
   cholk::genz_block_smem(M, n, a, b, dvec, svec, perm, i0, i1, ii1, eps0_ptr, rank, genz_sh);
 }
 
-// The same with the block's factor entries on chip (panels of up to
-// cholk::kOnchipSlots candidates, blocks of up to cholk::kOnchipPiv pivots):
-// the slot warps and the y_i warp.
-constexpr int kOnchipThreads = cholk::kOnchipSlots + 32;
-__global__ void __launch_bounds__(kOnchipThreads)
-k_genz_block_onchip(double *M, int64_t n, double *a, double *b, double *dvec, double *svec, int64_t *perm,
-                    int64_t i0, int64_t i1, int64_t ii1, const double *eps0_ptr, int64_t *rank) {
-  extern __shared__ double genz_sh[];
-  cholk::genz_block_onchip(M, n, a, b, dvec, svec, perm, i0, i1, ii1, eps0_ptr, rank, genz_sh);
+// The same by a cluster of CTAs (panels of up to cholk::kPivPanel candidates,
+// blocks of up to cholk::kPivMax pivots); M stays as it is until the two
+// kernels below permute it and write the block's rows.
+__global__ void __launch_bounds__(cholk::kPivThreads)
+k_genz_block_cluster(const double *M, int64_t n, double *a, double *b, double *dvec, double *svec, int64_t *perm,
+                     int64_t i0, int64_t i1, int64_t ii1, const double *eps0_ptr, int64_t *rank, cholk::PivOut out) {
+  __shared__ cholk::PivSmem sm;
+  cholk::genz_block_cluster(M, n, a, b, dvec, svec, perm, i0, i1, ii1, eps0_ptr, rank, out, sm);
+}
+// The block's swaps as one permutation of the panel's positions: rows and
+// columns of the panel, the panel's rows in the columns after it, and the
+// panel's columns in the rows outside it; the block's completed pivots put
+// their factor entries into their row and (mirrored) column.
+// T1[c * n + r]: column i0 + c; T2[k * len + p]: row i0 + p of column ii1 + 1 + k.
+__global__ void k_genz_gather(const double *M, int64_t n, int64_t i0, int64_t ii1, cholk::PivOut o, double *T1,
+                              double *T2) {
+  const int nb = *o.done;
+  if (nb < 0) return;
+  const int64_t len = ii1 - i0 + 1, n1 = len * n, n2 = (n - 1 - ii1) * len;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n1 + n2; e += (int64_t)gridDim.x * blockDim.x) {
+    if (e < n1) {
+      const int64_t c = e / n, r = e - c * n, pr = r - i0;
+      double v;
+      if (pr >= 0 && pr < len) {
+        const int64_t lo = pr < c ? pr : c, hi = pr < c ? c : pr;
+        if (lo < nb) v = lo == hi ? o.fd[lo] : o.f[lo * cholk::kPivPanel + o.ord[hi]];
+        else v = M[(i0 + o.ord[c]) * n + i0 + o.ord[pr]];
+      } else {
+        v = M[(i0 + o.ord[c]) * n + r];
+      }
+      T1[e] = v;
+    } else {
+      const int64_t q = e - n1, k = q / len, p = q - k * len;
+      T2[q] = M[(ii1 + 1 + k) * n + i0 + o.ord[p]];
+    }
+  }
+}
+__global__ void k_genz_scatter(double *M, int64_t n, int64_t i0, int64_t ii1, cholk::PivOut o, const double *T1,
+                               const double *T2) {
+  if (*o.done < 0) return;
+  const int64_t len = ii1 - i0 + 1, n1 = len * n, n2 = (n - 1 - ii1) * len;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n1 + n2; e += (int64_t)gridDim.x * blockDim.x) {
+    if (e < n1) {
+      M[i0 * n + e] = T1[e];
+    } else {
+      const int64_t q = e - n1, k = q / len, p = q - k * len;
+      M[(ii1 + 1 + k) * n + i0 + p] = T2[q];
+    }
+  }
 }
 
 // One bs1 block of cholesky_rowmax! (src/cholesky.jl:290-357), one CTA: the
@@ -447,6 +488,43 @@ int scale_correlation(dbgz_ctx *ctx, double *M, int64_t n, double *a, double *b,
   return DBGZ_OK;
 }
 
+// One Genz block: pivots, then the permutation of M.  work: scratch of
+// genz_cluster_bytes(n, panel); its end holds the pivots' records.
+size_t genz_cluster_bytes(int64_t n, int64_t panel) {
+  return sizeof(double) * ((size_t)2 * panel * n + (size_t)cholk::kPivMax * (cholk::kPivPanel + 1)) +
+         sizeof(int) * (cholk::kPivPanel + 4) + 512;
+}
+int launch_genz_cluster(dbgz_ctx *ctx, double *M, int64_t n, double *a, double *b, double *dvec, double *svec,
+                        int64_t *perm, int64_t i0, int64_t i1, int64_t ii1, const double *eps0, int64_t *rank,
+                        DevBuf &work) {
+  const int64_t len = ii1 - i0 + 1;
+  double *T1 = (double *)work.p, *T2 = T1 + len * n;
+  cholk::PivOut o;
+  o.f = (double *)work.p + work.bytes / 8 - cholk::kPivMax * (cholk::kPivPanel + 1) - (cholk::kPivPanel + 4) / 2;
+  o.fd = o.f + cholk::kPivMax * cholk::kPivPanel;
+  o.ord = (int *)(o.fd + cholk::kPivMax);
+  o.done = o.ord + cholk::kPivPanel;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((len + cholk::kPivSlots - 1) / cholk::kPivSlots));
+  cfg.blockDim = dim3(cholk::kPivThreads);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cfg.gridDim.x;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  DBGZ_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, k_genz_block_cluster, (const double *)M, n, a, b, dvec, svec, perm, i0,
+                                        i1, ii1, eps0, rank, o));
+  const int64_t el = len * n + (n - 1 - ii1) * len;
+  const unsigned gr = (unsigned)std::min<int64_t>((el + 255) / 256, 4096);
+  k_genz_gather<<<gr, 256, 0, ctx->stream>>>(M, n, i0, ii1, o, T1, T2);
+  k_genz_scatter<<<gr, 256, 0, ctx->stream>>>(M, n, i0, ii1, o, T1, T2);
+  dbgz_count_launch(ctx, 3);
+  DBGZ_CUDA_TRY(ctx, cudaGetLastError());
+  return DBGZ_OK;
+}
+
 }  // namespace
 
 int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b, int64_t bs1,
@@ -456,6 +534,11 @@ int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b
     return dbgz_fail(ctx, DBGZ_ERR_INVALID_ARGUMENT, "block sizes must be positive");
   DevBuf work;
   DBGZ_TRY(dbgz_ensure(ctx, work, sizeof(double) * (3 * n + 2) + sizeof(int64_t) * 2));
+  DevBuf work2;  // the permutation's scratch, for the widest panel
+  if (int rc2 = dbgz_ensure(ctx, work2, genz_cluster_bytes(n, std::min(std::min(n, bs2), (int64_t)cholk::kPivPanel)))) {
+    dbgz_release(work);
+    return rc2;
+  }
   double *dvec = (double *)work.p, *svec = dvec + n, *ovec = svec + n, *eps0 = ovec + n;
   int64_t *rank = (int64_t *)(eps0 + 2);
   cudaStream_t st = ctx->stream;
@@ -463,7 +546,7 @@ int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b
   k_diag_absmax<<<1, 1024, 0, st>>>(M, n, eps0);
   dbgz_count_launch(ctx);
   int st_ = scale_correlation(ctx, M, n, a, b, scale, 1);
-  if (st_) { dbgz_release(work); return st_; }
+  if (st_) { dbgz_release(work); dbgz_release(work2); return st_; }
   {
     std::vector<int64_t> id(n);
     for (int64_t i = 0; i < n; ++i) id[i] = i;
@@ -482,15 +565,9 @@ int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b
         for (int64_t i0 = ii0; i0 <= ii1 && rc == DBGZ_OK; i0 += bs1) {
           int64_t i1 = std::min(ii1, i0 + bs1 - 1);
           const int64_t panel = ii1 - i0 + 1;
-          if (panel <= cholk::kOnchipSlots && i1 - i0 + 1 <= cholk::kOnchipPiv) {
-            static bool attr_oc[64] = {};
-            if (ctx->device < 0 || ctx->device >= 64 || !attr_oc[ctx->device]) {
-              cudaFuncSetAttribute(k_genz_block_onchip, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)cholk::genz_block_onchip_bytes(cholk::kOnchipSlots));
-              if (ctx->device >= 0 && ctx->device < 64) attr_oc[ctx->device] = true;
-            }
-            k_genz_block_onchip<<<1, kOnchipThreads, cholk::genz_block_onchip_bytes(panel), st>>>(
-                M, n, a, b, dvec, svec, perm, i0, i1, ii1, eps0, rank);
+          if (panel <= cholk::kPivPanel && i1 - i0 + 1 <= cholk::kPivMax) {
+            rc = launch_genz_cluster(ctx, M, n, a, b, dvec, svec, perm, i0, i1, ii1, eps0, rank, work2);
+            if (rc != DBGZ_OK) break;
           } else if (panel <= kGenzSmemPanel) {
             const size_t sm = cholk::genz_block_smem_bytes(panel);
             static bool attr[64] = {};
@@ -500,10 +577,11 @@ int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b
               if (ctx->device >= 0 && ctx->device < 64) attr[ctx->device] = true;
             }
             k_genz_block_smem<<<1, kStepThreads, sm, st>>>(M, n, a, b, dvec, svec, perm, i0, i1, ii1, eps0, rank);
+            dbgz_count_launch(ctx);
           } else {
             k_genz_block<<<1, kStepThreads, 0, st>>>(M, n, a, b, dvec, svec, ovec, perm, i0, i1, ii1, eps0, rank);
+            dbgz_count_launch(ctx);
           }
-          dbgz_count_launch(ctx);
           if (i1 < ii1) rc = launch_schur(ctx, M, n, i0, i1, i1 + 1, ii1, 1, rank);
         }
         if (ii1 < iii1 && rc == DBGZ_OK) {
@@ -531,6 +609,7 @@ int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b
   }
   cudaStreamSynchronize(st);
   dbgz_release(work);
+  dbgz_release(work2);
   return rc;
 }
 

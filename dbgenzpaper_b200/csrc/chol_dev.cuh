@@ -359,303 +359,234 @@ __device__ __forceinline__ void genz_block_smem(double *M, int64_t n, double *a,
   write_back();
 }
 
-// genz_block_smem with the block's factor entries kept on chip.  The entries
-// m[l, k] of the block's pivots l for every candidate k of the panel, which
-// the row update's dot products read, live in the registers of the
-// candidate's thread (the first kFReg pivots) and in shared memory (the rest),
-// and follow their candidate through the swaps.  Thread t < kOnchipSlots owns
-// panel position i0 + t; it takes the value M[i, k] its update needs while it
-// does its part of the row/column swap, so the pivot chain makes no global
-// read but that one.  A last warp computes y_i (:533-546) while the slot
-// threads run the update's dot products (named barrier 2: y_i ready).  Panels
-// of at most kOnchipSlots positions, blocks of at most kOnchipPiv pivots.  Same
-// operations in the same order as genz_block_dev: the same bits.
-constexpr int kFReg = 16;          // block pivots whose entries live in registers
-constexpr int kOnchipPiv = 64;     // pivots per block at most
-constexpr int kOnchipSlots = 512;  // slot threads; the block has one more warp
-constexpr int kSwapBatch = 2;      // swap indices per memory round trip
-__host__ __device__ inline size_t genz_block_onchip_bytes(int64_t panel_len) {
-  return (size_t)(56 + 8 * (kOnchipPiv - kFReg)) * (size_t)panel_len + 8 * 2 * kFReg;
+// One bs1 block of cholesky_genz! by a cluster of CTAs, 64 candidates each
+// (panels of at most 512 candidates, blocks of at most 64 pivots).  One CTA
+// for all candidates was bound by its FP64 pipe (two erf, two divisions and a
+// square root a candidate and pivot) and by the row and column swaps, 4 n
+// strided accesses of one SM a pivot: 10.7 us a pivot at 512 candidates with
+// two finite bounds.  Here
+//   * two threads a candidate take one bound each; det_erf's two polynomials
+//     run as one chain with the coefficients picked from shared memory (the
+//     shorter one led by zeros: the same bits), so lanes do not diverge;
+//   * a candidate stays in its thread and only its position changes; M is read
+//     where it lies (one coalesced column a pivot, in flight under the dot
+//     products and the y_i) and permuted once per block by the whole GPU
+//     (k_genz_gather, k_genz_scatter in chol.cu);
+//   * each CTA sends its best candidate, factor entries included, to every CTA
+//     of the cluster: one cluster barrier a pivot, after which every CTA takes
+//     the pivot, its root and y_i by itself.
+// Same operations in the same order as genz_block_dev: the same bits.
+constexpr int kPivSlots = 64;     // candidates per CTA
+constexpr int kPivThreads = 128;  // two per candidate
+constexpr int kPivCtas = 8;       // CTAs per cluster at most
+constexpr int kPivMax = 64;       // pivots per block at most
+constexpr int kPivPanel = kPivSlots * kPivCtas;
+
+struct PivRec {
+  unsigned long long key;  // argmin_key of the score, ~0: no candidate
+  unsigned idx, pad;       // position << 16 | slot
+  double m_raw, o, a, b, s;
+  double f[kPivMax];
+};
+struct PivSmem {
+  PivRec rec[2][kPivCtas];
+  double f[kPivMax][kPivSlots];  // m[pivot, candidate]
+  double o[kPivSlots], s[kPivSlots], m[kPivSlots], a[kPivSlots], b[kPivSlots];
+  double fd[kPivMax];
+  double tab[2][29];
+  unsigned long long wk[2][kPivThreads / 32];
+  unsigned wi[2][kPivThreads / 32];
+};
+// What the block leaves for the permutation of M.
+struct PivOut {
+  int *ord;    // [panel] slot at each position
+  double *f;   // [pivot][kPivPanel] factor entries by slot
+  double *fd;  // [pivot] diagonal
+  int *done;   // pivots completed (-1: the block did not run)
+};
+
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, int cta) {
+  uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(cta));
+  return r;
 }
-__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+__device__ __forceinline__ void cluster_store(uint32_t a, unsigned long long v) {
+  asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
 
-__device__ __forceinline__ void genz_block_onchip(double *M, int64_t n, double *a, double *b, double *dvec,
-                                                  double *svec, int64_t *perm, int64_t i0, int64_t i1,
-                                                  int64_t ii1, const double *eps0_ptr, int64_t *rank, double *sh) {
-  __shared__ unsigned long long red_k[32];
-  __shared__ unsigned red_t[32];
-  __shared__ double sh_yi, sh_mij_im;
+// det_erf with its coefficients in tab[0] (|x| < 2.5, padded to 29) and tab[1]
+__device__ __forceinline__ double det_erf_tab(const double (*tab)[29], double x) {
+  const double ax = fabs(x);
+  const bool small = ax < 2.5;
+  const double w = small ? dm_fma(dm_mul(ax, ax), 0x1.47ae147ae147bp-2, -1.0)
+                         : dm_fma(ax, 0x1.2492492492492p-1, -0x1.36db6db6db6dbp+1);
+  const double *c = tab[small ? 0 : 1];
+  double q = c[28];
+#pragma unroll
+  for (int j = 27; j >= 0; --j) q = dm_fma(q, w, c[j]);
+  double r = small ? dm_mul(ax, q) : dm_sub(1.0, q);
+  r = ax < 6.0 ? r : 1.0;
+  r = x < 0 ? -r : r;
+  return x != x ? x : r;
+}
+
+__device__ __forceinline__ void genz_block_cluster(const double *M, int64_t n, double *a, double *b, double *dvec,
+                                                   double *svec, int64_t *perm, int64_t i0, int64_t i1, int64_t ii1,
+                                                   const double *eps0_ptr, int64_t *rank, PivOut out, PivSmem &sm) {
   const double c2 = dm_div(1.0, dm_sqrt(2.0));
   const double is2pi = dm_div(2.0, dm_sqrt(dm_mul(2.0, M_PI)));
   const double eps0 = eps0_ptr[0];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  constexpr int NS = kOnchipSlots, NALL = kOnchipSlots + 32;
-  if (rank[0] < n) return;  // an earlier block already stopped
-  const int64_t len = ii1 - i0 + 1;
-  double *s_d = sh, *s_s = sh + len, *s_a = sh + 2 * len, *s_b = sh + 3 * len, *s_g = sh + 4 * len,
-         *s_o = sh + 5 * len;
-  int64_t *s_p = reinterpret_cast<int64_t *>(sh + 6 * len);
-  double *s_f = sh + 7 * len;                        // [kOnchipPiv - kFReg][len]: pivots kFReg.. of each position
-  double *s_piv = s_f + (kOnchipPiv - kFReg) * len;  // the pivot's register entries
-  double *s_x = s_piv + kFReg;                       // the displaced candidate's register entries
-  for (int64_t k = tid; k < len; k += blockDim.x) {
-    const int64_t g = i0 + k;
-    s_d[k] = 0.0;
-    s_s[k] = svec[g];
-    s_a[k] = a[g];
-    s_b[k] = b[g];
-    s_g[k] = M[g * n + g];
-    s_p[k] = perm[g];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, C = (int)gridDim.x, cid = (int)blockIdx.x;
+  const int sl = tid >> 1, slot = cid * kPivSlots + sl;
+  const bool upper = (tid & 1) == 0;  // this thread's bound: b (even) or a (odd)
+  const int len = (int)(ii1 - i0 + 1);
+  const bool has = slot < len;
+  const int64_t g = i0 + slot;
+  if (rank[0] < n) {  // an earlier block already stopped
+    if (cid == 0 && tid == 0) *out.done = -1;
+    return;
   }
-  __syncthreads();
-  auto write_back = [&]() {
-    __syncthreads();
-    for (int64_t k = tid; k < len; k += blockDim.x) {
-      const int64_t g = i0 + k;
-      dvec[g] = s_d[k];
-      svec[g] = s_s[k];
-      a[g] = s_a[k];
-      b[g] = s_b[k];
-      perm[g] = s_p[k];
-    }
-  };
-  const bool yw = wid == NS / 32;  // the y_i warp
-  const int t = tid;               // this thread's panel position: kk = i0 + t
-  const bool has_slot = !yw && t < len;
-  const int64_t kk = i0 + t;
-  double f[kFReg];                 // m[i0 + u, kk] for u < kFReg
+  if (tid < 58) {
+    const double c_small[21] = DBGZ_ERF_SMALL_TABLE;
+    const double c_mid[29] = DBGZ_ERFC_MID_TABLE;
+    double v = 0.0;
 #pragma unroll
-  for (int u = 0; u < kFReg; ++u) f[u] = 0.0;
-  double mij = 0.0;                // M[i, kk] of the coming update
-  // pivot score of this position for step i (:500-512), and the warp's minimum
-  auto score = [&](int64_t i) {
+    for (int j = 0; j < 29; ++j) {
+      if (tid == j && j < 21) v = c_small[j < 21 ? j : 0];
+      if (tid == 29 + j) v = c_mid[j];
+    }
+    (&sm.tab[0][0])[tid] = v;
+  }
+  const double gd = has ? M[g * n + g] : 0.0, av = has ? a[g] : 0.0, bv = has ? b[g] : 0.0;
+  const int64_t pv = has ? perm[g] : 0;
+  const double xb = upper ? bv : av;
+  double ds = 0.0, s = has ? svec[g] : 0.0;
+  int pos = slot;
+  if (upper) {
+    sm.a[sl] = av;
+    sm.b[sl] = bv;
+  }
+  const int np = (int)(i1 - i0 + 1);
+  int done = np;
+  cluster_sync_all();  // every CTA's shared memory is up (and this one's tables)
+#pragma unroll 1
+  for (int u = 0; u < np; ++u) {
+    const int par = u & 1;
+    // pivot scores (:500-512) and the CTA's least (argmin :514)
+    const double m_raw = dm_sub(gd, ds);
+    const double m_kk = m_raw < 0 ? 0.0 : dm_sqrt(m_raw);
+    const double e = det_erf_tab(sm.tab, dm_mul(dm_div(dm_sub(xb, s), m_kk), c2));
+    const double eo = __shfl_xor_sync(0xffffffffu, e, 1);
+    const double o = upper ? dm_sub(e, eo) : dm_sub(eo, e);
     unsigned long long key = ~0ull;
-    unsigned pos = ~0u;
-    if (has_slot && kk >= i) {
-      double m_kk = dm_sub(s_g[t], s_d[t]);
-      m_kk = m_kk < 0 ? 0.0 : dm_sqrt(m_kk);
-      double a_k = dm_mul(dm_div(dm_sub(s_a[t], s_s[t]), m_kk), c2);
-      double b_k = dm_mul(dm_div(dm_sub(s_b[t], s_s[t]), m_kk), c2);
-      double o = dm_sub(det_erf(b_k), det_erf(a_k));
-      s_o[t] = o;
+    unsigned idx = ~0u;
+    if (has && pos >= u && upper) {
       key = argmin_key(o);
-      pos = (unsigned)t;
+      idx = ((unsigned)pos << 16) | (unsigned)slot;
     }
-    warp_argmin(key, pos);
+    if (upper) {
+      sm.o[sl] = o;
+      sm.s[sl] = s;
+      sm.m[sl] = m_raw;
+    }
+    warp_argmin(key, idx);
     if (lane == 0) {
-      red_k[wid] = key;
-      red_t[wid] = pos;
+      sm.wk[par][wid] = key;
+      sm.wi[par][wid] = idx;
     }
-  };
-  for (int64_t i = i0; i <= i1; ++i) {
-    const int np = (int)(i - i0);  // block pivots before i
-    // one call site of the scores (their special functions are long code)
-    if (!yw) score(i);
     __syncthreads();
-    // every warp reduces the warps' minima itself (the key order with the
-    // position as tie-break is a strict total order: the same pivot in each)
-    unsigned long long key = lane < NS / 32 ? red_k[lane] : ~0ull;
-    unsigned pos = lane < NS / 32 ? red_t[lane] : ~0u;
-    warp_argmin(key, pos);
-    const int qm = (int)pos;
-    const int64_t im = i0 + qm;
-    const double m_raw = dm_sub(s_g[qm], s_d[qm]);
-    const bool stop = !(m_raw > eps0);  // the rank test of :533-537
-    const double m_pp = stop ? 0.0 : dm_sqrt(m_raw);
-    if (yw) {
-      // y_i (:538-546) while the slot threads swap and update
-      // (the pivot's values are read at qm, before its swap with position np)
-      if (lane == 0) {
-        if (stop) {
-          rank[0] = i;  // 0-based i == reference's i - 1
-        } else {
-          double a_norm = dm_div(dm_sub(s_a[qm], s_s[qm]), m_pp);
-          double b_norm = dm_div(dm_sub(s_b[qm], s_s[qm]), m_pp);
-          double ea = det_exp(dm_div(-dm_mul(a_norm, a_norm), 2.0));
-          double eb = det_exp(dm_div(-dm_mul(b_norm, b_norm), 2.0));
-          sh_yi = dm_div(dm_mul(dm_sub(ea, eb), is2pi), s_o[qm]);
-        }
-      }
-      __syncwarp();
-      named_bar_arrive(1, NALL);  // its reads of position qm are done
-      if (stop) {
-        write_back();
-        return;
-      }
-      named_bar_arrive(2, NALL);
-    } else {
-      // :518-523, the per-position values of np and qm trade places after
-      // barrier 1, when every read of them for this step is done: d and s,
-      // which the displaced candidate's update uses next, by the two threads
-      // (each takes the other's now and stores its own), the rest by thread np
-      const bool swp = im != i && (t == np || t == qm);
-      double x_d = 0.0, x_s = 0.0;
-      if (swp) {
-        const int o2 = t == np ? qm : np;
-        x_d = s_d[o2];
-        x_s = s_s[o2];
-      }
-      // the pivot's register entries for every candidate's dot product, the
-      // displaced candidate's for its new position
-      if (t == qm) {
-#pragma unroll
-        for (int u = 0; u < kFReg; ++u) s_piv[u] = f[u];
-      }
-      if (im != i && t == np) {
-#pragma unroll
-        for (int u = 0; u < kFReg; ++u) s_x[u] = f[u];
-      }
-      if (im != i) {
-        // the shared-memory entries of the two positions trade places
-        for (int u = kFReg + t; u < np; u += NS) {
-          double *row = s_f + (int64_t)(u - kFReg) * len;
-          const double tt = row[np];
-          row[np] = row[qm];
-          row[qm] = tt;
-        }
-        // :525-530, rows i <-> im over columns i0..n-1, then columns i <-> im,
-        // in one pass: for k outside {i, im} the two swaps touch four distinct
-        // elements; the 2 x 2 block on {i, im} ends up as (i,i) <- (im,im),
-        // (im,im) <- (i,i), (i,im) <- (im,i), (im,i) <- (i,im), and (i,i)
-        // then takes the pivot m_ii.  Position k's thread does index k
-        // (k >= i0), so it keeps the value its update reads: M[k, i] after the
-        // swap, or M[i, k] for the block's first pivot.  This thread's indices
-        // are its own position i0 + t, then the indices outside the panel
-        // ([0, i0) and (ii1, n), numbered o = 0, 1, ...) o = t + e NS:
-        // kSwapBatch of them at a time, all loaded before any is stored (no
-        // element is shared between threads), so the swap costs one memory
-        // round trip per batch -- one in all when n <= len + NS.
-        const int64_t nOwn = has_slot ? 1 : 0;
-        const int64_t nOut = t < n - len ? (n - len - t + NS - 1) / NS : 0;
-        for (int64_t e0 = 0; e0 < nOwn + nOut; e0 += kSwapBatch) {
-          auto kidx = [&](int e) -> int64_t {
-            const int64_t q = e0 + e;
-            if (q < nOwn) return kk;
-            if (q >= nOwn + nOut) return -1;
-            const int64_t o = t + (q - nOwn) * NS;
-            return o < i0 ? o : o + len;
-          };
-          double ri[kSwapBatch], rm[kSwapBatch], ci[kSwapBatch], cm[kSwapBatch];
-          bool diag = false;
-#pragma unroll
-          for (int e = 0; e < kSwapBatch; ++e) {
-            const int64_t k = kidx(e);
-            diag = diag || k == i;
-            const bool live = k >= 0 && k != i && k != im, row = live && k >= i0;
-            ri[e] = row ? M[k * n + i] : 0.0;
-            rm[e] = row ? M[k * n + im] : 0.0;
-            ci[e] = live ? M[i * n + k] : 0.0;
-            cm[e] = live ? M[im * n + k] : 0.0;
-          }
-          double d_ii = 0.0, d_mm = 0.0, d_mi = 0.0, d_im = 0.0;
-          if (diag) {
-            d_ii = M[i * n + i];
-            d_mm = M[im * n + im];
-            d_mi = M[i * n + im];
-            d_im = M[im * n + i];
-          }
-#pragma unroll
-          for (int e = 0; e < kSwapBatch; ++e) {
-            const int64_t k = kidx(e);
-            const bool live = k >= 0 && k != i && k != im, row = live && k >= i0;
-            if (row) {
-              M[k * n + i] = rm[e];
-              M[k * n + im] = ri[e];
-            }
-            if (live) {
-              M[i * n + k] = cm[e];
-              M[im * n + k] = ci[e];
-              if (k == kk) mij = np == 0 ? rm[e] : cm[e];
-            }
-          }
-          if (diag) {
-            M[i * n + i] = stop ? d_mm : m_pp;
-            M[im * n + im] = d_ii;
-            M[im * n + i] = d_mi;
-            M[i * n + im] = d_im;
-            sh_mij_im = np == 0 ? d_mi : d_im;  // for position im
-          }
+    key = lane < kPivThreads / 32 ? sm.wk[par][lane] : ~0ull;
+    idx = lane < kPivThreads / 32 ? sm.wi[par][lane] : ~0u;
+    warp_argmin(key, idx);
+    // this CTA's best candidate to every CTA (two buffers: a CTA that is a
+    // step ahead writes the other one)
+    {
+      const int lb = key == ~0ull ? 0 : (int)(idx & 0xffffu) - cid * kPivSlots;
+      const PivRec *R = &sm.rec[par][cid];
+      const void *dst = nullptr;
+      unsigned long long v = 0;
+      if (tid < kPivMax) {
+        if (tid < u) {
+          dst = &R->f[tid];
+          v = (unsigned long long)__double_as_longlong(sm.f[tid][lb]);
         }
       } else {
-        if (has_slot && kk > i) mij = np == 0 ? M[kk * n + i] : M[i * n + kk];
-        if (t == np && !stop) M[i * n + i] = m_pp;
-      }
-      named_bar_sync(1, NALL);
-      if (swp) {
-        s_d[t] = x_d;
-        s_s[t] = x_s;
-        if (t == np) {
-          const int64_t tp = s_p[np]; s_p[np] = s_p[qm]; s_p[qm] = tp;
-          double tt;
-          tt = s_a[np]; s_a[np] = s_a[qm]; s_a[qm] = tt;
-          tt = s_b[np]; s_b[np] = s_b[qm]; s_b[qm] = tt;
-          tt = s_g[np]; s_g[np] = s_g[qm]; s_g[qm] = tt;
+        switch (tid - kPivMax) {
+          case 0: dst = &R->key; v = key; break;
+          case 1: dst = &R->idx; v = idx; break;
+          case 2: dst = &R->m_raw; v = (unsigned long long)__double_as_longlong(sm.m[lb]); break;
+          case 3: dst = &R->o; v = (unsigned long long)__double_as_longlong(sm.o[lb]); break;
+          case 4: dst = &R->a; v = (unsigned long long)__double_as_longlong(sm.a[lb]); break;
+          case 5: dst = &R->b; v = (unsigned long long)__double_as_longlong(sm.b[lb]); break;
+          case 6: dst = &R->s; v = (unsigned long long)__double_as_longlong(sm.s[lb]); break;
+          default: break;
         }
       }
-      if (im != i) {
-        if (t == np) {
+      if (dst)
+        for (int c = 0; c < C; ++c) cluster_store(cluster_addr(dst, c), v);
+    }
+    cluster_sync_all();
+    key = lane < C ? sm.rec[par][lane].key : ~0ull;
+    idx = lane < C ? sm.rec[par][lane].idx : ~0u;
+    warp_argmin(key, idx);
+    const int pslot = (int)(idx & 0xffffu), ppos = (int)(idx >> 16);
+    const PivRec &R = sm.rec[par][pslot / kPivSlots];
+    // :518-531: the pivot and the candidate at position u trade places
+    if (slot == pslot) pos = u;
+    else if (pos == u) pos = ppos;
+    const bool live = has && pos > u;
+    const double mij = live ? M[(i0 + pslot) * n + g] : 0.0;
+    const double p_raw = R.m_raw;
+    if (!(p_raw > eps0)) {  // the rank test of :533-537
+      if (cid == 0 && tid == 0) rank[0] = i0 + u;
+      done = u;
+      break;
+    }
+    const double m_pp = dm_sqrt(p_raw);
+    if (tid == 0) sm.fd[u] = m_pp;
+    // the ascending fma chain over the block's pivots
+    double acc = 0.0;
+    int t = 0;
+    for (; t + 8 <= u; t += 8) {
+      double x[8], y[8];
 #pragma unroll
-          for (int u = 0; u < kFReg; ++u) f[u] = s_piv[u];
-        } else if (t == qm) {
-#pragma unroll
-          for (int u = 0; u < kFReg; ++u) f[u] = s_x[u];
-          mij = sh_mij_im;
-        }
+      for (int q = 0; q < 8; ++q) {
+        x[q] = sm.f[t + q][sl];
+        y[q] = R.f[t + q];
       }
-      if (stop) {
-        write_back();
-        return;
-      }
-      // the update of step i (:547-570) for this position
-      const bool upd = has_slot && kk > i;
-      double m = 0.0;
-      if (upd) {
-        if (np == 0) {
-          m = dm_div(mij, m_pp);
-        } else {
-          // the ascending fma chain over the block's pivots l = i0 .. i - 1
-          double acc = 0.0;
 #pragma unroll
-          for (int u = 0; u < kFReg; ++u)
-            if (u < np) acc = dm_fma(f[u], s_piv[u], acc);
-          int u = kFReg;
-          for (; u + 8 <= np; u += 8) {
-            double x[8], y[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const double *row = s_f + (int64_t)(u + e - kFReg) * len;
-              x[e] = row[t];
-              y[e] = row[np];
-            }
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc = dm_fma(x[e], y[e], acc);
-          }
-          for (; u < np; ++u) {
-            const double *row = s_f + (int64_t)(u - kFReg) * len;
-            acc = dm_fma(row[t], row[np], acc);
-          }
-          m = dm_div(dm_sub(mij, acc), m_pp);
-        }
-        s_d[t] = dm_add(s_d[t], dm_mul(m, m));
-        if (np < kFReg) {
-#pragma unroll
-          for (int u2 = 0; u2 < kFReg; ++u2) f[u2] = u2 == np ? m : f[u2];
-        } else {
-          s_f[(int64_t)(np - kFReg) * len + t] = m;
-        }
-        M[kk * n + i] = m;
-        M[i * n + kk] = m;
-      }
-      named_bar_sync(2, NALL);  // y_i
-      if (upd) s_s[t] = dm_add(s_s[t], dm_mul(sh_yi, m));
+      for (int q = 0; q < 8; ++q) acc = dm_fma(x[q], y[q], acc);
+    }
+    for (; t < u; ++t) acc = dm_fma(sm.f[t][sl], R.f[t], acc);
+    // y_i (:538-546), each side's term in half of the threads (x / 2 = x * 0.5)
+    const double nrm = dm_div(dm_sub(upper ? R.b : R.a, R.s), m_pp);
+    const double ex = det_exp(dm_mul(-dm_mul(nrm, nrm), 0.5));
+    const double exo = __shfl_xor_sync(0xffffffffu, ex, 1);
+    const double yi = dm_div(dm_mul(upper ? dm_sub(exo, ex) : dm_sub(ex, exo), is2pi), R.o);
+    if (live) {  // :547-570
+      const double m = dm_div(dm_sub(mij, acc), m_pp);
+      ds = dm_add(ds, dm_mul(m, m));
+      s = dm_add(s, dm_mul(yi, m));
+      if (upper) sm.f[u][sl] = m;
     }
   }
-  write_back();
+  __syncthreads();
+  if (has && upper) {
+    const int64_t q = i0 + pos;
+    dvec[q] = ds;
+    svec[q] = s;
+    a[q] = av;
+    b[q] = bv;
+    perm[q] = pv;
+    out.ord[pos] = slot;
+    for (int t = 0; t < done; ++t) out.f[t * kPivPanel + slot] = sm.f[t][sl];
+  }
+  if (cid == 0 && tid < done) out.fd[tid] = sm.fd[tid];
+  if (cid == 0 && tid == 0) *out.done = done;
+  cluster_sync_all();  // no CTA leaves while another may still write to it
 }
 
 // C[j,k] -= sum_{l=p0..p1} A(l,j) * B(l,k) for j,k in [c0, c1], one

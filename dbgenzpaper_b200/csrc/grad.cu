@@ -111,7 +111,7 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   // samples alone, whatever the checkpoint setting: no recomputation (the
   // setting applies to the CSC loop).
   if (sparse && !p->csc_colptr.p) DBGZ_TRY(dbgz_build_csc(p));
-  const int64_t seg = sparse && !dbgz_band_loop(p, precision) ? ctx->grad_ckpt_seg : 0;
+  const int64_t seg = sparse && !dbgz_band_loop(p, true) ? ctx->grad_ckpt_seg : 0;
   const int64_t nY = d - 1, K = seg > 0 ? (nY + seg - 1) / seg : 0;
   const bool ckpt = seg > 0 && K >= 1;
   int64_t Wf = 0, Wb = 0;  // ring sizes of the forward and adjoint banded loops

@@ -257,7 +257,7 @@ void dbgz_umma_batch_free(UmmaBatchPlan *B);
 int dbgz_loop_sparse(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,
                      int64_t n_tiles);
 int dbgz_build_csc(dbgz_problem *p);
-bool dbgz_band_loop(dbgz_problem *p, int precision);  // after dbgz_build_csc
+bool dbgz_band_loop(const dbgz_problem *p, bool grad);  // after dbgz_build_csc
 void dbgz_drop_graphs(dbgz_problem *p);
 // dU[t*d + l] (+)= sum_n Y(l, n) S(t, n) over the nc samples, for l < t only,
 // Y and S tile-major ([tile][row < d][128 samples], the FP32 layout of

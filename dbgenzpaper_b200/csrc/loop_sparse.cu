@@ -412,17 +412,24 @@ static int launch_sparse_gen(dbgz_problem *p, const PassArgs &pa, double *partia
   return launch_sparse_kind<T, DBGZ_QMC_RICHTMYER>(p, pa, partials, n_tiles);
 }
 
-// Whether the problem runs in the loops that treat the band as dense
-// (loop_f64_kernels.cuh, loop_w32_kernels.cuh) rather than in the CSC loop.
-bool dbgz_band_loop(dbgz_problem *p, int precision) {
-  static const char *e = getenv("W32_BAND");
-  return p->bandwidth <= (e ? atoi(e) : 100000);
+// Whether a pass (grad: one that keeps its state, or its adjoint) runs in the
+// loops that treat the band as dense (loop_f64_kernels.cuh,
+// loop_w32_kernels.cuh) rather than in the CSC loop, whose cost grows with the
+// entries and not with the bandwidth.  d = 1500, 2^13 x 12 or x 10 Sobol samples,
+// CSC against band loop, entries per column = bandwidth b:
+//   FP32 pass      b = 4: 1.35 / 1.48 ms   8: 1.54 / 1.48   64: 5.3 / 1.7   256: 31 / 2.9
+//   FP64 pass      b = 4: 2.64 / 2.72      8: 2.83 / 2.70   64: 9.5 / 3.5   256: 83 / 5.8
+//   FP32 gradient  b = 1: 5.2 / 3.2       16: 6.8 / 3.4     64: 18 / 3.9    256: 99 / 5.8
+// so an entry costs the CSC loop about 16 times what a unit of bandwidth costs
+// the band loop, and the CSC loop starts 4 entries ahead (a gradient: 12 behind).
+bool dbgz_band_loop(const dbgz_problem *p, bool grad) {
+  return 16 * p->nnz > p->d * (p->bandwidth + (grad ? -16 * 12 : 16 * 4));
 }
 
 int dbgz_loop_sparse(dbgz_problem *p, const PassArgs &pa, int precision, double *partials, int64_t n_tiles) {
   if (!p->csc_colptr.p) DBGZ_TRY(dbgz_build_csc(p));
   const bool segments = pa.i_begin != 0 || pa.i_end >= 0 || pa.ck_save || pa.ck_load || pa.store_p;
-  if (!segments && dbgz_band_loop(p, precision))
+  if (!segments && dbgz_band_loop(p, pa.kind == kLoopForwardStore || pa.kind == kLoopAdjoint))
     return precision == DBGZ_PREC_FP64 ? dbgz_loop_simt(p, pa, precision, partials, n_tiles)
                                        : dbgz_loop_w32_band(p, pa, partials, n_tiles);
   if (pa.kind == kLoopAdjoint && !p->cscb_colptr.p) {

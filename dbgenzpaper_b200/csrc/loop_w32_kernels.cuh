@@ -10,8 +10,8 @@
 // 16 warps fit on an SM, and mma.m16n8k16 (8 cycles of a scheduler, in the
 // shadow of the other warps' steps) feeds them without a round trip to
 // another warp.  The larger the dimension, the more the contraction weighs:
-// mma.sync runs at about a quarter of tcgen05's rate (dbgz_use_w32 has the
-// crossover).
+// mma.sync runs at about a quarter of tcgen05's rate (dbgz_loop_umma has
+// the crossover).
 //
 // One CTA = one tile of 128 samples = four warps of 32.  y-indices run in
 // groups of G, each in chunks of 8:
@@ -22,7 +22,10 @@
 //   * chunk: its sums + the group's own earlier chunks by mma (a chunk's y's
 //     take the place of the sums they consumed), 8 sequential steps with the
 //     chunk's triangle as FMAs in registers, the y's back as BF16 parts.
-// Operands are NPART BF16 parts: 2 (hi hi + hi lo + lo hi: the split-BF16
+// The tensor unit truncates as it accumulates, so the products of high parts
+// have accumulators of their own: their sum is truncated once per 16 y-indices,
+// not once per product (relative error of P, batch of d 16..256: 4.7e-6 with
+// one accumulator).  Operands are NPART BF16 parts: 2 (hi hi + hi lo + lo hi: the split-BF16
 // mode) or 3 (six products, about 2^-24: FP32 operands' accuracy, for the
 // banded loop).  Warps meet once per chunk of the ring and per 32 dimensions
 // (their staged constants, copied one block ahead).
@@ -227,13 +230,15 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
     const bool keep = g0 + G < nY;
     const int64_t k0 = first_k<G>(g0, P.band), lofs = P.band > 0 ? k0 : 0;
     if (g0 > 0) {
-      float acc[2][G / CH][4];
+      float acc[2][2][G / CH][4];  // [0]: high parts' products, [1]: the others
 #pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int ni = 0; ni < G / CH; ++ni)
+        for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[mi][ni][e] = 0.f;
+          for (int ni = 0; ni < G / CH; ++ni)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[h][mi][ni][e] = 0.f;
       const int nch = (int)((g0 - k0) / KC);
       // this thread's share of a stage: NPART pieces of each of its warp's two
       // Y chunks (a pair never straddles the workspace's wrap: both sizes are
@@ -287,27 +292,27 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
         asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
         __syncthreads();
         issue();
-        uint32_t a[2][NPART][4];
+        // one m-tile after the other: half the A fragments at a time (with
+        // both, three parts spilled)
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
+        for (int mi = 0; mi < 2; ++mi) {
+          uint32_t a[NPART][4];
 #pragma unroll
-          for (int p = 0; p < NPART; ++p) ldsm4(a[mi][p], ya + s * (uint32_t)sizeof(sm.u.ring.y[0]) + p * 512 + mi * 256);
+          for (int p = 0; p < NPART; ++p) ldsm4(a[p], ya + s * (uint32_t)sizeof(sm.u.ring.y[0]) + p * 512 + mi * 256);
 #pragma unroll
-        for (int n2 = 0; n2 < G / CH; n2 += 2)
-          if (n2 < nt) {
-            // (targets n2, k half 0), (n2, 1), (n2 + 1, 0), (n2 + 1, 1)
-            uint32_t b[NPART][4];
+          for (int n2 = 0; n2 < G / CH; n2 += 2)
+            if (n2 < nt) {
+              // (targets n2, k half 0), (n2, 1), (n2 + 1, 0), (n2 + 1, 1)
+              uint32_t b[NPART][4];
 #pragma unroll
-            for (int p = 0; p < NPART; ++p)
-              ldsm4(b[p], ua + s * (uint32_t)sizeof(sm.u.ring.u[0]) + p * (2 * G * 16) + n2 * (CH * 16));
-            products<NPART>([&](int i, int jj) {
-#pragma unroll
-              for (int mi = 0; mi < 2; ++mi) {
-                mma16(acc[mi][n2], a[mi][i], b[jj][0], b[jj][1]);
-                mma16(acc[mi][n2 + 1], a[mi][i], b[jj][2], b[jj][3]);
-              }
-            });
-          }
+              for (int p = 0; p < NPART; ++p)
+                ldsm4(b[p], ua + s * (uint32_t)sizeof(sm.u.ring.u[0]) + p * (2 * G * 16) + n2 * (CH * 16));
+              products<NPART>([&](int i, int jj) {
+                mma16(acc[i + jj > 0][mi][n2], a[i], b[jj][0], b[jj][1]);
+                mma16(acc[i + jj > 0][mi][n2 + 1], a[i], b[jj][2], b[jj][3]);
+              });
+            }
+        }
         s = s + 1 == NST ? 0 : s + 1;
       }
       __syncthreads();  // the ring is read: S may be written
@@ -318,7 +323,8 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
           for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int h = 0; h < 2; ++h)
-              sts2(Sa + ni * SM::SLOT + sf + mi * 512 + h * 256, acc[mi][ni][2 * h], acc[mi][ni][2 * h + 1]);
+              sts2(Sa + ni * SM::SLOT + sf + mi * 512 + h * 256, acc[0][mi][ni][2 * h] + acc[1][mi][ni][2 * h],
+                   acc[0][mi][ni][2 * h + 1] + acc[1][mi][ni][2 * h + 1]);
         }
       __syncwarp();
     }
@@ -335,11 +341,12 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
         float s[8];
         if (q > 0) {
           // the group's earlier chunks, two at a time
-          float c[2][4];
+          float c[2][4], cs[2][4];
 #pragma unroll
           for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
+              cs[mi][2 * h] = cs[mi][2 * h + 1] = 0.f;
               c[mi][2 * h] = c[mi][2 * h + 1] = 0.f;
               if (g0 > 0) lds2(c[mi][2 * h], c[mi][2 * h + 1], Sq + sf + mi * 512 + h * 256);
             }
@@ -352,20 +359,20 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
 #pragma unroll
           for (int cc = 0; cc < G / CH; cc += 2)
             if (cc + 2 <= q) {
-              uint32_t b[NPART][2], a[2][NPART][4];
+              uint32_t b[NPART][2];
 #pragma unroll
               for (int p = 0; p < NPART; ++p) {
                 b[p][0] = __ldg(ub[p] + cc * (CH / 2));
                 b[p][1] = __ldg(ub[p] + cc * (CH / 2) + CH / 2);
               }
 #pragma unroll
-              for (int mi = 0; mi < 2; ++mi)
+              for (int mi = 0; mi < 2; ++mi) {
+                uint32_t a[NPART][4];
 #pragma unroll
-                for (int p = 0; p < NPART; ++p) ldsm4(a[mi][p], la + cc * SM::SLOT + p * 512 + mi * 256);
-              products<NPART>([&](int i, int jj) {
-#pragma unroll
-                for (int mi = 0; mi < 2; ++mi) mma16(c[mi], a[mi][i], b[jj][0], b[jj][1]);
-              });
+                for (int p = 0; p < NPART; ++p) ldsm4(a[p], la + cc * SM::SLOT + p * 512 + mi * 256);
+                products<NPART>(
+                    [&](int i, int jj) { mma16(i + jj > 0 ? cs[mi] : c[mi], a[i], b[jj][0], b[jj][1]); });
+              }
             }
           if (q & 1) {
             uint32_t b[NPART], a[NPART][4];  // a: samples 0-7, 8-15, 16-23, 24-31 of one chunk
@@ -375,14 +382,15 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
             for (int p = 0; p < NPART; ++p) ldsm4(a[p], Sq - SM::SLOT + p * 512 + lane * 16);
             products<NPART>([&](int i, int jj) {
 #pragma unroll
-              for (int mi = 0; mi < 2; ++mi) mma8(c[mi], a[i][2 * mi], a[i][2 * mi + 1], b[jj]);
+              for (int mi = 0; mi < 2; ++mi) mma8(i + jj > 0 ? cs[mi] : c[mi], a[i][2 * mi], a[i][2 * mi + 1], b[jj]);
             });
           }
           __syncwarp();  // every lane has read its part of the chunk's sums
 #pragma unroll
           for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) sts2(Sq + sf + mi * 512 + h * 256, c[mi][2 * h], c[mi][2 * h + 1]);
+            for (int h = 0; h < 2; ++h)
+              sts2(Sq + sf + mi * 512 + h * 256, c[mi][2 * h] + cs[mi][2 * h], c[mi][2 * h + 1] + cs[mi][2 * h + 1]);
           __syncwarp();
         }
         if (g0 > 0 || q > 0) {
