@@ -85,6 +85,19 @@ __global__ void k_first_nonfinite(const double *x, int64_t n, unsigned long long
     if (!isfinite(x[i])) atomicMin(first, (unsigned long long)i);
 }
 
+// FP32 copies of the Richtmyer shifts.
+__global__ void k_shifts_f32(const double *s, int64_t n, float *s32) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    s32[i] = (float)s[i];
+}
+
+// What a prepare reads back, in one copy at its end.
+struct PrepareResult {
+  unsigned long long first_nonfinite;  // index in Sigma, ~0: none
+  int64_t rank;
+  double head[3];  // a_0, b_0, U_00 of the first variable
+};
+
 static int upload(dbgz_ctx *ctx, DevBuf &b, const void *src, size_t bytes) {
   DBGZ_TRY(dbgz_ensure(ctx, b, bytes));
   DBGZ_CUDA_TRY(ctx, cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
@@ -364,28 +377,20 @@ int dbgz_prepare(dbgz_ctx *ctx, int64_t d, const double *Sigma, const double *a,
   const size_t nn = (size_t)d * d;
   const int64_t launches0 = ctx->launch_count;
   if (ctx->profiling) cudaEventRecord(ctx->ev[0], ctx->stream);
-  DevBuf chk;  // first non-finite index of Sigma (UINT64_MAX: none)
+  DevBuf chk;  // PrepareResult
+  PrepareResult pr{};
   do {
     if ((rc = upload(ctx, p->U, Sigma, nn * 8))) break;
-    if ((rc = dbgz_ensure(ctx, chk, 8))) break;
+    if ((rc = dbgz_ensure(ctx, chk, sizeof(PrepareResult)))) break;
+    PrepareResult *dres = (PrepareResult *)chk.p;
     if (cudaMemsetAsync(chk.p, 0xff, 8, ctx->stream) != cudaSuccess) {
       rc = dbgz_fail(ctx, DBGZ_ERR_CUDA, "prepare: memset failed");
       break;
     }
     k_first_nonfinite<<<(unsigned)std::min<int64_t>(((int64_t)nn + 255) / 256, 2048), 256, 0, ctx->stream>>>(
-        (const double *)p->U.p, (int64_t)nn, (unsigned long long *)chk.p);
+        (const double *)p->U.p, (int64_t)nn, &dres->first_nonfinite);
     dbgz_count_launch(ctx);
-    // the factorisation runs on whatever Sigma holds (its loops are bounded);
-    // a non-finite entry is reported before its rank
-    auto sigma_ok = [&]() -> int {
-      unsigned long long first = ~0ull;
-      if (cudaMemcpy(&first, chk.p, 8, cudaMemcpyDeviceToHost) != cudaSuccess)
-        return dbgz_fail(ctx, DBGZ_ERR_CUDA, "prepare: %s", cudaGetErrorString(cudaGetLastError()));
-      if (first != ~0ull)
-        return dbgz_fail(ctx, DBGZ_ERR_NONFINITE_INPUT, "prepare: Sigma has a non-finite entry at %lld",
-                         (long long)first);
-      return DBGZ_OK;
-    };
+    // (the factorisation runs on whatever Sigma holds: its loops are bounded)
     if ((rc = upload(ctx, p->a, a, d * 8))) break;
     if ((rc = upload(ctx, p->b, b, d * 8))) break;
     if ((rc = dbgz_ensure(ctx, p->perm, d * 8))) break;
@@ -393,21 +398,13 @@ int dbgz_prepare(dbgz_ctx *ctx, int64_t d, const double *Sigma, const double *a,
     if (structure == DBGZ_STRUCTURE_DENSE) {
       rc = dbgz_chol_genz_dev(ctx, d, (double *)p->U.p, (double *)p->a.p, (double *)p->b.p,
                               o.chol_block_size, o.chol_block_size2, 1024, 2048,
-                              (int64_t *)p->perm.p, (double *)p->scale.p, &p->rank);
+                              (int64_t *)p->perm.p, (double *)p->scale.p, &dres->rank);
       if (rc) break;
-      if ((rc = sigma_ok())) break;
-      if (p->rank != d) {
-        rc = dbgz_fail(ctx, DBGZ_ERR_RANK_DEFICIENT, "QMCData requires a full-rank Cholesky factorization. (rank %lld of %lld)",
-                       (long long)p->rank, (long long)d);
-        break;
-      }
     } else {
       rc = dbgz_chol_classic_dev(ctx, d, (double *)p->U.p, (double *)p->a.p, (double *)p->b.p,
                                  o.chol_block_size, o.chol_block_size2, 1024, 2048,
                                  (double *)p->scale.p);
       if (rc) break;
-      if ((rc = sigma_ok())) break;
-      p->rank = d;
       std::vector<int64_t> id(d);
       for (int64_t i = 0; i < d; ++i) id[i] = i;
       if ((rc = upload(ctx, p->perm, id.data(), d * 8))) break;
@@ -416,11 +413,13 @@ int dbgz_prepare(dbgz_ctx *ctx, int64_t d, const double *Sigma, const double *a,
     if (qmc_type == DBGZ_QMC_RICHTMYER) {
       std::vector<double> q(d - 1);
       dbgz_sqrt_primes(d - 1, q.data());
-      std::vector<float> s32((d - 1) * o.n_reps);
-      for (size_t i = 0; i < s32.size(); ++i) s32[i] = (float)shifts[i];
+      const int64_t ns = (d - 1) * o.n_reps;
       if ((rc = upload(ctx, p->q, q.data(), (d - 1) * 8))) break;
-      if ((rc = upload(ctx, p->shifts, shifts, (d - 1) * o.n_reps * 8))) break;
-      if ((rc = upload(ctx, p->shifts32, s32.data(), s32.size() * 4))) break;
+      if ((rc = upload(ctx, p->shifts, shifts, ns * 8))) break;
+      if ((rc = dbgz_ensure(ctx, p->shifts32, ns * 4))) break;
+      k_shifts_f32<<<(unsigned)std::min<int64_t>((ns + 255) / 256, 1024), 256, 0, ctx->stream>>>(
+          (const double *)p->shifts.p, ns, (float *)p->shifts32.p);
+      dbgz_count_launch(ctx);
     } else {
       std::vector<uint32_t> V;
       const uint32_t *Vp = sobol_dirnums;
@@ -435,12 +434,26 @@ int dbgz_prepare(dbgz_ctx *ctx, int64_t d, const double *Sigma, const double *a,
       if ((rc = upload(ctx, p->V, Vp, (d - 1) * 32 * 4))) break;
       if ((rc = upload(ctx, p->ushifts, ushifts, (d - 1) * o.n_reps * 8))) break;
     }
-    if ((rc = dbgz_make_targets(p))) break;
+    if ((rc = dbgz_make_targets(p, dres->head))) break;
     if (ctx->profiling) cudaEventRecord(ctx->ev[1], ctx->stream);
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    if (cudaMemcpyAsync(&pr, dres, sizeof(pr), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
       rc = dbgz_fail(ctx, DBGZ_ERR_CUDA, "prepare: %s", cudaGetErrorString(cudaGetLastError()));
       break;
     }
+    // a non-finite entry is reported before the rank it led to
+    if (pr.first_nonfinite != ~0ull) {
+      rc = dbgz_fail(ctx, DBGZ_ERR_NONFINITE_INPUT, "prepare: Sigma has a non-finite entry at %lld",
+                     (long long)pr.first_nonfinite);
+      break;
+    }
+    p->rank = structure == DBGZ_STRUCTURE_DENSE ? pr.rank : d;
+    if (p->rank != d) {
+      rc = dbgz_fail(ctx, DBGZ_ERR_RANK_DEFICIENT, "QMCData requires a full-rank Cholesky factorization. (rank %lld of %lld)",
+                     (long long)p->rank, (long long)d);
+      break;
+    }
+    for (int e = 0; e < 3; ++e) p->head[e] = pr.head[e];
   } while (0);
   dbgz_release(chk);
   if (rc != DBGZ_OK) {
@@ -522,12 +535,7 @@ int dbgz_problem_factor(const dbgz_problem *p, double *U, int64_t *perm, double 
 
 int dbgz_first_dim_cdf(dbgz_problem *p) {
   if (p->c1_ready) return DBGZ_OK;
-  dbgz_ctx *ctx = p->ctx;
-  double a0, b0, u00;
-  cudaMemcpyAsync(&a0, p->a.p, 8, cudaMemcpyDeviceToHost, ctx->stream);
-  cudaMemcpyAsync(&b0, p->b.p, 8, cudaMemcpyDeviceToHost, ctx->stream);
-  cudaMemcpyAsync(&u00, p->U.p, 8, cudaMemcpyDeviceToHost, ctx->stream);
-  DBGZ_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  const double a0 = p->head[0], b0 = p->head[1], u00 = p->head[2];
   // src/qmc.jl:800-809
   double arg_a = a0 / (u00 * std::sqrt(2.0));
   double arg_b = b0 / (u00 * std::sqrt(2.0));
@@ -561,12 +569,10 @@ int dbgz_pnorm(dbgz_problem *p, int precision, double *result, double *err, int6
   const dbgz_opts &o = p->opts;
   const int64_t n_reps = o.n_reps, m = o.m;
   DBGZ_TRY(dbgz_first_dim_cdf(p));
-  if (precision != DBGZ_PREC_FP64 && !p->U32.p) DBGZ_TRY(dbgz_make_U32(p));
   const int64_t tps = (m + 127) / 128;
   const int64_t n_tiles = tps * n_reps;
   DBGZ_TRY(dbgz_ensure(ctx, p->partials, sizeof(double) * n_tiles));
   DBGZ_TRY(dbgz_ensure(ctx, p->reps, sizeof(double) * n_reps));
-  DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(p->reps.p, 0, sizeof(double) * n_reps, ctx->stream));
   std::vector<double> reps(n_reps);
   PassArgs pa{};
   pa.d = p->d;
@@ -596,6 +602,7 @@ int dbgz_pnorm(dbgz_problem *p, int precision, double *result, double *err, int6
     if (prof) cudaEventRecord(ctx->ev[2], ctx->stream);
     const bool sparse = p->structure == DBGZ_STRUCTURE_SPARSE;
     const bool tensor = !sparse && (precision == DBGZ_PREC_FP32_TF32 || precision == DBGZ_PREC_FP32_SPLIT_BF16);
+    const bool waits = tensor && dbgz_umma_waits(p, precision);  // the loop has bounded waits: read its status
     if (sparse)
       DBGZ_TRY(dbgz_loop_sparse(p, pa, precision, (double *)p->partials.p, n_tiles));
     else if (tensor)
@@ -610,7 +617,7 @@ int dbgz_pnorm(dbgz_problem *p, int precision, double *result, double *err, int6
     DBGZ_CUDA_TRY(ctx, cudaMemcpyAsync(reps.data(), p->reps.p, sizeof(double) * n_reps,
                                        cudaMemcpyDeviceToHost, ctx->stream));
     int dev_status = 0;
-    if (tensor)
+    if (waits)
       DBGZ_CUDA_TRY(ctx, cudaMemcpyAsync(&dev_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost,
                                          ctx->stream));
     if (prof) cudaEventRecord(ctx->ev[1], ctx->stream);
@@ -652,7 +659,6 @@ int dbgz_pnorm_logw(dbgz_problem *p, int precision, double *logw, double *qmc_re
   const dbgz_opts &o = p->opts;
   const int64_t n_reps = o.n_reps, m = o.m;
   DBGZ_TRY(dbgz_first_dim_cdf(p));
-  if (precision != DBGZ_PREC_FP64 && !p->U32.p) DBGZ_TRY(dbgz_make_U32(p));
   const int64_t tps = (m + 127) / 128;
   const int64_t n_tiles = tps * n_reps;
   DBGZ_TRY(dbgz_ensure(ctx, p->partials, sizeof(double) * n_tiles));
@@ -663,7 +669,6 @@ int dbgz_pnorm_logw(dbgz_problem *p, int precision, double *logw, double *qmc_re
     ~Release() { dbgz_release(b); }
   } release_lw{lw};
   DBGZ_TRY(dbgz_ensure(ctx, lw, sizeof(double) * (size_t)n_tiles * 128));
-  DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(p->reps.p, 0, sizeof(double) * n_reps, ctx->stream));
   DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
   PassArgs pa{};
   pa.kind = kLoopLogWeight;

@@ -164,25 +164,15 @@ __global__ void k_shifts32(const double *sh, int64_t n, float *s32, int *bad) {
   }
 }
 
-// Per (problem, shift): the Neumaier sum of the shift's tile sums in tile
-// order and its mean, as simt::k_finalize does for one problem.
+// One warp per (problem, shift): the sum of the shift's tile sums and its
+// mean, as simt::k_finalize does for one problem.
 __global__ void k_finalize_batch(const double *partials, const int64_t *part_off, int64_t tps, int64_t n_reps,
                                  int64_t n_probs, int64_t m, double *reps) {
-  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (g >= n_probs * n_reps) return;
   const int64_t prob = g / n_reps, k = g - prob * n_reps;
-  const double *pk = partials + part_off[prob] + k * tps;
-  double s = 0.0, c = 0.0;
-  for (int64_t t = 0; t < tps; ++t) {
-    const double x = pk[t];
-    const double tt = s + x;
-    if (fabs(s) >= fabs(x)) c += (s - tt) + x;
-    else c += (x - tt) + s;
-    s = tt;
-  }
-  s += c;
-  const double inv_tot = 1.0 / (double)m;
-  reps[g] = fma(0.0, 0.0, s * inv_tot);
+  const double s = simt::warp_shift_sum(partials + part_off[prob] + k * tps, tps);
+  if ((threadIdx.x & 31) == 0) reps[g] = simt::running_mean(s, 0, m, nullptr);
 }
 
 // The persistent CUDA-core loop over the work queue: the FP64 loop
@@ -538,7 +528,7 @@ int plan_enqueue(dbgz_batch_plan *P, const double *Sigma, const double *a, const
     ++launches;
   }
   plan_event(P, 4, capturing);
-  k_finalize_batch<<<(unsigned)((np * P->R + 127) / 128), 128, 0, st>>>(P->dpart, P->dpo, P->tps, P->R, np, P->m,
+  k_finalize_batch<<<(unsigned)((np * P->R + 3) / 4), 128, 0, st>>>(P->dpart, P->dpo, P->tps, P->R, np, P->m,
                                                                           P->dreps);
   ++launches;
   DBGZ_CUDA_TRY(ctx, cudaGetLastError());

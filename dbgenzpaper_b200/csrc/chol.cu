@@ -28,15 +28,21 @@ namespace {
 
 constexpr int kStepThreads = 1024;
 
-__global__ void k_diag_absmax(const double *M, int64_t n, double *out) {
+// One block: eps0 = eps max |diag| (NaN if a diagonal is NaN), the scale
+// vector, the identity permutation, rank = n and zeroed vectors (src/cholesky.jl:452-471).
+__global__ void k_chol_init(const double *M, int64_t n, double *eps0, double *scale, int64_t *perm, int64_t *rank,
+                            double *zero, int64_t n_zero) {
   __shared__ double sh[32];
   double mx = 0.0;
   bool nan = false;
   for (int64_t j = threadIdx.x; j < n; j += blockDim.x) {
-    double v = fabs(M[j * n + j]);
+    const double x = M[j * n + j], v = fabs(x);
     if (v != v) nan = true;
     else if (v > mx) mx = v;
+    scale[j] = x > 0 ? dm_sqrt(x) : 1.0;
+    perm[j] = j;
   }
+  for (int64_t j = threadIdx.x; j < n_zero; j += blockDim.x) zero[j] = 0.0;
   nan = __syncthreads_or(nan);
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
@@ -44,7 +50,8 @@ __global__ void k_diag_absmax(const double *M, int64_t n, double *out) {
   if (threadIdx.x == 0) {
     double r = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, sh[w]);
-    out[0] = nan ? NAN : dm_mul(DBL_EPSILON, r);
+    eps0[0] = nan ? NAN : dm_mul(DBL_EPSILON, r);
+    rank[0] = n;
   }
 }
 
@@ -432,10 +439,16 @@ __global__ void k_anti_transpose(const double *U, int64_t d, double *Ub) {
     Ub[j * d + i] = U[(d - 1 - i) * d + (d - 1 - j)];
 }
 
+// (head: a_0, b_0 and U_00 for the first variable's CDF on the host)
 __global__ void k_targets(const double *U, int64_t n, const double *a, const double *b,
-                          TargetParams64 *t64, TargetParams32 *t32) {
+                          TargetParams64 *t64, TargetParams32 *t32, double *head) {
   int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n) return;
+  if (t == 0) {
+    head[0] = a[0];
+    head[1] = b[0];
+    head[2] = U[0];
+  }
   const double c2 = sqrt(2.0);
   double inv_u = 1.0 / (U[t * n + t] * c2);
   t64[t] = TargetParams64{a[t], b[t], inv_u};
@@ -478,9 +491,11 @@ int launch_trsm(dbgz_ctx *ctx, double *M, int64_t n, int64_t p0, int64_t p1, int
 }
 
 int scale_correlation(dbgz_ctx *ctx, double *M, int64_t n, double *a, double *b, double *scale,
-                      int mirror) {
-  k_scale_vec<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(M, n, scale);
-  dbgz_count_launch(ctx);
+                      int mirror, bool scale_ready = false) {
+  if (!scale_ready) {
+    k_scale_vec<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(M, n, scale);
+    dbgz_count_launch(ctx);
+  }
   dim3 grid((unsigned)((n + 255) / 256), (unsigned)n);
   k_scale_apply<<<grid, 256, 0, ctx->stream>>>(M, n, a, b, scale, mirror);
   dbgz_count_launch(ctx);
@@ -529,7 +544,7 @@ int launch_genz_cluster(dbgz_ctx *ctx, double *M, int64_t n, double *a, double *
 
 int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b, int64_t bs1,
                        int64_t bs2, int64_t bs3, int64_t bs4, int64_t *perm, double *scale,
-                       int64_t *rank_host) {
+                       int64_t *rank_out) {
   if (bs1 < 1 || bs2 < 1 || bs3 < 1 || bs4 < 1)
     return dbgz_fail(ctx, DBGZ_ERR_INVALID_ARGUMENT, "block sizes must be positive");
   DevBuf work;
@@ -542,19 +557,10 @@ int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b
   double *dvec = (double *)work.p, *svec = dvec + n, *ovec = svec + n, *eps0 = ovec + n;
   int64_t *rank = (int64_t *)(eps0 + 2);
   cudaStream_t st = ctx->stream;
-  cudaMemsetAsync(dvec, 0, sizeof(double) * 3 * n, st);
-  k_diag_absmax<<<1, 1024, 0, st>>>(M, n, eps0);
+  k_chol_init<<<1, 1024, 0, st>>>(M, n, eps0, scale, perm, rank, dvec, 3 * n);
   dbgz_count_launch(ctx);
-  int st_ = scale_correlation(ctx, M, n, a, b, scale, 1);
+  int st_ = scale_correlation(ctx, M, n, a, b, scale, 1, true);
   if (st_) { dbgz_release(work); dbgz_release(work2); return st_; }
-  {
-    std::vector<int64_t> id(n);
-    for (int64_t i = 0; i < n; ++i) id[i] = i;
-    cudaMemcpyAsync(perm, id.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, st);
-    int64_t rn = n;
-    cudaMemcpyAsync(rank, &rn, sizeof(int64_t), cudaMemcpyHostToDevice, st);
-    cudaStreamSynchronize(st);
-  }
   int rc = DBGZ_OK;
   for (int64_t iv0 = 0; iv0 < n && rc == DBGZ_OK; iv0 += bs4) {
     int64_t iv1 = std::min(n - 1, iv0 + bs4 - 1);
@@ -602,12 +608,10 @@ int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b
   // Blocks after a rank failure return immediately (they read rank < n),
   // and the Schur updates after it only touch entries the reference leaves
   // as scratch beyond the failure point; callers reject rank < n anyway.
-  if (rc == DBGZ_OK) {
-    cudaError_t e = cudaMemcpyAsync(rank_host, rank, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) rc = dbgz_fail(ctx, DBGZ_ERR_CUDA, "cholesky_genz: %s", cudaGetErrorString(e));
-  }
-  cudaStreamSynchronize(st);
+  // (the buffers go back to the pool in stream order, their kernels in flight)
+  if (rc == DBGZ_OK && cudaGetLastError() != cudaSuccess) rc = dbgz_fail(ctx, DBGZ_ERR_CUDA, "cholesky_genz: launch failed");
+  if (rc == DBGZ_OK && cudaMemcpyAsync(rank_out, rank, sizeof(int64_t), cudaMemcpyDefault, st) != cudaSuccess)
+    rc = dbgz_fail(ctx, DBGZ_ERR_CUDA, "cholesky_genz: %s", cudaGetErrorString(cudaGetLastError()));
   dbgz_release(work);
   dbgz_release(work2);
   return rc;
@@ -734,14 +738,14 @@ int dbgz_band_dev(dbgz_ctx *ctx, int64_t d, double *U, int64_t band) {
   return DBGZ_OK;
 }
 
-int dbgz_make_targets(dbgz_problem *p) {
+int dbgz_make_targets(dbgz_problem *p, double *head) {
   dbgz_ctx *ctx = p->ctx;
   int64_t n = p->d;
   DBGZ_TRY(dbgz_ensure(ctx, p->tgt64, sizeof(TargetParams64) * n));
   DBGZ_TRY(dbgz_ensure(ctx, p->tgt32, sizeof(TargetParams32) * n));
   k_targets<<<(unsigned)((n + 127) / 128), 128, 0, ctx->stream>>>(
       (const double *)p->U.p, n, (const double *)p->a.p, (const double *)p->b.p,
-      (TargetParams64 *)p->tgt64.p, (TargetParams32 *)p->tgt32.p);
+      (TargetParams64 *)p->tgt64.p, (TargetParams32 *)p->tgt32.p, head);
   dbgz_count_launch(p->ctx);
   DBGZ_CUDA_TRY(ctx, cudaGetLastError());
   return DBGZ_OK;

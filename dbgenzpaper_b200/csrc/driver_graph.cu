@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "loop_simt_kernels.cuh"
 
 extern "C" int dbgz_first_dim_cdf(dbgz_problem *p);  // api.cu
 
@@ -30,28 +31,16 @@ struct DriverState {
   double res, err;
 };
 
-// One block of 32 threads.  Shift k: Neumaier sum of its tile sums in tile
-// order and the running mean, as simt::k_finalize; then the mean over the
+// One block.  A warp per shift: the sum of its tile sums and the running mean,
+// as simt::k_finalize; then the mean over the
 // shifts and 3 * sd (the host loop's sd_ref), in FP64 with explicit
 // round-to-nearest operations so that no contraction changes a bit.
 __global__ void k_adaptive_step(const double *partials, int64_t tps, int64_t n_reps, int64_t m, double *reps,
                                 DriverState *S, int64_t max_pts, double max_abs_err, cudaGraphConditionalHandle h) {
   const int64_t n0 = S->npts;
-  for (int64_t k = threadIdx.x; k < n_reps; k += blockDim.x) {
-    const double *pk = partials + k * tps;
-    double s = 0.0, c = 0.0;
-    for (int64_t t = 0; t < tps; ++t) {
-      const double x = pk[t];
-      const double tt = __dadd_rn(s, x);
-      if (fabs(s) >= fabs(x)) c = __dadd_rn(c, __dadd_rn(__dsub_rn(s, tt), x));
-      else c = __dadd_rn(c, __dadd_rn(__dsub_rn(x, tt), s));
-      s = tt;
-    }
-    s = __dadd_rn(s, c);
-    const double inv_tot = __ddiv_rn(1.0, (double)(n0 + m));
-    const double mean_rep = __dmul_rn(s, inv_tot);
-    const double old_weight = __dmul_rn((double)n0, inv_tot);
-    reps[k] = fma(reps[k], old_weight, mean_rep);
+  for (int64_t k = threadIdx.x >> 5; k < n_reps; k += blockDim.x >> 5) {
+    const double s = simt::warp_shift_sum(partials + k * tps, tps);
+    if ((threadIdx.x & 31) == 0) reps[k] = simt::running_mean(s, n0, m, reps + k);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -155,7 +144,7 @@ int build_graph(dbgz_problem *p, int precision, const PassArgs &pa, int64_t tps,
   const int64_t lc = ctx->launch_count;
   int rc = run_pass(p, pa, precision, (double *)p->partials.p, n_tiles);
   if (rc == DBGZ_OK) {
-    k_adaptive_step<<<1, 32, 0, st>>>((const double *)p->partials.p, tps, p->opts.n_reps, p->opts.m,
+    k_adaptive_step<<<1, 512, 0, st>>>((const double *)p->partials.p, tps, p->opts.n_reps, p->opts.m,
                                       (double *)p->reps.p, (DriverState *)p->drv_state.p, p->opts.max_pts,
                                       p->opts.max_abs_err, h);
   }
@@ -194,7 +183,6 @@ extern "C" int dbgz_pnorm_graph(dbgz_problem *p, int precision, double *result, 
   const dbgz_opts &o = p->opts;
   const int64_t n_reps = o.n_reps, m = o.m;
   DBGZ_TRY(dbgz_first_dim_cdf(p));
-  if (precision != DBGZ_PREC_FP64 && !p->U32.p) DBGZ_TRY(dbgz_make_U32(p));
   const int64_t tps = (m + 127) / 128;
   const int64_t n_tiles = tps * n_reps;
   DBGZ_TRY(dbgz_ensure(ctx, p->partials, sizeof(double) * n_tiles));

@@ -95,7 +95,6 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   const int64_t tps = (m + 127) / 128, n_tiles = tps * n_reps;
   const size_t esz = precision == DBGZ_PREC_FP64 ? 8 : 4;
   DBGZ_TRY(dbgz_first_dim_cdf(p));
-  if (precision != DBGZ_PREC_FP64 && !p->U32.p && !sparse) DBGZ_TRY(dbgz_make_U32(p));
   if (!p->Ub.p) DBGZ_TRY(dbgz_make_Ub(p));
   // Banded problems with dimension checkpoints (ctx->grad_ckpt_seg > 0): the
   // forward pass keeps, every `seg` y-indices, each sample's ring of the last
@@ -193,7 +192,6 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
 
   DBGZ_TRY(dbgz_ensure(ctx, p->partials, sizeof(double) * n_tiles));
   DBGZ_TRY(dbgz_ensure(ctx, p->reps, sizeof(double) * n_reps));
-  DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(p->reps.p, 0, sizeof(double) * n_reps, ctx->stream));
   DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
   const bool prof = ctx->profiling;
   const int64_t launches0 = ctx->launch_count;

@@ -123,6 +123,7 @@ struct dbgz_problem {
   // workspaces
   DevBuf yws, partials, reps;
   double c1 = 0, dc1 = 0;
+  double head[3] = {};  // a_0, b_0, U_00
   bool c1_ready = false;
   // every lower bound is -inf: the forward loops take the one-sided step
   // (dbgz::StepFp64LowerInf / StepFp32LowerInf, the same bits)
@@ -132,13 +133,13 @@ struct dbgz_problem {
 // ---- factorisation (chol.cu) -------------------------------------------
 int dbgz_chol_genz_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b, int64_t bs1,
                        int64_t bs2, int64_t bs3, int64_t bs4, int64_t *perm, double *scale,
-                       int64_t *rank_host);
+                       int64_t *rank_out);  // rank_out: host or device; in stream order, no synchronisation
 int dbgz_chol_rowmax_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b, int64_t bs1, int64_t bs2,
                          int64_t bs3, int64_t bs4, int64_t *perm, double *scale, int64_t *rank_host);
 int dbgz_chol_classic_dev(dbgz_ctx *ctx, int64_t n, double *M, double *a, double *b,
                           int64_t bs1, int64_t bs2, int64_t bs3, int64_t bs4, double *scale);
 int dbgz_truncate_dev(dbgz_ctx *ctx, int64_t n, double *U, double eps_T);
-int dbgz_make_targets(dbgz_problem *p);
+int dbgz_make_targets(dbgz_problem *p, double *head);  // head: 3 doubles on the device
 int dbgz_band_dev(dbgz_ctx *ctx, int64_t d, double *U, int64_t band);
 int dbgz_make_U32(dbgz_problem *p);
 int dbgz_make_Ub(dbgz_problem *p);
@@ -199,6 +200,8 @@ struct PassArgs {
 };
 int dbgz_loop_simt(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,
                    int64_t n_tiles);
+// whether dbgz_loop_umma runs the kernel with bounded waits (ctx->d_status)
+bool dbgz_umma_waits(const dbgz_problem *p, int precision);
 int dbgz_loop_umma(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,
                    int64_t n_tiles);
 // The warp-level FP32 loop: dense split-BF16, and banded (p->bandwidth).

@@ -66,6 +66,7 @@ int launch_simt(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   P.partials = partials;
   const bool adj = pa.kind == kLoopAdjoint;
   if (adj && !p->Ub.p) DBGZ_TRY(dbgz_make_Ub(p));
+  if (sizeof(T) == 4 && !p->U32.p) DBGZ_TRY(dbgz_make_U32(p));
   if (sizeof(T) == 8) {
     P.U = (const T *)(adj ? p->Ub.p : p->U.p);
     P.tgt = (const typename TgtOf<T>::type *)p->tgt64.p;
@@ -148,7 +149,7 @@ int dbgz_loop_simt(dbgz_problem *p, const PassArgs &pa, int precision, double *p
 int dbgz_finalize_pass(dbgz_problem *p, const double *partials, int64_t tiles_per_shift,
                        int64_t n_pts0, int64_t m, double *reps) {
   int64_t n_reps = p->opts.n_reps;
-  k_finalize<<<(unsigned)((n_reps + 127) / 128), 128, 0, p->ctx->stream>>>(
+  k_finalize<<<(unsigned)((n_reps + 3) / 4), 128, 0, p->ctx->stream>>>(
       partials, tiles_per_shift, n_reps, n_pts0, m, reps);
   dbgz_count_launch(p->ctx);
   DBGZ_CUDA_TRY(p->ctx, cudaGetLastError());

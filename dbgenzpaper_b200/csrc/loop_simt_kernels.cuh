@@ -234,26 +234,40 @@ __global__ void __launch_bounds__(NT, 2) k_genz_simt_batch(const SimtParams<T> *
   }
 }
 
-// Per shift: Neumaier-compensated sum of its tile sums in tile order, then
-// the running mean of src/qmc.jl:437-442.
-static __global__ void k_finalize(const double *partials, int64_t tiles_per_shift, int64_t n_reps,
-                           int64_t n_pts0, int64_t m, double *reps) {
-  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= n_reps) return;
-  const double *pk = partials + k * tiles_per_shift;
+// Compensated sum of pk[0..n) by one warp: lane l takes entries l, l + 32, ...
+// in order (Neumaier), and the lanes' sums and compensations are added in a
+// fixed tree, with the error of every addition kept.  Explicit rounding, so
+// that every kernel that calls it gives the same bits.  (One thread per shift,
+// a load after the other, took 11 us for 79 tiles and 24 us for 256.)
+__device__ __forceinline__ double warp_shift_sum(const double *pk, int64_t n) {
   double s = 0.0, c = 0.0;
-  for (int64_t t = 0; t < tiles_per_shift; ++t) {
-    double x = pk[t];
-    double tt = s + x;
-    if (fabs(s) >= fabs(x)) c += (s - tt) + x;
-    else c += (x - tt) + s;
+  auto add = [&](double x, double cx) {
+    const double tt = __dadd_rn(s, x);
+    const double e = fabs(s) >= fabs(x) ? __dadd_rn(__dsub_rn(s, tt), x) : __dadd_rn(__dsub_rn(x, tt), s);
+    c = __dadd_rn(__dadd_rn(c, cx), e);
     s = tt;
+  };
+  for (int64_t t = threadIdx.x & 31; t < n; t += 32) add(pk[t], 0.0);
+  for (int o = 16; o > 0; o >>= 1) {
+    const double so = __shfl_xor_sync(0xffffffffu, s, o), co = __shfl_xor_sync(0xffffffffu, c, o);
+    add(so, co);
   }
-  s += c;
-  double inv_tot = 1.0 / (double)(n_pts0 + m);
-  double mean_rep = s * inv_tot;
-  double old_weight = (double)n_pts0 * inv_tot;
-  reps[k] = fma(reps[k], old_weight, mean_rep);
+  return __dadd_rn(s, c);
+}
+// The running mean of src/qmc.jl:437-442 after n_pts0 earlier points per shift
+// (a first pass does not read the old mean).
+__device__ __forceinline__ double running_mean(double s, int64_t n_pts0, int64_t m, const double *old) {
+  const double inv_tot = __ddiv_rn(1.0, (double)(n_pts0 + m));
+  const double mean_rep = __dmul_rn(s, inv_tot);
+  return n_pts0 > 0 ? fma(*old, __dmul_rn((double)n_pts0, inv_tot), mean_rep) : mean_rep;
+}
+// One warp per shift: its tile sums, then the running mean.
+static __global__ void k_finalize(const double *partials, int64_t tiles_per_shift, int64_t n_reps,
+                                  int64_t n_pts0, int64_t m, double *reps) {
+  const int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (k >= n_reps) return;
+  const double s = warp_shift_sum(partials + k * tiles_per_shift, tiles_per_shift);
+  if ((threadIdx.x & 31) == 0) reps[k] = running_mean(s, n_pts0, m, reps + k);
 }
 
 }  // namespace simt

@@ -1098,14 +1098,17 @@ void dbgz_umma_batch_free(UmmaBatchPlan *B) {
   delete B;
 }
 
+bool dbgz_umma_waits(const dbgz_problem *p, int precision) {
+  // up to d = 512 the warp-level loop is faster (split BF16, 1.6e6 to 2e6
+  // samples, forward / with gradient: 1.47x / 1.30x at d = 100, 1.24x / 1.17x
+  // at d = 300, 1.15x / 1.11x at d = 400, 0.94x / 0.96x at d = 600)
+  constexpr int64_t kWarpLoopMaxD = 512;
+  return precision != DBGZ_PREC_FP32_SPLIT_BF16 || p->d > kWarpLoopMaxD;
+}
+
 int dbgz_loop_umma(dbgz_problem *p, const PassArgs &pa, int precision, double *partials, int64_t n_tiles) {
-  if (precision == DBGZ_PREC_FP32_SPLIT_BF16) {
-    // up to d = 512 the warp-level loop is faster (split BF16, 1.6e6 to 2e6
-    // samples, forward / with gradient: 1.47x / 1.30x at d = 100, 1.24x / 1.17x
-    // at d = 300, 1.15x / 1.11x at d = 400, 0.94x / 0.96x at d = 600)
-    constexpr int64_t kWarpLoopMaxD = 512;
-    if (p->d <= kWarpLoopMaxD) return dbgz_loop_w32(p, pa, partials, n_tiles);
+  if (!dbgz_umma_waits(p, precision)) return dbgz_loop_w32(p, pa, partials, n_tiles);
+  if (precision == DBGZ_PREC_FP32_SPLIT_BF16)
     return launch_umma<DBGZ_PREC_FP32_SPLIT_BF16>(p, pa, partials, n_tiles);
-  }
   return launch_umma<DBGZ_PREC_FP32_TF32>(p, pa, partials, n_tiles);
 }

@@ -190,13 +190,7 @@ extern "C" int dbgz_pnorm_pass_noalloc(int64_t d, const double *U, const double 
   P.yws = yws;
   P.partials = partials;
   f64::k_genz_f64<NoallocPolicy><<<(unsigned)grid, f64::NT, sizeof(f64::Smem), st>>>(P);
-  // the output accumulates a running mean with weight 0 for a first pass:
-  // clear it so that stale or uninitialised contents cannot leak in
-  if (cudaMemsetAsync(qmc_reps, 0, sizeof(double) * n_reps, st) != cudaSuccess) {
-    cudaGetLastError();
-    return DBGZ_ERR_CUDA;
-  }
-  k_finalize<<<(unsigned)((n_reps + 127) / 128), 128, 0, st>>>(partials, tps, n_reps, 0, m,
+  k_finalize<<<(unsigned)((n_reps + 3) / 4), 128, 0, st>>>(partials, tps, n_reps, 0, m,
                                                                  qmc_reps);
   if (cudaGetLastError() != cudaSuccess) return DBGZ_ERR_CUDA;
   return DBGZ_OK;

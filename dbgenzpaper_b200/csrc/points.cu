@@ -15,6 +15,8 @@
 // richtmyer_mat!/sobol_mat! entry points of the ABI.
 #include "internal.cuh"
 #include <algorithm>
+#include <cmath>
+#include <vector>
 
 namespace {
 
@@ -123,17 +125,17 @@ extern "C" int dbgz_sobol_dirnums(int64_t dims, uint32_t *V) {
 
 extern "C" int dbgz_sqrt_primes(int64_t n, double *q) {
   if (n < 0 || (n > 0 && !q)) return DBGZ_ERR_INVALID_ARGUMENT;
-  int64_t p = 1;
-  for (int64_t i = 0; i < n; ++i) {
-    p = p + 1;  // nextprime(p + 1)
-    for (;; ++p) {
-      bool prime = p >= 2;
-      for (int64_t f = 2; f * f <= p && prime; ++f)
-        if (p % f == 0) prime = false;
-      if (prime) break;
-    }
-    double sp = sqrt((double)p);
-    q[i] = sp - floor(sp);
+  // the first n primes by a sieve (the n-th prime is below n (ln n + ln ln n)
+  // from n = 6 on)
+  const double ln = std::log((double)(n > 6 ? n : 6));
+  const int64_t lim = (int64_t)((double)(n > 6 ? n : 6) * (ln + std::log(ln))) + 1;
+  std::vector<bool> composite(lim + 1, false);
+  int64_t i = 0;
+  for (int64_t p = 2; p <= lim && i < n; ++p) {
+    if (composite[p]) continue;
+    for (int64_t f = p * p; f <= lim; f += p) composite[f] = true;
+    const double sp = sqrt((double)p);
+    q[i++] = sp - floor(sp);
   }
   return DBGZ_OK;
 }
