@@ -374,10 +374,13 @@ __device__ __forceinline__ void genz_block_smem(double *M, int64_t n, double *a,
 //     (k_genz_gather, k_genz_scatter in chol.cu);
 //   * each CTA sends its best candidate, factor entries included, to every CTA
 //     of the cluster: one cluster barrier a pivot, after which every CTA takes
-//     the pivot, its root and y_i by itself.
+//     the pivot by itself.  The pivot's root and normalised bounds are its
+//     score's (the same operands, the same bits), and a warp of its own forms
+//     y_i under the others' dot products.
 // Same operations in the same order as genz_block_dev: the same bits.
 constexpr int kPivSlots = 64;     // candidates per CTA
-constexpr int kPivThreads = 128;  // two per candidate
+constexpr int kPivThreads = 160;  // two per candidate, and the y_i warp
+constexpr int kPivSlotThreads = 128;
 constexpr int kPivCtas = 8;       // CTAs per cluster at most
 constexpr int kPivMax = 64;       // pivots per block at most
 constexpr int kPivPanel = kPivSlots * kPivCtas;
@@ -385,17 +388,17 @@ constexpr int kPivPanel = kPivSlots * kPivCtas;
 struct PivRec {
   unsigned long long key;  // argmin_key of the score, ~0: no candidate
   unsigned idx, pad;       // position << 16 | slot
-  double m_raw, o, a, b, s;
+  double m_raw, o, m_pp, nb, na;  // :533-541
   double f[kPivMax];
 };
 struct PivSmem {
   PivRec rec[2][kPivCtas];
   double f[kPivMax][kPivSlots];  // m[pivot, candidate]
-  double o[kPivSlots], s[kPivSlots], m[kPivSlots], a[kPivSlots], b[kPivSlots];
-  double fd[kPivMax];
+  double o[kPivSlots], m[kPivSlots], r[kPivSlots], nb[kPivSlots], na[kPivSlots];
+  double fd[kPivMax], y;
   double tab[2][29];
-  unsigned long long wk[2][kPivThreads / 32];
-  unsigned wi[2][kPivThreads / 32];
+  unsigned long long wk[2][kPivSlotThreads / 32];
+  unsigned wi[2][kPivSlotThreads / 32];
 };
 // What the block leaves for the permutation of M.
 struct PivOut {
@@ -440,10 +443,11 @@ __device__ __forceinline__ void genz_block_cluster(const double *M, int64_t n, d
   const double is2pi = dm_div(2.0, dm_sqrt(dm_mul(2.0, M_PI)));
   const double eps0 = eps0_ptr[0];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, C = (int)gridDim.x, cid = (int)blockIdx.x;
-  const int sl = tid >> 1, slot = cid * kPivSlots + sl;
+  const bool ywarp = tid >= kPivSlotThreads;
+  const int sl = ywarp ? 0 : tid >> 1, slot = cid * kPivSlots + sl;
   const bool upper = (tid & 1) == 0;  // this thread's bound: b (even) or a (odd)
   const int len = (int)(ii1 - i0 + 1);
-  const bool has = slot < len;
+  const bool has = !ywarp && slot < len;
   const int64_t g = i0 + slot;
   if (rank[0] < n) {  // an earlier block already stopped
     if (cid == 0 && tid == 0) *out.done = -1;
@@ -465,10 +469,6 @@ __device__ __forceinline__ void genz_block_cluster(const double *M, int64_t n, d
   const double xb = upper ? bv : av;
   double ds = 0.0, s = has ? svec[g] : 0.0;
   int pos = slot;
-  if (upper) {
-    sm.a[sl] = av;
-    sm.b[sl] = bv;
-  }
   const int np = (int)(i1 - i0 + 1);
   int done = np;
   cluster_sync_all();  // every CTA's shared memory is up (and this one's tables)
@@ -476,30 +476,36 @@ __device__ __forceinline__ void genz_block_cluster(const double *M, int64_t n, d
   for (int u = 0; u < np; ++u) {
     const int par = u & 1;
     // pivot scores (:500-512) and the CTA's least (argmin :514)
-    const double m_raw = dm_sub(gd, ds);
-    const double m_kk = m_raw < 0 ? 0.0 : dm_sqrt(m_raw);
-    const double e = det_erf_tab(sm.tab, dm_mul(dm_div(dm_sub(xb, s), m_kk), c2));
-    const double eo = __shfl_xor_sync(0xffffffffu, e, 1);
-    const double o = upper ? dm_sub(e, eo) : dm_sub(eo, e);
     unsigned long long key = ~0ull;
     unsigned idx = ~0u;
-    if (has && pos >= u && upper) {
-      key = argmin_key(o);
-      idx = ((unsigned)pos << 16) | (unsigned)slot;
-    }
-    if (upper) {
-      sm.o[sl] = o;
-      sm.s[sl] = s;
-      sm.m[sl] = m_raw;
-    }
-    warp_argmin(key, idx);
-    if (lane == 0) {
-      sm.wk[par][wid] = key;
-      sm.wi[par][wid] = idx;
+    if (!ywarp) {
+      const double m_raw = dm_sub(gd, ds);
+      const double m_kk = m_raw < 0 ? 0.0 : dm_sqrt(m_raw);
+      const double nrm = dm_div(dm_sub(xb, s), m_kk);
+      const double e = det_erf_tab(sm.tab, dm_mul(nrm, c2));
+      const double eo = __shfl_xor_sync(0xffffffffu, e, 1);
+      const double o = upper ? dm_sub(e, eo) : dm_sub(eo, e);
+      if (upper) {
+        sm.o[sl] = o;
+        sm.m[sl] = m_raw;
+        sm.r[sl] = m_kk;
+        sm.nb[sl] = nrm;
+        if (has && pos >= u) {
+          key = argmin_key(o);
+          idx = ((unsigned)pos << 16) | (unsigned)slot;
+        }
+      } else {
+        sm.na[sl] = nrm;
+      }
+      warp_argmin(key, idx);
+      if (lane == 0) {
+        sm.wk[par][wid] = key;
+        sm.wi[par][wid] = idx;
+      }
     }
     __syncthreads();
-    key = lane < kPivThreads / 32 ? sm.wk[par][lane] : ~0ull;
-    idx = lane < kPivThreads / 32 ? sm.wi[par][lane] : ~0u;
+    key = lane < kPivSlotThreads / 32 ? sm.wk[par][lane] : ~0ull;
+    idx = lane < kPivSlotThreads / 32 ? sm.wi[par][lane] : ~0u;
     warp_argmin(key, idx);
     // this CTA's best candidate to every CTA (two buffers: a CTA that is a
     // step ahead writes the other one)
@@ -519,9 +525,9 @@ __device__ __forceinline__ void genz_block_cluster(const double *M, int64_t n, d
           case 1: dst = &R->idx; v = idx; break;
           case 2: dst = &R->m_raw; v = (unsigned long long)__double_as_longlong(sm.m[lb]); break;
           case 3: dst = &R->o; v = (unsigned long long)__double_as_longlong(sm.o[lb]); break;
-          case 4: dst = &R->a; v = (unsigned long long)__double_as_longlong(sm.a[lb]); break;
-          case 5: dst = &R->b; v = (unsigned long long)__double_as_longlong(sm.b[lb]); break;
-          case 6: dst = &R->s; v = (unsigned long long)__double_as_longlong(sm.s[lb]); break;
+          case 4: dst = &R->m_pp; v = (unsigned long long)__double_as_longlong(sm.r[lb]); break;
+          case 5: dst = &R->nb; v = (unsigned long long)__double_as_longlong(sm.nb[lb]); break;
+          case 6: dst = &R->na; v = (unsigned long long)__double_as_longlong(sm.na[lb]); break;
           default: break;
         }
       }
@@ -545,33 +551,50 @@ __device__ __forceinline__ void genz_block_cluster(const double *M, int64_t n, d
       done = u;
       break;
     }
-    const double m_pp = dm_sqrt(p_raw);
-    if (tid == 0) sm.fd[u] = m_pp;
-    // the ascending fma chain over the block's pivots
-    double acc = 0.0;
+    const double m_pp = R.m_pp;
+    if (ywarp) {
+      // y_i (:538-546), a side in half of the lanes (x / 2 = x * 0.5)
+      const double nrm = upper ? R.nb : R.na;
+      const double ex = det_exp(dm_mul(-dm_mul(nrm, nrm), 0.5));
+      const double exo = __shfl_xor_sync(0xffffffffu, ex, 1);
+      const double yi = dm_div(dm_mul(upper ? dm_sub(exo, ex) : dm_sub(ex, exo), is2pi), R.o);
+      if (lane == 0) {
+        sm.y = yi;
+        sm.fd[u] = m_pp;
+      }
+      __syncwarp();
+      asm volatile("bar.arrive 1, %0;" ::"n"(kPivThreads) : "memory");
+      continue;
+    }
+    // the ascending fma chain over the block's pivots, eight loaded ahead
+    double acc = 0.0, m = 0.0;
     int t = 0;
-    for (; t + 8 <= u; t += 8) {
+    if (u >= 8) {
       double x[8], y[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        x[q] = sm.f[t + q][sl];
-        y[q] = R.f[t + q];
+        x[q] = sm.f[q][sl];
+        y[q] = R.f[q];
+      }
+      for (t = 8; t + 8 <= u; t += 8) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          acc = dm_fma(x[q], y[q], acc);
+          x[q] = sm.f[t + q][sl];
+          y[q] = R.f[t + q];
+        }
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q) acc = dm_fma(x[q], y[q], acc);
     }
     for (; t < u; ++t) acc = dm_fma(sm.f[t][sl], R.f[t], acc);
-    // y_i (:538-546), each side's term in half of the threads (x / 2 = x * 0.5)
-    const double nrm = dm_div(dm_sub(upper ? R.b : R.a, R.s), m_pp);
-    const double ex = det_exp(dm_mul(-dm_mul(nrm, nrm), 0.5));
-    const double exo = __shfl_xor_sync(0xffffffffu, ex, 1);
-    const double yi = dm_div(dm_mul(upper ? dm_sub(exo, ex) : dm_sub(ex, exo), is2pi), R.o);
     if (live) {  // :547-570
-      const double m = dm_div(dm_sub(mij, acc), m_pp);
+      m = dm_div(dm_sub(mij, acc), m_pp);
       ds = dm_add(ds, dm_mul(m, m));
-      s = dm_add(s, dm_mul(yi, m));
       if (upper) sm.f[u][sl] = m;
     }
+    asm volatile("bar.sync 1, %0;" ::"n"(kPivThreads) : "memory");  // y_i is there
+    if (live) s = dm_add(s, dm_mul(sm.y, m));
   }
   __syncthreads();
   if (has && upper) {
