@@ -11,8 +11,9 @@
 //
 // Used by the Cholesky adjoint (chol_adjoint.cu: U Ubar', U^-1 (.) U^-T,
 // U'U) and by the FP64 factor gradient dU[l, t] = sum_n y[l][n] (p sbar)[t][n]
-// (grad.cu).  No library GEMM: the same operand sizes run on CUDA cores in
-// FP64 (the B200's FP64 rate is the same on CUDA cores and tensor cores).
+// (grad.cu).  No library GEMM.  The products are mma.m8n8k4.f64: the FP64 rate
+// is that of scalar FMAs (16 a cycle and scheduler, measured), with an eighth of
+// the instructions and a third of the shared-memory reads.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -20,7 +21,7 @@
 namespace dense64 {
 namespace {  // internal linkage: every translation unit that includes this gets its own copy
 
-constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
+constexpr int BM = 64, BN = 64, BK = 8, NST = 4, NT = 256;
 
 enum OutMode {
   kOutFull = 0,         // every C entry
@@ -34,6 +35,11 @@ struct GemmArgs {
   int64_t lda = 0;
   const double *B = nullptr;
   int64_t ldb = 0;
+  // > 0 (op = transpose only): the operand is stored in tiles of 128 k, element
+  // (k, i) at ((k / 128) * rows + i) * 128 + k % 128 (GradIO's layout): the rows
+  // a step reads lie on few pages (with rows 1 MB apart the factor gradient at
+  // d = 150 took 457 us)
+  int64_t a_rows = 0, b_rows = 0;
   double *C = nullptr;
   int64_t ldc = 0;
   // k range per output tile [i0, i1) x [j0, j1): from max(i0 if kmin_row,
@@ -70,14 +76,27 @@ __device__ __forceinline__ double out_value(int out, int64_t i, int64_t j, doubl
   return v;
 }
 
-// One 64 x 64 output tile per CTA (256 threads, 4 x 4 per thread: rows
-// tx + 16 a, columns ty + 16 b), k in steps of 16 through shared memory, the
-// next step's operands loaded into registers while this one is used.
+__device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+// 8 bytes global -> shared, or zero
+__device__ __forceinline__ void cp8(double *dst, const double *src, bool v) {
+  const int n = v ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(n)
+               : "memory");
+}
+
+// One 64 x 64 output tile per CTA (8 warps of 16 x 32), k in steps of 8
+// through a four-stage cp.async ring; row strides of 68 doubles make the
+// fragment reads conflict-free.
 // TA / TB: op(A) = A' / op(B) = B'.
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(NT) k_gemm64(const GemmArgs g) {
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN + 1];
+  __shared__ double As[NST][BK][BM + 4];
+  __shared__ double Bs[NST][BK][BN + 4];
   const int64_t tiles_n = (g.n + BN - 1) / BN;
   const int64_t ti = blockIdx.x / tiles_n, tj = blockIdx.x % tiles_n;
   const int64_t i0 = ti * BM, j0 = tj * BN;
@@ -94,81 +113,85 @@ __global__ void __launch_bounds__(NT) k_gemm64(const GemmArgs g) {
     k1 = s1 < k1 ? s1 : k1;
     k0 = s0;
   }
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  double acc[4][4];
+  const int tid = threadIdx.x, warp = tid >> 5, fr = (tid & 31) >> 2, fk = tid & 3;
+  const int wm = (warp & 3) * 16, wn = (warp >> 2) * 32;
+  double acc[2][4][2];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-
-  // operand loads: 1024 elements per tile, 4 per thread
-  double ra[4], rb[4];
-  auto load = [&](int64_t kk) {
+    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  const int64_t steps = k1 > k0 ? (k1 - k0 + BK - 1) / BK : 0;
+  auto load = [&](int64_t step) {
+    if (step < steps) {
+      const int st = (int)(step % NST);
+      const int64_t kk = k0 + step * BK;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + NT * q;
-      // A tile element (i, k): op N -> i fastest (coalesced), op T -> k fastest
-      const int ai = TA ? e / BK : e % BM, ak = TA ? e % BK : e / BM;
-      const int64_t gi = i0 + ai, gk = kk + ak;
-      ra[q] = (gi < i1 && gk < k1) ? (TA ? g.A[gk + gi * g.lda] : g.A[gi + gk * g.lda]) : 0.0;
-      // B tile element (k, j): op N -> k fastest, op T -> j fastest
-      const int bj = TB ? e % BN : e / BK, bk = TB ? e / BN : e % BK;
-      const int64_t gj = j0 + bj, gk2 = kk + bk;
-      rb[q] = (gj < j1 && gk2 < k1) ? (TB ? g.B[gj + gk2 * g.ldb] : g.B[gk2 + gj * g.ldb]) : 0.0;
+      for (int q = 0; q < BM * BK / NT; ++q) {
+        const int e = tid + NT * q;
+        // A tile element (i, k): op N -> i fastest (coalesced), op T -> k fastest
+        const int ai = TA ? e / BK : e % BM, ak = TA ? e % BK : e / BM;
+        const int64_t gi = i0 + ai, gk = kk + ak;
+        const bool va = gi < i1 && gk < k1;
+        const int64_t oa = !TA ? gi + gk * g.lda : (g.a_rows > 0 ? ((gk >> 7) * g.a_rows + gi) * 128 + (gk & 127) : gk + gi * g.lda);
+        cp8(&As[st][ak][ai], va ? g.A + oa : g.A, va);
+        // B tile element (k, j): op N -> k fastest, op T -> j fastest
+        const int bj = TB ? e % BN : e / BK, bk = TB ? e / BN : e % BK;
+        const int64_t gj = j0 + bj, gk2 = kk + bk;
+        const bool vb = gj < j1 && gk2 < k1;
+        const int64_t ob = TB ? gj + gk2 * g.ldb : (g.b_rows > 0 ? ((gk2 >> 7) * g.b_rows + gj) * 128 + (gk2 & 127) : gk2 + gj * g.ldb);
+        cp8(&Bs[st][bk][bj], vb ? g.B + ob : g.B, vb);
+      }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  auto store = [&]() {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = tid + NT * q;
-      const int ai = TA ? e / BK : e % BM, ak = TA ? e % BK : e / BM;
-      As[ak][ai] = ra[q];
-      const int bj = TB ? e % BN : e / BK, bk = TB ? e / BN : e % BK;
-      Bs[bk][bj] = rb[q];
-    }
-  };
-  if (k0 < k1) load(k0);
-  for (int64_t kk = k0; kk < k1; kk += BK) {
+  for (int p = 0; p < NST - 1; ++p) load(p);
+  for (int64_t s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
     __syncthreads();
-    store();
-    __syncthreads();
-    if (kk + BK < k1) load(kk + BK);
+    load(s + NST - 1);
+    const int st = (int)(s % NST);
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      double av[4], bv[4];
+    for (int k4 = 0; k4 < BK; k4 += 4) {
+      double av[2], bv[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = As[k][tx + 16 * a];
+      for (int a = 0; a < 2; ++a) av[a] = As[st][k4 + fk][wm + 8 * a + fr];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = Bs[k][ty + 16 * b];
+      for (int b = 0; b < 4; ++b) bv[b] = Bs[st][k4 + fk][wn + 8 * b + fr];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
+        for (int b = 0; b < 4; ++b) dmma(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
     }
   }
   if (g.splits > 1) {
     double *pt = g.partial + (((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * BM) * BN;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) pt[(ty + 16 * b) * BM + tx + 16 * a] = acc[a][b];
+      for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) pt[(wn + 8 * b + 2 * fk + e) * BM + wm + 8 * a + fr] = acc[a][b][e];
     return;
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int64_t i = i0 + tx + 16 * a, j = j0 + ty + 16 * b;
-      if (i >= i1 || j >= j1) continue;
-      bool w;
-      double v = acc[a][b];
-      if (g.accumulate) v += g.C[i + j * g.ldc];
-      v = out_value(g.out, i, j, v, w);
-      if (w) g.C[i + j * g.ldc] = v;
-    }
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int64_t i = i0 + wm + 8 * a + fr, j = j0 + wn + 8 * b + 2 * fk + e;
+        if (i >= i1 || j >= j1) continue;
+        bool w;
+        double v = acc[a][b][e];
+        if (g.accumulate) v += g.C[i + j * g.ldc];
+        v = out_value(g.out, i, j, v, w);
+        if (w) g.C[i + j * g.ldc] = v;
+      }
 }
 
-// Sum of the split partial tiles in split order, then the output rule.
+// Sum of the split partial tiles in split order, then the output rule
+// (blockIdx.y: a part of the tile's entries).
 __global__ void k_gemm64_reduce(const GemmArgs g, int64_t n_tiles) {
   const int64_t tiles_n = (g.n + BN - 1) / BN;
   const int64_t tile = blockIdx.x;
@@ -176,11 +199,12 @@ __global__ void k_gemm64_reduce(const GemmArgs g, int64_t n_tiles) {
   const int64_t i0 = ti * BM, j0 = tj * BN;
   const int64_t i1 = i0 + BM < g.m ? i0 + BM : g.m, j1 = j0 + BN < g.n ? j0 + BN : g.n;
   if (!tile_needed(g, i0, i1, j0, j1)) return;
-  for (int e = threadIdx.x; e < BM * BN; e += blockDim.x) {
+  for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < BM * BN; e += blockDim.x * gridDim.y) {
     const int li = e % BM, lj = e / BM;
     const int64_t i = i0 + li, j = j0 + lj;
     if (i >= i1 || j >= j1) continue;
     double v = 0.0;
+#pragma unroll 8
     for (int s = 0; s < g.splits; ++s) v += g.partial[((int64_t)s * n_tiles + tile) * BM * BN + e];
     bool w;
     if (g.accumulate) v += g.C[i + j * g.ldc];
@@ -205,7 +229,7 @@ inline cudaError_t gemm64(const GemmArgs &g, cudaStream_t st, int *launches = nu
   k_gemm64<TA, TB><<<dim3((unsigned)tiles, (unsigned)(g.splits > 1 ? g.splits : 1)), NT, 0, st>>>(g);
   if (launches) ++*launches;
   if (g.splits > 1) {
-    k_gemm64_reduce<<<(unsigned)tiles, 256, 0, st>>>(g, tiles);
+    k_gemm64_reduce<<<dim3((unsigned)tiles, BM * BN / 256), 256, 0, st>>>(g, tiles);
     if (launches) ++*launches;
   }
   return cudaGetLastError();

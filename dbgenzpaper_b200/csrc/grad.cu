@@ -29,6 +29,7 @@ __global__ void k_reduce_rows(const double *ga, const double *gb, const double *
   if (t >= d) return;
   const int64_t r0 = blockIdx.y * chunk, r1 = r0 + chunk < rows ? r0 + chunk : rows;
   double a = 0.0, b = 0.0, u = 0.0;
+#pragma unroll 8
   for (int64_t r = r0; r < r1; ++r) {
     a += ga[r * d + t];
     b += gb[r * d + t];
@@ -43,6 +44,7 @@ __global__ void k_reduce_chunks(const double *csum, int64_t n_chunks, int64_t d,
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // i in [0, 3d)
   if (i >= 3 * d) return;
   double v = 0.0;
+#pragma unroll 16
   for (int64_t c = 0; c < n_chunks; ++c) v += csum[c * 3 * d + i];
   out[i] = accumulate ? out[i] + v : v;
 }
@@ -183,13 +185,6 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   // the adjoint pass writes per-tile values too (zeros); keep them away from
   // the forward pass's tile sums, which are reduced after the last chunk
   double *adj_tiles = (double *)take(8 * (size_t)n_tiles);
-  if (!sparse && precision == DBGZ_PREC_FP64) {
-    // rows the passes leave unwritten (y row d-1, sbar row 0) enter the DGEMM:
-    // clear them (the FP32 GEMM computes l < t only, which never reads them)
-    DBGZ_CUDA_TRY(ctx, cudaMemsetAsync((char *)ga.y + esz * (size_t)(d - 1) * N, 0, esz * N, ctx->stream));
-    DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(ga.sbar, 0, esz * N, ctx->stream));
-  }
-
   DBGZ_TRY(dbgz_ensure(ctx, p->partials, sizeof(double) * n_tiles));
   DBGZ_TRY(dbgz_ensure(ctx, p->reps, sizeof(double) * n_reps));
   DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
@@ -296,15 +291,15 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
     if (want_U) {
       const int nc = (int)((t1 - t0) * 128);
       if (precision == DBGZ_PREC_FP64) {
-        // dU[l, t] (+)= sum_n Y[n, l] SB[n, t] for l < t, Y and SB the stored
-        // rows as N x d column-major matrices
+        // dU[l, t] (+)= sum_n Y[n, l] SB[n, t] for l < t on the stored state
+        // (rows the passes leave unwritten, y row d-1 and sbar row 0, only enter
+        // entries that are not written)
         dense64::GemmArgs g;
         g.m = g.n = d;
         g.k = nc;
         g.A = (const double *)ga.y;
-        g.lda = N;
+        g.a_rows = g.b_rows = d;
         g.B = (const double *)ga.sbar;
-        g.ldb = N;
         g.C = (double *)dU;
         g.ldc = d;
         g.out = dense64::kOutStrictUpper;

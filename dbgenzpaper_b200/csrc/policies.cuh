@@ -62,14 +62,12 @@ struct Staged {
 };
 
 // Arrays of the forward state kept for the adjoint, `rows` (= d) indices per
-// sample, N samples.  FP64: [index][sample] (row stride N, the layout of the
-// library DGEMM of the factor gradient).  FP32: tile-major, [tile][index]
-// [128 samples of the tile]: one tile's state is one contiguous block of
-// d x 512 bytes, so a step's 128 values are one coalesced 512-byte row and
-// the factor-gradient GEMM reads 32-sample slices of many rows from a few
-// pages (with row stride N = 2^21 samples every row lies on its own page of
-// the GPU's address translation; this layout took the d = 1000 gradient from
-// 92 to 81 ms).
+// sample, N samples, tile-major: [tile][index][128 samples of the tile].  One
+// tile's state is one contiguous block of d rows, so a step's 128 values are one
+// coalesced row and the factor-gradient GEMM reads slices of many rows from a
+// few pages (with rows of N samples each row lies on pages of its own: the FP32
+// d = 1000 gradient went from 92 to 81 ms, the FP64 factor gradient at d = 150
+// from 457 us as measured beside dense64::GemmArgs).
 template <typename T>
 struct GradIO {
   int64_t N = 0, rows = 0;
@@ -85,18 +83,11 @@ struct GradIO {
   // rows row0 .. row0 + rows - 1)
   int64_t row0 = 0;
   int store_p = 0;    // a forward pass without stored state still writes p (checkpointed gradients)
-  __device__ __forceinline__ int64_t at(int64_t row, int64_t g) const {
-    if (sizeof(T) == 4) return ((g >> 7) * rows + (row - row0)) * 128 + (g & 127);
-    return (row - row0) * N + g;
-  }
-  // at(row, g) = at0(g) + row * stride(): the sample's part, computed once per
-  // tile, and a row stride (a constant 128 for FP32), so that a step's
-  // address is one multiply-add on the row (constant offsets inside a chunk)
-  __device__ __forceinline__ int64_t at0(int64_t g) const {
-    if (sizeof(T) == 4) return ((g >> 7) * rows - row0) * 128 + (g & 127);
-    return g - row0 * N;
-  }
-  __device__ __forceinline__ int64_t stride() const { return sizeof(T) == 4 ? (int64_t)128 : N; }
+  // row `row` of sample g is at at0(g) + row * stride(): the sample's part,
+  // computed once per tile, so that a step's address is one multiply-add on the
+  // row (constant offsets inside a chunk)
+  __device__ __forceinline__ int64_t at0(int64_t g) const { return ((g >> 7) * rows - row0) * 128 + (g & 127); }
+  __device__ __forceinline__ int64_t stride() const { return 128; }
 };
 
 // Asynchronous global -> shared copy of `BYTES` (4, 8 or 16) bytes, or zeros
