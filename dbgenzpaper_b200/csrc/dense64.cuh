@@ -121,29 +121,45 @@ __global__ void __launch_bounds__(NT) k_gemm64(const GemmArgs g) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
   const int64_t steps = k1 > k0 ? (k1 - k0 + BK - 1) / BK : 0;
+  // a thread's elements: (i, k) of the A tile, op N -> i fastest (coalesced), op
+  // T -> k fastest; (k, j) of the B tile, op N -> k fastest, op T -> j fastest;
+  // offsets from the step's first k
+  constexpr int EL = BM * BK / NT;
+  int64_t oa[EL], ob[EL];
+  int ka[EL], kb[EL];
+  bool va[EL], vb[EL];
+#pragma unroll
+  for (int q = 0; q < EL; ++q) {
+    const int e = tid + NT * q;
+    const int ai = TA ? e / BK : e % BM, bj = TB ? e % BN : e / BK;
+    ka[q] = TA ? e % BK : e / BM;
+    kb[q] = TB ? e / BN : e % BK;
+    const int64_t gi = i0 + ai, gj = j0 + bj;
+    va[q] = gi < i1;
+    vb[q] = gj < j1;
+    oa[q] = !TA ? gi + ka[q] * g.lda : (g.a_rows > 0 ? gi * 128 : gi * g.lda) + ka[q];
+    ob[q] = TB ? gj + kb[q] * g.ldb : (g.b_rows > 0 ? gj * 128 : gj * g.ldb) + kb[q];
+  }
   auto load = [&](int64_t step) {
     if (step < steps) {
       const int st = (int)(step % NST);
       const int64_t kk = k0 + step * BK;
+      // (a step never straddles a 128-k tile: k0 and 128 are multiples of BK)
+      const double *A = g.A + (!TA ? kk * g.lda : (g.a_rows > 0 ? (kk >> 7) * g.a_rows * 128 + (kk & 127) : kk));
+      const double *B = g.B + (TB ? kk * g.ldb : (g.b_rows > 0 ? (kk >> 7) * g.b_rows * 128 + (kk & 127) : kk));
 #pragma unroll
-      for (int q = 0; q < BM * BK / NT; ++q) {
+      for (int q = 0; q < EL; ++q) {
         const int e = tid + NT * q;
-        // A tile element (i, k): op N -> i fastest (coalesced), op T -> k fastest
-        const int ai = TA ? e / BK : e % BM, ak = TA ? e % BK : e / BM;
-        const int64_t gi = i0 + ai, gk = kk + ak;
-        const bool va = gi < i1 && gk < k1;
-        const int64_t oa = !TA ? gi + gk * g.lda : (g.a_rows > 0 ? ((gk >> 7) * g.a_rows + gi) * 128 + (gk & 127) : gk + gi * g.lda);
-        cp8(&As[st][ak][ai], va ? g.A + oa : g.A, va);
-        // B tile element (k, j): op N -> k fastest, op T -> j fastest
-        const int bj = TB ? e % BN : e / BK, bk = TB ? e / BN : e % BK;
-        const int64_t gj = j0 + bj, gk2 = kk + bk;
-        const bool vb = gj < j1 && gk2 < k1;
-        const int64_t ob = TB ? gj + gk2 * g.ldb : (g.b_rows > 0 ? ((gk2 >> 7) * g.b_rows + gj) * 128 + (gk2 & 127) : gk2 + gj * g.ldb);
-        cp8(&Bs[st][bk][bj], vb ? g.B + ob : g.B, vb);
+        const bool a = va[q] && kk + ka[q] < k1, b = vb[q] && kk + kb[q] < k1;
+        cp8(&As[st][ka[q]][TA ? e / BK : e % BM], a ? A + oa[q] : g.A, a);
+        cp8(&Bs[st][kb[q]][TB ? e % BN : e / BK], b ? B + ob[q] : g.B, b);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  // a warp whose 16 x 32 part is not needed only loads
+  const bool mine = i0 + wm < i1 && j0 + wn < j1 &&
+                    tile_needed(g, i0 + wm, i0 + wm + 16, j0 + wn, j0 + wn + 32);
 #pragma unroll
   for (int p = 0; p < NST - 1; ++p) load(p);
   for (int64_t s = 0; s < steps; ++s) {
@@ -151,6 +167,7 @@ __global__ void __launch_bounds__(NT) k_gemm64(const GemmArgs g) {
     __syncthreads();
     load(s + NST - 1);
     const int st = (int)(s % NST);
+    if (mine)
 #pragma unroll
     for (int k4 = 0; k4 < BK; k4 += 4) {
       double av[2], bv[4];

@@ -229,19 +229,20 @@ struct StepFp64 {
       u = shiftv + x;
       u = u > 1.0 ? u - 1.0 : u;
     } else {
+      // n_bits <= 32: the shifted integer has at most 32 bits
       const int L = g.n_bits;
-      const uint64_t mask = (L >= 64) ? ~0ull : ((1ull << L) - 1);
+      const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
       const uint32_t xw = g.sobol_staged ? x0 : sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j));
-      uint64_t xi = (uint64_t)xw & mask;
-      uint64_t sh = g.sobol_staged ? 0ull : g.ushift[k * (d - 1) + l] & mask;
-      u = (double)((xi ^ sh) & mask) * ldexp(1.0, -L);
+      const uint32_t sh = g.sobol_staged ? 0u : (uint32_t)g.ushift[k * (d - 1) + l];
+      u = (double)((xw ^ sh) & mask) * __hiloint2double((1023 - L) << 20, 0);  // 2^-L
     }
     return fabs(fma(u, 2.0, -1.0));
   }
   // y_l from w
   __device__ __forceinline__ double quantile_w(double w) const {
     double u = fma(w, dc, c);
-    u = fmin(fmax(u, DBL_EPSILON), 1.0 - DBL_EPSILON);
+    u = u > DBL_EPSILON ? u : DBL_EPSILON;
+    u = u < 1.0 - DBL_EPSILON ? u : 1.0 - DBL_EPSILON;
     return sqrt2_erfinv_tab(*tab, fma(2.0, u, -1.0));
   }
   template <bool kIntTent = true>  // (no effect in FP64)

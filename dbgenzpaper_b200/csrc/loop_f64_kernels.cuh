@@ -125,28 +125,46 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
         for (int ni = 0; ni < G / 8; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
       const int64_t k0 = P.band > 0 && g0 + 1 > P.band ? (g0 + 1 - P.band) / KC * KC : 0;
       const int nch = (int)((g0 - k0) / KC);
-      int64_t yrow = P.band > 0 ? k0 % P.ring : 0;
+      // this thread's share of a chunk: four 16-byte pieces of its warp's Y rows
+      // and UP coefficients; sources advance by a chunk.  (No rows past the
+      // group's last 8 targets; in those, rows past the last target read the
+      // last one's, for sums that nobody takes.)
+      constexpr int UP = G * KC / NT;
+      const double *ysrc = Yw + (P.band > 0 ? k0 % P.ring : 0) * TS + 32 * warp;
+      const double *usrc[UP];
+      uint32_t ydst[KC / 2], udst[UP];
+#pragma unroll
+      for (int e = 0; e < KC / 2; ++e) {
+        const int kk = (lane + 32 * e) >> 4, row = 2 * (lane & 15);
+        ydst[e] = (uint32_t)__cvta_generic_to_shared(&sm.u.ring.Y[0][warp][0][0] + swz(kk, row));
+      }
+#pragma unroll
+      for (int e = 0; e < UP; ++e) {
+        const int t = (tid + NT * e) >> 3, kk = tid & 7;
+        usrc[e] = P.U + (g0 + 1 + t < d ? g0 + 1 + t : d - 1) * d + k0 + kk;
+        udst[e] = (uint32_t)__cvta_generic_to_shared(&sm.u.ring.U[0][t][kk]);
+      }
       int is = 0, ich = 0;  // stage and number of the next chunk to issue
       auto issue = [&]() {
         if (ich < nch) {
-          const int st = is;
-          const int64_t l0 = k0 + (int64_t)ich * KC;
+          const double *ys = ysrc + (lane >> 4) * TS + 2 * (lane & 15);
 #pragma unroll
-          for (int e = 0; e < KC * 16 / 32; ++e) {
-            const int pc = lane + 32 * e, kk = pc >> 4, row = 2 * (pc & 15);
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.u.ring.Y[st][warp][0][0] + swz(kk, row));
-            const double *src = Yw + (yrow + kk) * TS + 32 * warp + row;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-          }
+          for (int e = 0; e < KC / 2; ++e)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             ydst[e] + is * (uint32_t)sizeof(sm.u.ring.Y[0])),
+                         "l"(ys + 2 * e * TS)
+                         : "memory");
+          ysrc += KC * TS;
+          if (ysrc == yend - tid + 32 * warp) ysrc -= P.ring * TS;
 #pragma unroll
-          for (int e = 0; e < G * KC / NT; ++e) {
-            const int el = tid + NT * e, t = el >> 3, kk = el & 7;
-            if (t < 8 * nt) {
-              const bool v = g0 + 1 + t < d;
-              pol::cp_async_or_zero<8>(&sm.u.ring.U[st][t][kk], v ? P.U + (g0 + 1 + t) * d + l0 + kk : P.U, v);
-            }
+          for (int e = 0; e < UP; ++e) {
+            if (((tid + NT * e) >> 3) < 8 * nt)
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                               udst[e] + is * (uint32_t)sizeof(sm.u.ring.U[0])),
+                           "l"(usrc[e])
+                           : "memory");
+            usrc[e] += KC;
           }
-          yrow = yrow + KC == P.ring ? 0 : yrow + KC;
         }
         pol::cp_async_commit();
         ++ich;
@@ -213,14 +231,14 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
           for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
             for (int e = 0; e < 2; ++e) c[mi][e] = g0 > 0 ? S[swz(q8 + 2 * fk + e, 8 * mi + fr)] : 0.0;
-          const bool v = g0 + q8 + 1 + fr < d;
-          const double *Ut = v ? P.U + (g0 + q8 + 1 + fr) * d + g0 + fk : P.U;
+          const int64_t tr = g0 + q8 + 1 + fr;  // (past the last target: its sums are not taken)
+          const double *Ut = P.U + (tr < d ? tr : d - 1) * d + g0 + fk;
           // 8 y's (two k steps) a round; the next round's coefficients are
           // loaded while this one's products run
-          double b0v = v ? __ldg(Ut) : 0.0, b1v = v ? __ldg(Ut + 4) : 0.0;
+          double b0v = __ldg(Ut), b1v = __ldg(Ut + 4);
           for (int kk = 0; kk < q8; kk += 8) {
             const double c0v = b0v, c1v = b1v;
-            if (kk + 8 < q8 && v) {
+            if (kk + 8 < q8) {
               b0v = __ldg(Ut + kk + 8);
               b1v = __ldg(Ut + kk + 12);
             }

@@ -78,7 +78,8 @@ struct NormNode {
 
 // erf(x) for any x that is not NaN (|x| > 6 rounds to 1)
 __device__ __forceinline__ double erf_tab(const NormTab &t, double x) {
-  const NormNode n(fmin(fabs(x), 6.0));
+  const double ax = fabs(x);
+  const NormNode n(ax < 6.0 ? ax : 6.0);
   const double2 eg = t.eg[n.i];
   const double ec = fma(-(eg.y * n.delta), n.q<false>(), eg.x);
   return copysign(1.0 - ec, x);
@@ -91,7 +92,7 @@ __device__ __forceinline__ double erf_tab(const NormTab &t, double x) {
 // 3e-16 at x0 = 5).  1 / g(x0) = exp(2 a delta + delta^2) / g(a).
 __device__ __forceinline__ double sqrt2_erfinv_tab(const NormTab &t, double v) {
   const double q = 1.0 - fabs(v);
-  const double x0 = fmin((double)(-0.70710678f * phi_inv_lower_f32(0.5f * (float)q)), 6.0);
+  const double x0 = (double)fminf(-0.70710678f * phi_inv_lower_f32(0.5f * (float)q), 6.0f);
   const NormNode n(x0);
   const double2 eg = t.eg[n.i];
   const double res = fma(-(eg.y * n.delta), n.q<true>(), eg.x - q);

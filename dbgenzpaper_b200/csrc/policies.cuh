@@ -411,13 +411,11 @@ struct Adjoint {
       u = (double)sg.shv[li] + x;
       u = u > 1.0 ? u - 1.0 : u;
     } else {
-      const int L = gen.n_bits;
-      const uint64_t mask = (L >= 64) ? ~0ull : ((1ull << L) - 1);
-      const uint64_t xi =
-          (uint64_t)(staged ? xs : dbgz::sobol_warp(gen.V + t * 32, (uint64_t)(gen.sobol_first + gen.gen_base + j))) &
-          mask;
-      const uint64_t sh = staged ? 0ull : gen.ushift[k * (d - 1) + t] & mask;
-      u = (double)((xi ^ sh) & mask) * ldexp(1.0, -L);
+      const int L = gen.n_bits;  // <= 32
+      const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
+      const uint32_t xi = staged ? xs : dbgz::sobol_warp(gen.V + t * 32, (uint64_t)(gen.sobol_first + gen.gen_base + j));
+      const uint32_t sh = staged ? 0u : (uint32_t)gen.ushift[k * (d - 1) + t];
+      u = (double)((xi ^ sh) & mask) * __hiloint2double((1023 - L) << 20, 0);  // 2^-L
     }
     return fabs(fma(u, 2.0, -1.0));
   }
