@@ -197,20 +197,22 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
   return t;
 }
 
-// s[8 .. 8+N) += sum_k ys[k] * u[k * kUld + 0 .. N), k = 0..7 in order.
-template <int N>
-__device__ __forceinline__ void rank8_update(float (&s)[BK], const float (&ys)[8], const float *u) {
+// s[8 G .. 8 G + 8) = s[8 G + 8 .. 8 G + 16) + sum_k ys[k] * u[k * kUld + 0 .. 8),
+// k = 0..7 in order: a chunk's y's into 8 later targets, moved down by 8 on
+// the way (the first product's addend), which leaves no moves of s[].  One
+// copy of the code per group of 8 targets: the sample threads' chunk loop is
+// larger than the instruction cache with one copy per (chunk, group) --
+// instruction fetches ran at 91% of the cache's rate -- and takes 19.3 ms
+// with this form against 20.4 ms (d = 1000, 1.6e6 lattice points).
+template <int G>
+__device__ __forceinline__ void rank8_shift(float (&s)[BK], const float (&ys)[8], const float *u) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const float4 *row = reinterpret_cast<const float4 *>(u + k * kUld);
+    const float4 v = row[0], w = row[1];
+    const float uu[8] = {v.x, v.y, v.z, v.w, w.x, w.y, w.z, w.w};
 #pragma unroll
-    for (int q = 0; q < N / 4; ++q) {
-      const float4 v = row[q];
-      s[8 + 4 * q] = fmaf(ys[k], v.x, s[8 + 4 * q]);
-      s[9 + 4 * q] = fmaf(ys[k], v.y, s[9 + 4 * q]);
-      s[10 + 4 * q] = fmaf(ys[k], v.z, s[10 + 4 * q]);
-      s[11 + 4 * q] = fmaf(ys[k], v.w, s[11 + 4 * q]);
-    }
+    for (int t = 0; t < 8; ++t) s[8 * G + t] = fmaf(ys[k], uu[t], k == 0 ? s[8 * G + 8 + t] : s[8 * G + t]);
   }
 }
 
@@ -610,6 +612,18 @@ __global__ void __launch_bounds__(NT, 2) k_genz_umma(const __grid_constant__ Umm
               uint32_t hi[4], lo[4];
               float ys[8];
               pl.chunk_begin(lbase + 8 * ch, nval - 8 * ch);
+              // the chunk's points, which do not depend on the recursion, ahead
+              // of it: their FP64 and conversion latencies overlap each other
+              // (21.4 -> 20.4 ms at that size)
+              typename Policy::Point pt[8];
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const int li = 8 * ch + k;
+                uint32_t xs = 0u;
+                if constexpr (Policy::kSobolTable)
+                  if (pl.gen.sobol_staged) xs = sob_lane.at(ms->sob[cur], li);
+                pt[k] = pl.point(sgc, li, lbase + li, xs);
+              }
               // full chunks (all but the last of a problem) run without the
               // per-step bounds test: one uniform branch per chunk instead of 8
               auto steps = [&](auto checked, auto fast) {
@@ -622,8 +636,10 @@ __global__ void __launch_bounds__(NT, 2) k_genz_umma(const __grid_constant__ Umm
                   uint32_t xs = 0u;
                   if constexpr (Policy::kSobolTable)
                     if (pl.gen.sobol_staged) xs = sob_lane.at(ms->sob[cur], li);
-                  if constexpr (decltype(fast)::value)
-                    y = pl.emit_k_fast(sgc, li, l, k, xs);
+                  if constexpr (Policy::kDeferTail)
+                    y = pl.emit_k_at(sgc, li, l, k, pt[k]);
+                  else if constexpr (decltype(fast)::value)
+                    y = pl.emit_k_fast_at(sgc, li, l, k, pt[k]);
                   else
                     y = pl.emit_k(sgc, li, l, k, xs);
                   const float4 *urow = reinterpret_cast<const float4 *>(&ublk[li][8 * ch]);
@@ -664,12 +680,6 @@ __global__ void __launch_bounds__(NT, 2) k_genz_umma(const __grid_constant__ Umm
               }
               pl.chunk_end(lbase + 8 * ch, nval - 8 * ch);
               if constexpr (Policy::kDeferTail) pl.tail_repair(sgc, s, 8 * ch, lbase + 8 * ch);
-              switch (ch) {
-                case 0: rank8_update<24>(s, ys, &ublk[0][8]); break;
-                case 1: rank8_update<16>(s, ys, &ublk[8][16]); break;
-                case 2: rank8_update<8>(s, ys, &ublk[16][24]); break;
-                default: break;
-              }
               if (MODE == DBGZ_PREC_FP32_SPLIT_BF16) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -690,10 +700,15 @@ __global__ void __launch_bounds__(NT, 2) k_genz_umma(const __grid_constant__ Umm
                                  to_tf32(ys[4 * h2 + 3]));
                 }
               }
-#pragma unroll
-              for (int t = 0; t < BK - 8; ++t) s[t] = s[t + 8];
-#pragma unroll
-              for (int t = BK - 8; t < BK; ++t) s[t] = 0.f;
+              // the later chunks' targets, moved down by 8 on the way
+              if (ch < 3) {
+                const float *u = &ublk[8 * ch][8 * ch + 8];
+                rank8_shift<0>(s, ys, u);
+                if (ch < 2) {
+                  rank8_shift<1>(s, ys, u + 8);
+                  if (ch < 1) rank8_shift<2>(s, ys, u + 16);
+                }
+              }
             }
           }
           fence_proxy_async_smem();

@@ -601,7 +601,7 @@ struct Adjoint {
   using Point = T;
   __device__ __forceinline__ Point point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
     const int64_t t = d - 1 - l;
-    const bool has_u = t <= d - 2;
+    const bool has_u = (uint64_t)t <= (uint64_t)(d - 2);  // (t < 0: a step past the last, formed ahead and not used)
     if constexpr (sizeof(T) == 4) return has_u ? point_w32(sg, li, t, xs, gen.sobol_staged != 0) : 0.0f;
     else return has_u ? point_w(sg, li, t, xs, gen.sobol_staged != 0) : 0.0;
   }
