@@ -379,8 +379,8 @@ struct StepFp32 {
     const float t = fmaf(q.w, dc, lo);
     const bool lower = t <= 0.5f;
     const float arg = lower ? t : fmaf(q.w1, dc, up);
-    const float y = phi_inv_lower_f32(fmaxf(arg, kEps));
-    return lower ? y : -y;
+    const float y = phi_inv_mag_f32(fmaxf(arg, kEps));
+    return lower ? -y : y;
   }
   template <bool kIntTent = true>
   __device__ __forceinline__ float quantile(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l, double qv,
@@ -407,16 +407,17 @@ struct StepFp32 {
   // within a factor 2).
   __device__ __forceinline__ float cdf_core(float s, float a, float b, float inv_u, float &x0, float &x1,
                                             bool &need64) {
-    const float xa = fminf(fmaxf((a - s) * inv_u, -9.0f), 9.0f);
-    const float xb = fminf(fmaxf((b - s) * inv_u, -9.0f), 9.0f);
-    const float ea = tail_mass_f32(fabsf(xa));  // mass beyond |alpha| on its side
-    const float eb = tail_mass_f32(fabsf(xb));
+    const float va = (a - s) * inv_u, vb = (b - s) * inv_u;
+    const float ea = tail_mass_f32(fminf(fabsf(va), 9.0f));  // mass beyond |alpha| on its side
+    const float eb = tail_mass_f32(fminf(fabsf(vb), 9.0f));
     // both bounds in the upper tail (hi_t), both in the lower tail (lo_t), or
     // alpha < 0 < beta; selects rather than branches (the step is a serial
-    // chain per sample, and branch resolution stalls it)
-    const bool hi_t = xa >= 0.0f, lo_t = !hi_t && xb <= 0.0f;
+    // chain per sample, and branch resolution stalls it).  A NaN argument
+    // counts as -9.
+    const bool hi_t = va >= 0.0f, lo_t = !hi_t && !(vb > 0.0f);
     const float d = hi_t ? ea - eb : (lo_t ? eb - ea : (1.0f - ea) - eb);
     need64 = (hi_t && eb > 0.5f * ea) || (lo_t && ea > 0.5f * eb);
+    const float xa = fminf(fmaxf(va, -9.0f), 9.0f), xb = fminf(fmaxf(vb, -9.0f), 9.0f);
     x0 = hi_t ? xa : -xb;
     x1 = hi_t ? xb : -xa;
     lo = hi_t ? 1.0f - ea : ea;
@@ -469,11 +470,11 @@ struct StepFp32LowerInf : StepFp32 {
     ea9 = tail_mass_f32(nine);
   }
   __device__ __forceinline__ float cdf_core(float s, float b, float inv_u, bool &need64) {
-    const float xb = fminf(fmaxf((b - s) * inv_u, -9.0f), 9.0f);
+    const float vb = (b - s) * inv_u;
     const float ea = ea9;
-    const float eb = tail_mass_f32(fabsf(xb));
+    const float eb = tail_mass_f32(fminf(fabsf(vb), 9.0f));
     // alpha = -9 < 0: the interval is in the lower tail or straddles 0
-    const bool lo_t = xb <= 0.0f;
+    const bool lo_t = !(vb > 0.0f);
     const float d = lo_t ? eb - ea : (1.0f - ea) - eb;
     need64 = lo_t && ea > 0.5f * eb;
     lo = ea;

@@ -8,8 +8,9 @@
 // function of Press, Teukolsky, Vetterling and Flannery (Numerical Recipes,
 // "erfcc").  The coefficients here are our own: a least-squares fit of
 // P(t) = ln(erfcx(x)) - ln(t) on 400,001 points of [0, 9] in double
-// precision (maximum error of the fit 2.2e-7 in P).  Evaluated in FP32 with
-// one reciprocal, nine FMAs and one exp2 and no branches; the relative error
+// precision (maximum error of the fit 2.2e-7 in P), times log2(e), so that
+// t 2^(P'(t) - x (x log2 e)) takes no multiply after the polynomial.
+// Evaluated in FP32 with one reciprocal, ten FMAs and one exp2 and no branches; the relative error
 // against erfc is below 3e-6 for x <= 4.5 and below 1.5e-5 up to x = 9 (the
 // FP32 rounding of the exponent P - x^2 dominates there, where the mass is
 // below 1e-10).
@@ -45,23 +46,27 @@ __device__ __forceinline__ float rsqrt_sfu(float x) {
   return r;
 }
 
+constexpr double kL2 = 1.4426950408889634;  // log2(e)
+constexpr float kLog2e = (float)kL2;
 __device__ __forceinline__ float tail_mass_f32(float x) {
   const float t = rcp_sfu(fmaf(0.5f, x, 1.0f));
-  float p = 1.6112529716e-01f;
-  p = fmaf(p, t, -7.6098558876e-01f);
-  p = fmaf(p, t, 1.3262850294e+00f);
-  p = fmaf(p, t, -8.9638341094e-01f);
-  p = fmaf(p, t, 6.4102997549e-02f);
-  p = fmaf(p, t, -6.4260147179e-02f);
-  p = fmaf(p, t, 5.3133554076e-02f);
-  p = fmaf(p, t, 3.8353175424e-01f);
-  p = fmaf(p, t, 9.9890822443e-01f);
-  p = fmaf(p, t, -1.2654574945e+00f);
-  // z = (p - x^2) log2(e) >= -117 here, so no subnormal result is flushed
-  return 0.5f * t * exp2_sfu((p - x * x) * 1.4426950408889634f);
+  const float xl = x * kLog2e;
+  float p = (float)(1.6112529716e-01 * kL2);
+  p = fmaf(p, t, (float)(-7.6098558876e-01 * kL2));
+  p = fmaf(p, t, (float)(1.3262850294e+00 * kL2));
+  p = fmaf(p, t, (float)(-8.9638341094e-01 * kL2));
+  p = fmaf(p, t, (float)(6.4102997549e-02 * kL2));
+  p = fmaf(p, t, (float)(-6.4260147179e-02 * kL2));
+  p = fmaf(p, t, (float)(5.3133554076e-02 * kL2));
+  p = fmaf(p, t, (float)(3.8353175424e-01 * kL2));
+  p = fmaf(p, t, (float)(9.9890822443e-01 * kL2));
+  p = fmaf(p, t, (float)(-1.2654574945e+00 * kL2));
+  return 0.5f * t * exp2_sfu(fmaf(-xl, x, p));
 }
 
-// Phi^-1(p) for 0 < p <= 1/2 (the smaller tail: the step forms u or 1 - u,
+constexpr double kR2 = 1.4142135623730951;
+
+// -Phi^-1(p) for 0 < p <= 1/2 (the smaller tail: the step forms u or 1 - u,
 // whichever is below 1/2), FP32, without branches.  The form is M. Giles'
 // ("Approximating the erfinv function", GPU Computing Gems Jade, 2011):
 // with x = 1 - 2p and w = -ln(4 p (1 - p)) = -ln(1 - x^2),
@@ -69,33 +74,36 @@ __device__ __forceinline__ float tail_mass_f32(float x) {
 //   erfinv(x) = T(sqrt(w) - 4)        for w >= 5  (p down to 2.2e-16, w <= 34.7),
 // and Phi^-1(p) = -sqrt(2) erfinv(x).  P (degree 8) and T (degree 9) are our
 // own weighted least-squares fits of the relative error in double precision
-// (maximum 9.4e-8 and 5.8e-8); both are evaluated and the region selected, so
+// (maximum 9.4e-8 and 5.8e-8), the coefficients times sqrt(2); w enters as
+// -log2(4 p (1 - p)) with ln 2 in the two arguments' FMAs; both are evaluated and the region selected, so
 // the code has no branch.  Relative error in FP32 below 4e-7 for p >= 2.2e-16.
-__device__ __forceinline__ float phi_inv_lower_f32(float p) {
-  const float w = log2_sfu(4.0f * p * (1.0f - p)) * -0.69314718056f;
+__device__ __forceinline__ float phi_inv_mag_f32(float p) {
+  const float lg = log2_sfu(4.0f * p * (1.0f - p));
   const float x = fmaf(-2.0f, p, 1.0f);
-  const float tc = w - 2.5f;
-  float pc = 2.854775242e-08f;
-  pc = fmaf(pc, tc, 3.437494356e-07f);
-  pc = fmaf(pc, tc, -3.528993161e-06f);
-  pc = fmaf(pc, tc, -4.396994196e-06f);
-  pc = fmaf(pc, tc, 2.186026004e-04f);
-  pc = fmaf(pc, tc, -1.253706953e-03f);
-  pc = fmaf(pc, tc, -4.177708101e-03f);
-  pc = fmaf(pc, tc, 2.466407258e-01f);
-  pc = fmaf(pc, tc, 1.501409422e+00f);
-  const float ts = w * rsqrt_sfu(w) - 4.0f;
-  float pt = 8.193106379e-07f;
-  pt = fmaf(pt, ts, -1.490730122e-06f);
-  pt = fmaf(pt, ts, -6.624017282e-06f);
-  pt = fmaf(pt, ts, 2.765589313e-05f);
-  pt = fmaf(pt, ts, -8.117484620e-05f);
-  pt = fmaf(pt, ts, 2.877970689e-04f);
-  pt = fmaf(pt, ts, -8.563289957e-04f);
-  pt = fmaf(pt, ts, 1.256645993e-03f);
-  pt = fmaf(pt, ts, 1.009495442e+00f);
-  pt = fmaf(pt, ts, 3.839783388e+00f);
-  return -1.41421356237f * (w < 5.0f ? pc * x : pt);
+  const float tc = fmaf(lg, -0.69314718056f, -2.5f);
+  float pc = (float)(2.854775242e-08 * kR2);
+  pc = fmaf(pc, tc, (float)(3.437494356e-07 * kR2));
+  pc = fmaf(pc, tc, (float)(-3.528993161e-06 * kR2));
+  pc = fmaf(pc, tc, (float)(-4.396994196e-06 * kR2));
+  pc = fmaf(pc, tc, (float)(2.186026004e-04 * kR2));
+  pc = fmaf(pc, tc, (float)(-1.253706953e-03 * kR2));
+  pc = fmaf(pc, tc, (float)(-4.177708101e-03 * kR2));
+  pc = fmaf(pc, tc, (float)(2.466407258e-01 * kR2));
+  pc = fmaf(pc, tc, (float)(1.501409422e+00 * kR2));
+  const float ts = fmaf(-lg * rsqrt_sfu(-lg), 0.83255461116f, -4.0f);  // sqrt(w) - 4
+  float pt = (float)(8.193106379e-07 * kR2);
+  pt = fmaf(pt, ts, (float)(-1.490730122e-06 * kR2));
+  pt = fmaf(pt, ts, (float)(-6.624017282e-06 * kR2));
+  pt = fmaf(pt, ts, (float)(2.765589313e-05 * kR2));
+  pt = fmaf(pt, ts, (float)(-8.117484620e-05 * kR2));
+  pt = fmaf(pt, ts, (float)(2.877970689e-04 * kR2));
+  pt = fmaf(pt, ts, (float)(-8.563289957e-04 * kR2));
+  pt = fmaf(pt, ts, (float)(1.256645993e-03 * kR2));
+  pt = fmaf(pt, ts, (float)(1.009495442e+00 * kR2));
+  pt = fmaf(pt, ts, (float)(3.839783388e+00 * kR2));
+  return lg > -7.2134752044f ? pc * x : pt;  // w < 5
 }
+// Phi^-1(p), 0 < p <= 1/2
+__device__ __forceinline__ float phi_inv_lower_f32(float p) { return -phi_inv_mag_f32(p); }
 
 }  // namespace dbgz
