@@ -104,61 +104,57 @@ __device__ __forceinline__ uint32_t sobol_warp(const uint32_t *Vl, uint64_t idx)
 // bits), [5 + a] = V[0], V[1] XORed by the bits of a, [9 + b] = V[2..4] by
 // the bits of b.  A step then reads three words (SobolLane::at).
 //
-// sobol_stage_entries: the 32 lanes of one warp together fill entries
-// li0 .. li0 + n - 1 of a block of 32: entry li < nv is dimension l0 + dir li
-// when that lies in [0, lmax]; tile first index base0, shift row ush (the
-// shift of dimension l at ush[l]).
+// sobol_stage_block: the 128 threads r of a tile together (all lanes of their
+// four warps) fill the 32 entries of a block: entry li < nv is dimension
+// l0 + dir li when that lies in [0, lmax]; tile first index base0, shift row
+// ush (the shift of dimension l at ush[l]).  Four lanes per dimension, each
+// with 8 of its 32 direction numbers (V 16-byte aligned) and one step of the
+// recurrence: about 60 instructions of a warp per block.  (With a warp per
+// dimension and one direction number per lane it took 480, a tenth of the
+// FP32 step's instructions: batch of 256 problems 24.0 -> 20.6 ms, banded
+// d = 4000 FP32 pass 12.4 -> 10.5 and gradient 10.1 -> 8.3, FP64 d = 2000
+// 3.90 -> 3.63.)
 constexpr int kSobolRow = 17;  // words per staged dimension
-template <int UNROLL>
-__device__ __forceinline__ void sobol_stage_entries(uint32_t (*tab)[kSobolRow], const uint32_t *V,
-                                                    const uint64_t *ush, uint64_t base0, int64_t l0, int dir,
-                                                    int64_t lmax, int nv, int li0, int n) {
-  const uint64_t B = base0 & ~31ull;
-  const uint32_t gB = (uint32_t)(B ^ (B >> 1));
-  const int ln = (int)(threadIdx.x & 31);
-  // lanes 1..4: bit 5 + ctz(c + ln) of the recurrence (c = B / 32)
-  const int zb = (ln >= 1 && ln <= 4) ? 5 + __ffsll((long long)((B >> 5) + (uint64_t)ln)) - 1 : 32;
-#pragma unroll UNROLL
-  for (int q = 0; q < n; ++q) {
-    const int li = li0 + q;
-    const int64_t l = l0 + dir * li;
-    const bool ok = li < nv && l >= 0 && l <= lmax;
-    // x(B): lane k contributes V[k] when bit k of gray(B) is set
-    const uint32_t vk = ok ? __ldg(V + l * 32 + ln) : 0u;
-    uint32_t t = ((gB >> ln) & 1u) ? vk : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t ^= __shfl_xor_sync(0xffffffffu, t, o);
-    uint32_t v[5];
-#pragma unroll
-    for (int e = 0; e < 5; ++e) v[e] = __shfl_sync(0xffffffffu, vk, e);
-    // x(B + 32 ln) = x(B) ^ XOR_{s = 1..ln} (V[4] ^ V[5 + ctz(c + s)]), lanes 0..4
-    const uint32_t vz = __shfl_sync(0xffffffffu, vk, zb & 31);
-    uint32_t term = (ln >= 1 && ln <= 4) ? v[4] ^ (zb < 32 ? vz : 0u) : 0u;
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, term, o);
-      if (ln >= o) term ^= u;
-    }
-    const uint32_t sh = (ln < 5 && ok) ? (uint32_t)__ldg(ush + l) : 0u;
-    uint32_t x;
-    if (ln < 5) {
-      x = t ^ term ^ sh;
-    } else if (ln < 9) {
-      const int a = ln - 5;
-      x = ((a & 1) ? v[0] : 0u) ^ ((a & 2) ? v[1] : 0u);
-    } else {
-      const int b = ln - 9;
-      x = ((b & 1) ? v[2] : 0u) ^ ((b & 2) ? v[3] : 0u) ^ ((b & 4) ? v[4] : 0u);
-    }
-    if (ln < 17) tab[li][ln] = x;
-  }
-}
-// The 128 threads r of a tile together (all lanes of their four warps), warp
-// w filling entries 8w..8w+7.
 __device__ __forceinline__ void sobol_stage_block(uint32_t (*tab)[kSobolRow], const uint32_t *V,
                                                   const uint64_t *ush, uint64_t base0, int64_t l0, int dir,
                                                   int64_t lmax, int nv, int r) {
-  sobol_stage_entries<8>(tab, V, ush, base0, l0, dir, lmax, nv, 8 * (r >> 5), 8);
+  const uint64_t B = base0 & ~31ull;
+  const int li = r >> 2, qd = r & 3;
+  const int64_t l = l0 + dir * li;
+  const bool ok = li < nv && l >= 0 && l <= lmax;
+  const uint32_t *Vl = V + (ok ? l : 0) * 32;
+  // x(B): direction number k when bit k of gray(B) is set
+  const uint4 *Vq = reinterpret_cast<const uint4 *>(Vl + 8 * qd);
+  uint4 w0 = __ldg(Vq), w1 = __ldg(Vq + 1);
+  // step s = qd + 1 of the recurrence: bit 5 + ctz(c + s), c = B / 32
+  const int zb = 5 + __ffsll((long long)((B >> 5) + (uint64_t)(qd + 1))) - 1;
+  uint32_t term = zb < 32 ? __ldg(Vl + zb) : 0u;
+  const uint32_t sh = ok ? (uint32_t)__ldg(ush + l) : 0u;
+  if (!ok) w0 = w1 = make_uint4(0u, 0u, 0u, 0u), term = 0u;
+  const uint32_t gq = (uint32_t)(B ^ (B >> 1)) >> (8 * qd);
+  const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+  uint32_t t = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) t ^= ((gq >> k) & 1u) ? w[k] : 0u;
+  t ^= __shfl_xor_sync(0xffffffffu, t, 1);
+  t ^= __shfl_xor_sync(0xffffffffu, t, 2);
+  uint32_t v[5];
+#pragma unroll
+  for (int e = 0; e < 5; ++e) v[e] = __shfl_sync(0xffffffffu, w[e], 0, 4);
+  // x(B + 32 (qd + 1)) = x(B) ^ XOR_{s = 1..qd + 1} (V[4] ^ V[5 + ctz(c + s)])
+  term ^= v[4];
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, term, o, 4);
+    if (qd >= o) term ^= u;
+  }
+  const uint32_t x = t ^ sh;
+  if (qd == 0) tab[li][0] = x;
+  tab[li][1 + qd] = x ^ term;
+  tab[li][5 + qd] = ((qd & 1) ? v[0] : 0u) ^ ((qd & 2) ? v[1] : 0u);
+  const uint32_t b = ((qd & 1) ? v[2] : 0u) ^ ((qd & 2) ? v[3] : 0u);
+  tab[li][9 + qd] = b;
+  tab[li][13 + qd] = b ^ v[4];
 }
 
 // The shifted integer of tile row r in block dimension li, for the tile
@@ -219,7 +215,6 @@ struct StepFp64 {
   // w = |2u - 1| of QMC dimension l of the sample (point index j in the pass,
   // 0-based; shift k): independent of the recursion, so that a loop can form
   // the next step's early.
-  template <bool kIntTent = true>  // (no effect in FP64)
   static __device__ __forceinline__ double tent(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l,
                                                 double qv, double shiftv, uint32_t x0, double jd) {
     double u;
@@ -245,7 +240,6 @@ struct StepFp64 {
     u = u < 1.0 - DBL_EPSILON ? u : 1.0 - DBL_EPSILON;
     return sqrt2_erfinv_tab(*tab, fma(2.0, u, -1.0));
   }
-  template <bool kIntTent = true>  // (no effect in FP64)
   __device__ __forceinline__ double quantile(const GenParams &g, int64_t d, int64_t j, int64_t k,
                                              int64_t l, double qv, double shiftv, uint32_t x0, double jd) const {
     return quantile_w(tent(g, d, j, k, l, qv, shiftv, x0, jd));
@@ -330,18 +324,12 @@ struct StepFp32 {
     up = (float)up1;
     p = dc1;
   }
-  // kIntTent: the Sobol tent transform on the integer (sobol_tent_f32), else
-  // through an FP64 u -- the same floats; the pass that stores its state for
-  // the adjoint keeps the FP64 form (measured on the banded d = 10^4,
-  // bandwidth 64 workload at 2^14 x 10 Sobol points: its
-  // gradient call 125.1 ms against 146.4 ms with the integer form)
   // The tent-transformed point of QMC dimension l, w = |2u - 1| and w1 = 1 - w
   // (jd: the lattice multiplier gen_base + j + 1): independent of the
   // recursion, so that a loop can form it early.
   struct Tent {
     float w, w1;
   };
-  template <bool kIntTent = true>
   static __device__ __forceinline__ Tent tent(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l, double qv,
                                               float shiftv, uint32_t x0, double jd) {
     Tent r;
@@ -352,22 +340,13 @@ struct StepFp32 {
       u = u > 1.0f ? u - 1.0f : u;
       r.w = fabsf(fmaf(u, 2.0f, -1.0f));
       r.w1 = 2.0f * fminf(u, 1.0f - u);  // 1 - |2u - 1|
-    } else if (kIntTent) {
+    } else {
       // n_bits <= 32: the shifted integer has at most 32 bits
       const int L = g.n_bits;
       const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
       const uint32_t xw = g.sobol_staged ? x0 : sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j));
       const uint32_t sh = g.sobol_staged ? 0u : (uint32_t)g.ushift[k * (d - 1) + l];
       sobol_tent_f32((xw ^ sh) & mask, L, r.w, r.w1);
-    } else {
-      const int L = g.n_bits;
-      const uint64_t mask = (L >= 64) ? ~0ull : ((1ull << L) - 1);
-      const uint32_t xw = g.sobol_staged ? x0 : sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j));
-      const uint64_t xi = (uint64_t)xw & mask;
-      const uint64_t sh = g.sobol_staged ? 0ull : g.ushift[k * (d - 1) + l] & mask;
-      const double u = (double)((xi ^ sh) & mask) * ldexp(1.0, -L);
-      r.w = (float)fabs(fma(u, 2.0, -1.0));
-      r.w1 = (float)(2.0 * fmin(u, 1.0 - u));
     }
     return r;
   }
@@ -382,10 +361,9 @@ struct StepFp32 {
     const float y = phi_inv_mag_f32(fmaxf(arg, kEps));
     return lower ? -y : y;
   }
-  template <bool kIntTent = true>
   __device__ __forceinline__ float quantile(const GenParams &g, int64_t d, int64_t j, int64_t k, int64_t l, double qv,
                                             float shiftv, uint32_t x0, double jd) const {
-    return quantile_w(tent<kIntTent>(g, d, j, k, l, qv, shiftv, x0, jd));
+    return quantile_w(tent(g, d, j, k, l, qv, shiftv, x0, jd));
   }
   __device__ __forceinline__ void set_form(int) {}
   // the state between two steps, as four doubles (checkpoints; the floats

@@ -840,7 +840,7 @@ int launch_umma(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   }
   if (!p->U32.p) DBGZ_TRY(dbgz_make_U32(p));
   const int Pw = 256;
-  const int smem = umma_smem_bytes<MODE>(Pw, pa.qmc_type == DBGZ_QMC_SOBOL && !adj);
+  const int smem = umma_smem_bytes<MODE>(Pw, pa.qmc_type == DBGZ_QMC_SOBOL);
   auto kern = pick_kernel<MODE>(pa, p->lower_inf);
   DBGZ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   DBGZ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
@@ -875,8 +875,7 @@ int launch_umma(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   P.gen.n_bits = pa.n_bits;
   P.gen.gen_base = pa.gen_base;
   P.gen.gen_base_dev = pa.gen_base_dev;
-  // Sobol points from the per-block staged integers (forward passes)
-  P.gen.sobol_staged = pa.qmc_type == DBGZ_QMC_SOBOL && !adj;
+  P.gen.sobol_staged = pa.qmc_type == DBGZ_QMC_SOBOL;
   P.gen.sobol_first = pa.sobol_first;
   P.gen.q = (const double *)p->q.p;
   P.gen.shift64 = (const double *)p->shifts.p;

@@ -211,7 +211,7 @@ struct Forward {
   // xs: the Sobol integer of this point in dimension l when the loop stages
   // them (GenParams::sobol_staged), else unused
   __device__ __forceinline__ T emit(const Staged<T> &sg, int li, int64_t l, uint32_t xs = 0u) {
-    const T y = st.template quantile<!STORE>(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs, jd);
+    const T y = st.quantile(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs, jd);
     if (STORE) __stcs(io.y + ga0 + l * io.stride(), y);
     return y;
   }
@@ -221,7 +221,7 @@ struct Forward {
   using Point = typename Step::Tent;
   __device__ __forceinline__ void state_begin() {}
   __device__ __forceinline__ Point point(const Staged<T> &sg, int li, int64_t l, uint32_t xs) const {
-    return Step::template tent<!STORE>(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs, jd);
+    return Step::tent(gen, d, j, k, l, sg.qv[li], sg.shv[li], xs, jd);
   }
   __device__ __forceinline__ T emit_next(const Staged<T> &, int, int64_t l, Point w) {
     const T y = st.quantile_w(w);
@@ -432,7 +432,13 @@ struct Adjoint {
       uf = uf > 1.0f ? uf - 1.0f : uf;
       return fabsf(fmaf(uf, 2.0f, -1.0f));
     }
-    return (float)point_w(sg, li, t, xs, staged);
+    const int L = gen.n_bits;
+    const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
+    const uint32_t xi = staged ? xs : dbgz::sobol_warp(gen.V + t * 32, (uint64_t)(gen.sobol_first + gen.gen_base + j));
+    const uint32_t sh = staged ? 0u : (uint32_t)gen.ushift[k * (d - 1) + t];
+    float w, w1;
+    dbgz::sobol_tent_f32((xi ^ sh) & mask, L, w, w1);
+    return w;
   }
 
   // adjoint of variable t given ybar_t; returns sbar_t (unit seed), records
