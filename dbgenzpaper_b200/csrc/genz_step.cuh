@@ -57,11 +57,16 @@ struct GenParams {
   // Sobol, nonzero when the loop stages the integers of each block of
   // dimensions per tile (sobol_stage_block) and passes the point's integer,
   // already XORed with the shift's low 32 bits (n_bits <= 32: the shift
-  // enters only there), into the step; zero: sobol_warp and the shift per
+  // enters only there) and cut to n_bits, into the step; zero: sobol_warp and the shift per
   // step.  Any first index: a tile's 128 points need the integers of 5
   // multiples of 32 and the terms of a 5-bit Gray code (SobolLane).
   int sobol_staged;
 };
+
+// The low n_bits bits of a Sobol integer (n_bits up to 32; it has no more).
+__device__ __forceinline__ uint32_t sobol_mask(int n_bits) {
+  return n_bits >= 32 ? 0xffffffffu : ((1u << n_bits) - 1u);
+}
 
 // Gray-code Sobol integer of point index idx in dimension l, computed by
 // the 32 lanes of a warp together.  Precondition: every lane of the warp
@@ -114,10 +119,11 @@ __device__ __forceinline__ uint32_t sobol_warp(const uint32_t *Vl, uint64_t idx)
 // FP32 step's instructions: batch of 256 problems 24.0 -> 20.6 ms, banded
 // d = 4000 FP32 pass 12.4 -> 10.5 and gradient 10.1 -> 8.3, FP64 d = 2000
 // 3.90 -> 3.63.)
+// mask: the low n_bits bits, which the entries are cut to.
 constexpr int kSobolRow = 17;  // words per staged dimension
 __device__ __forceinline__ void sobol_stage_block(uint32_t (*tab)[kSobolRow], const uint32_t *V,
-                                                  const uint64_t *ush, uint64_t base0, int64_t l0, int dir,
-                                                  int64_t lmax, int nv, int r) {
+                                                  const uint64_t *ush, uint32_t mask, uint64_t base0, int64_t l0,
+                                                  int dir, int64_t lmax, int nv, int r) {
   const uint64_t B = base0 & ~31ull;
   const int li = r >> 2, qd = r & 3;
   const int64_t l = l0 + dir * li;
@@ -149,12 +155,12 @@ __device__ __forceinline__ void sobol_stage_block(uint32_t (*tab)[kSobolRow], co
     if (qd >= o) term ^= u;
   }
   const uint32_t x = t ^ sh;
-  if (qd == 0) tab[li][0] = x;
-  tab[li][1 + qd] = x ^ term;
-  tab[li][5 + qd] = ((qd & 1) ? v[0] : 0u) ^ ((qd & 2) ? v[1] : 0u);
+  if (qd == 0) tab[li][0] = x & mask;
+  tab[li][1 + qd] = (x ^ term) & mask;
+  tab[li][5 + qd] = (((qd & 1) ? v[0] : 0u) ^ ((qd & 2) ? v[1] : 0u)) & mask;
   const uint32_t b = ((qd & 1) ? v[2] : 0u) ^ ((qd & 2) ? v[3] : 0u);
-  tab[li][9 + qd] = b;
-  tab[li][13 + qd] = b ^ v[4];
+  tab[li][9 + qd] = b & mask;
+  tab[li][13 + qd] = (b ^ v[4]) & mask;
 }
 
 // The shifted integer of tile row r in block dimension li, for the tile
@@ -177,16 +183,15 @@ struct SobolLane {
 
 // w = |2u - 1| and w1 = 2 min(u, 1 - u) of the Sobol point u = X 2^-L
 // (X < 2^L, 1 <= L <= 32), rounded to FP32.  Both are exact multiples of
-// 2^-(L-1) with integer parts |X - 2^(L-1)| and min(X, 2^L - X) <= 2^31, so
+// 2^-(L-1) with integer parts |X - 2^(L-1)| and 2^(L-1) less that, so
 // forming them on the integer and rounding once gives the same floats as
 // forming u in FP64 first (checked for every L on random and edge X).
 __device__ __forceinline__ void sobol_tent_f32(uint32_t X, int L, float &w, float &w1) {
   const uint32_t half = 1u << (L - 1);
-  const uint32_t dd = X >= half ? X - half : half - X;
-  const uint32_t mm = X <= half ? X : (uint32_t)((1ull << L) - X);
+  const uint32_t dd = max(X, half) - min(X, half);
   const float sc = __int_as_float((127 - (L - 1)) << 23);  // 2^-(L-1)
   w = __uint2float_rn(dd) * sc;
-  w1 = __uint2float_rn(mm) * sc;
+  w1 = __uint2float_rn(half - dd) * sc;
 }
 
 // The same integer by one thread alone (loop over the set bits).
@@ -224,12 +229,12 @@ struct StepFp64 {
       u = shiftv + x;
       u = u > 1.0 ? u - 1.0 : u;
     } else {
-      // n_bits <= 32: the shifted integer has at most 32 bits
       const int L = g.n_bits;
-      const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
-      const uint32_t xw = g.sobol_staged ? x0 : sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j));
-      const uint32_t sh = g.sobol_staged ? 0u : (uint32_t)g.ushift[k * (d - 1) + l];
-      u = (double)((xw ^ sh) & mask) * __hiloint2double((1023 - L) << 20, 0);  // 2^-L
+      uint32_t X = x0;
+      if (!g.sobol_staged)
+        X = (sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j)) ^
+             (uint32_t)g.ushift[k * (d - 1) + l]) & sobol_mask(L);
+      u = (double)X * __hiloint2double((1023 - L) << 20, 0);  // 2^-L
     }
     return fabs(fma(u, 2.0, -1.0));
   }
@@ -341,12 +346,11 @@ struct StepFp32 {
       r.w = fabsf(fmaf(u, 2.0f, -1.0f));
       r.w1 = 2.0f * fminf(u, 1.0f - u);  // 1 - |2u - 1|
     } else {
-      // n_bits <= 32: the shifted integer has at most 32 bits
-      const int L = g.n_bits;
-      const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
-      const uint32_t xw = g.sobol_staged ? x0 : sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j));
-      const uint32_t sh = g.sobol_staged ? 0u : (uint32_t)g.ushift[k * (d - 1) + l];
-      sobol_tent_f32((xw ^ sh) & mask, L, r.w, r.w1);
+      uint32_t X = x0;
+      if (!g.sobol_staged)
+        X = (sobol_warp(g.V + l * 32, (uint64_t)(g.sobol_first + g.gen_base + j)) ^
+             (uint32_t)g.ushift[k * (d - 1) + l]) & sobol_mask(g.n_bits);
+      sobol_tent_f32(X, g.n_bits, r.w, r.w1);
     }
     return r;
   }

@@ -100,8 +100,8 @@ __device__ __forceinline__ void tile(const Params &P, Smem &sm, double *Yw, int6
     pol::cp_async_commit();
     if constexpr (Policy::kSobolTable)
       if (pl.gen.sobol_staged)
-        dbgz::sobol_stage_block(st.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), base0, pl.sobol_l0(lb),
-                                Policy::kSobolDir, d - 2, nb, tid);
+        dbgz::sobol_stage_block(st.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), dbgz::sobol_mask(P.gen.n_bits),
+                                base0, pl.sobol_l0(lb), Policy::kSobolDir, d - 2, nb, tid);
   };
   // this sample's place in the workspace row of the next y (a ring of P.ring
   // rows for banded factors, a multiple of 8)

@@ -133,7 +133,7 @@ __device__ __forceinline__ void simt_tile(const SimtParams<T> &P, SimtSmem<T> &s
           pl.stage(sm.sg, P.tgt, tid, l_base, nsb);
           if constexpr (Policy::kSobolTable)
             if (pl.gen.sobol_staged)
-              dbgz::sobol_stage_block(sm.sob, P.gen.V, P.gen.ushift + k * (d - 1),
+              dbgz::sobol_stage_block(sm.sob, P.gen.V, P.gen.ushift + k * (d - 1), dbgz::sobol_mask(P.gen.n_bits),
                                       (uint64_t)(P.gen.sobol_first + pl.gen.gen_base + (j - r)),
                                       pl.sobol_l0(l_base), Policy::kSobolDir, d - 2, nsb, r);
         }

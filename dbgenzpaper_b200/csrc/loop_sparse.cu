@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(TS) k_genz_sparse(const SparseParams<T> P) {
       pl.stage(sg, P.tgt, r, i0, nb);
       if constexpr (Policy::kSobolTable)
         if (pl.gen.sobol_staged)
-          dbgz::sobol_stage_block(sob, P.gen.V, P.gen.ushift + k * (P.d - 1),
+          dbgz::sobol_stage_block(sob, P.gen.V, P.gen.ushift + k * (P.d - 1), dbgz::sobol_mask(P.gen.n_bits),
                                   (uint64_t)(P.gen.sobol_first + pl.gen.gen_base + (j - r)), pl.sobol_l0(i0),
                                   Policy::kSobolDir, P.d - 2, nb, r);
       __syncthreads();

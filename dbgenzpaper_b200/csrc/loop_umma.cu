@@ -554,8 +554,8 @@ __global__ void __launch_bounds__(NT, 2) k_genz_umma(const __grid_constant__ Umm
         if constexpr (Policy::kSobolTable) {
           const int nv = (int)(nYI - lb < BK ? nYI - lb : BK);
           dbgz::sobol_stage_block(ms->sob[buf], pl.gen.V, pl.gen.ushift + pl.k * (dI - 1),
-                                  (uint64_t)(pl.gen.sobol_first + pl.gen.gen_base + (pl.j - r)), pl.sobol_l0(lb),
-                                  Policy::kSobolDir, dI - 2, nv, r);
+                                  dbgz::sobol_mask(pl.gen.n_bits), (uint64_t)(pl.gen.sobol_first + pl.gen.gen_base + (pl.j - r)),
+                                  pl.sobol_l0(lb), Policy::kSobolDir, dI - 2, nv, r);
         }
       };
       if (sob_staged) {
@@ -1112,16 +1112,20 @@ void dbgz_umma_batch_free(UmmaBatchPlan *B) {
   delete B;
 }
 
-bool dbgz_umma_waits(const dbgz_problem *p, int precision) {
-  // up to d = 512 the warp-level loop is faster (split BF16, 1.6e6 to 2e6
-  // samples, forward / with gradient: 1.47x / 1.30x at d = 100, 1.24x / 1.17x
-  // at d = 300, 1.15x / 1.11x at d = 400, 0.94x / 0.96x at d = 600)
-  constexpr int64_t kWarpLoopMaxD = 512;
-  return precision != DBGZ_PREC_FP32_SPLIT_BF16 || p->d > kWarpLoopMaxD;
+bool dbgz_umma_waits(const PassArgs &pa, int precision) {
+  // the warp-level loop's products run on mma.sync and grow with d; this one's
+  // do not show, but its steps have half the warps to hide their latency.
+  // Measured (split BF16, 5.2e5 samples, this loop / that one): forward 1.08
+  // to 1.13 at d = 300, 0.99 to 1.01 at 400, 0.89 to 0.93 at 450, 0.84 to 0.88
+  // at 500; with gradient, lattice 1.05 at 400, 0.98 at 450, Sobol 1.16 at 450,
+  // 1.03 to 1.05 at 560, 0.98 to 1.01 at 620
+  const bool plain = pa.kind == kLoopForward || pa.kind == kLoopLogWeight;
+  const int64_t warp_loop_max_d = plain ? 400 : pa.qmc_type == DBGZ_QMC_SOBOL ? 600 : 430;
+  return precision != DBGZ_PREC_FP32_SPLIT_BF16 || pa.d > warp_loop_max_d;
 }
 
 int dbgz_loop_umma(dbgz_problem *p, const PassArgs &pa, int precision, double *partials, int64_t n_tiles) {
-  if (!dbgz_umma_waits(p, precision)) return dbgz_loop_w32(p, pa, partials, n_tiles);
+  if (!dbgz_umma_waits(pa, precision)) return dbgz_loop_w32(p, pa, partials, n_tiles);
   if (precision == DBGZ_PREC_FP32_SPLIT_BF16)
     return launch_umma<DBGZ_PREC_FP32_SPLIT_BF16>(p, pa, partials, n_tiles);
   return launch_umma<DBGZ_PREC_FP32_TF32>(p, pa, partials, n_tiles);

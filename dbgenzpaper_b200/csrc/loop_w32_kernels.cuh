@@ -212,8 +212,8 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
     pol::cp_async_commit();
     if constexpr (Policy::kSobolTable)
       if (sob_staged)
-        dbgz::sobol_stage_block(st.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), base0, pl.sobol_l0(lb),
-                                Policy::kSobolDir, d - 2, nb, tid);
+        dbgz::sobol_stage_block(st.sob, P.gen.V, P.gen.ushift + k_shift * (d - 1), dbgz::sobol_mask(P.gen.n_bits),
+                                base0, pl.sobol_l0(lb), Policy::kSobolDir, d - 2, nb, tid);
   };
   // this lane's place in the workspace chunk of the next 8 y's (a ring for
   // banded factors)

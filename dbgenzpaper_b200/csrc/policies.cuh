@@ -394,6 +394,13 @@ struct Adjoint {
     }
   }
 
+  // the shifted Sobol integer of y-index t: the staged one, or formed here
+  __device__ __forceinline__ uint32_t sobol_x(int64_t t, uint32_t xs, bool staged) const {
+    if (staged) return xs;
+    return (dbgz::sobol_warp(gen.V + t * 32, (uint64_t)(gen.sobol_first + gen.gen_base + j)) ^
+            (uint32_t)gen.ushift[k * (d - 1) + t]) & dbgz::sobol_mask(gen.n_bits);
+  }
+
   // tent-transformed point w_t of y-index t (as StepFp*::quantile forms it);
   // Sobol: from the staged integer xs (already XORed with the shift) when
   // `staged`, else generated here
@@ -411,11 +418,7 @@ struct Adjoint {
       u = (double)sg.shv[li] + x;
       u = u > 1.0 ? u - 1.0 : u;
     } else {
-      const int L = gen.n_bits;  // <= 32
-      const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
-      const uint32_t xi = staged ? xs : dbgz::sobol_warp(gen.V + t * 32, (uint64_t)(gen.sobol_first + gen.gen_base + j));
-      const uint32_t sh = staged ? 0u : (uint32_t)gen.ushift[k * (d - 1) + t];
-      u = (double)((xi ^ sh) & mask) * __hiloint2double((1023 - L) << 20, 0);  // 2^-L
+      u = (double)sobol_x(t, xs, staged) * __hiloint2double((1023 - gen.n_bits) << 20, 0);  // 2^-n_bits
     }
     return fabs(fma(u, 2.0, -1.0));
   }
@@ -432,12 +435,8 @@ struct Adjoint {
       uf = uf > 1.0f ? uf - 1.0f : uf;
       return fabsf(fmaf(uf, 2.0f, -1.0f));
     }
-    const int L = gen.n_bits;
-    const uint32_t mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
-    const uint32_t xi = staged ? xs : dbgz::sobol_warp(gen.V + t * 32, (uint64_t)(gen.sobol_first + gen.gen_base + j));
-    const uint32_t sh = staged ? 0u : (uint32_t)gen.ushift[k * (d - 1) + t];
     float w, w1;
-    dbgz::sobol_tent_f32((xi ^ sh) & mask, L, w, w1);
+    dbgz::sobol_tent_f32(sobol_x(t, xs, staged), gen.n_bits, w, w1);
     return w;
   }
 
