@@ -9,13 +9,14 @@
 //      Cholesky (cholk::genz_block_dev / schur_tile_dev, the same code and
 //      bits as chol.cu), truncation, the per-target constants, the FP32
 //      copy of U and the first dimension's CDF;
-//   2. simt::k_genz_simt_batch: persistent CTAs take work items (a run of
-//      tiles of one problem, about the same number of tile-dimensions per
-//      item, largest problems first) from a global counter and run the SIMT
-//      loop of loop_simt_kernels.cuh on them.  The SIMT loop and not the
-//      tensor-core loop: at d <= 512 the contraction is a small share of the
-//      per-sample work (d/2 FMAs per dimension against the step's special
-//      functions), and one tcgen05 tile pipeline per problem would idle;
+//   2. the integration, by precision: FP64 f64::k_genz_f64_batch, FP32 SIMT
+//      simt::k_genz_simt_batch, split BF16 w32::k_genz_w32_batch for d <= 257
+//      (16 warps an SM hide the step's latency; 24.3 against 37.2 ms of the
+//      tcgen05 loop at 256 problems of d = 16..256, 6.6e4 samples each), TF32
+//      the tcgen05 loop for d <= 257, both with the SIMT kernel for larger d.
+//      Persistent CTAs take work items (a run of tiles of one problem, about
+//      the same number of tile-dimensions per item, largest problems first)
+//      from a global counter;
 //   3. k_finalize_batch: per (problem, shift) sums of the tile sums in tile
 //      order (the one-problem finalize, so results agree bit for bit).
 // Limits: 2 <= d <= min(512, chol_block_size2) (one Cholesky panel), one
@@ -473,7 +474,7 @@ int plan_setup(dbgz_batch_plan *P, const dbgz_opts &o, const uint32_t *dirnums, 
     if (P->precision == DBGZ_PREC_FP32_SPLIT_BF16)
       DBGZ_TRY(dbgz_w32_batch_setup(ctx, A, &P->wb));
     else
-      DBGZ_TRY(dbgz_umma_batch_setup(ctx, P->precision, A, &P->tb));
+      DBGZ_TRY(dbgz_umma_batch_setup(ctx, A, &P->tb));
   }
   return DBGZ_OK;
 }

@@ -225,15 +225,15 @@ struct UmmaBatchArgs {
   const uint64_t *dush = nullptr;
   double *dpart = nullptr;
 };
-// Tensor-core part of a batch plan: the U^T panels, per-problem descriptors
+// Tensor-core part of a TF32 batch plan: the U^T panels, per-problem descriptors
 // (tensor maps of the plan's fixed buffers) and the item list, set up once;
 // enqueue issues the panel conversion, the status reset and the loop on
 // ctx->stream (no allocation, no host synchronisation: capturable).
 struct UmmaBatchPlan {
   dbgz_ctx *ctx = nullptr;
-  int mode = 0, qmc_type = 0;
+  int qmc_type = 0;
   DevBuf buf;
-  char *pan0 = nullptr, *pan1 = nullptr, *d_desc = nullptr;
+  char *pan = nullptr, *d_desc = nullptr;
   int64_t nsel = 0, n_items = 0, grid = 0;
   int smem = 0;
   int64_t *d_dims = nullptr, *d_off2 = nullptr, *d_ld = nullptr, *d_pan = nullptr;
@@ -254,7 +254,7 @@ struct W32BatchPlan {
 int dbgz_w32_batch_setup(dbgz_ctx *ctx, const UmmaBatchArgs &A, W32BatchPlan **out);
 int dbgz_w32_batch_enqueue(W32BatchPlan *B);
 void dbgz_w32_batch_free(W32BatchPlan *B);
-int dbgz_umma_batch_setup(dbgz_ctx *ctx, int precision, const UmmaBatchArgs &A, UmmaBatchPlan **out);
+int dbgz_umma_batch_setup(dbgz_ctx *ctx, const UmmaBatchArgs &A, UmmaBatchPlan **out);
 int dbgz_umma_batch_enqueue(UmmaBatchPlan *B);
 void dbgz_umma_batch_free(UmmaBatchPlan *B);
 int dbgz_loop_sparse(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,

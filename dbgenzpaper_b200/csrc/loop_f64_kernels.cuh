@@ -1,5 +1,5 @@
 // loop_f64_kernels.cuh -- device code of the FP64 integration loop (launched
-// by loop_f64.cu, batch.cu and noalloc.cu).
+// by loop_simt.cu, batch.cu and noalloc.cu).
 //
 // The FP64 units bound this loop: one warp-wide FMA takes 2 cycles of a
 // scheduler, as scalar DFMAs or inside mma.m8n8k4.f64 (16 cycles for 8 of

@@ -1,10 +1,10 @@
 // loop_simt.cu -- the dense Genz integration loop on CUDA cores.
 //
 // Replaces qmc_loop!(::QMCData) (reference src/qmc.jl:315-444) and
-// qmc_loop!(::QMCData_Distributions) (:485-608).  Two instantiations:
-//   T = double, StepFp64: the FP64 path (the reference's Float64 numerics);
-//   T = float,  StepFp32: FP32 numerics with the contraction on FP32 cores
-//                         (an ablation of the tensor-core path).
+// qmc_loop!(::QMCData_Distributions) (:485-608).  FP64 (StepFp64, the
+// reference's Float64 numerics) launches the kernel of loop_f64_kernels.cuh,
+// for dense and banded factors; FP32 (StepFp32, the contraction on FP32 cores:
+// an ablation of the tensor-core path) the kernel described here.
 //
 // Work decomposition (one CTA = one tile of 128 samples = 128 consecutive
 // points of one shift; persistent CTAs loop over tiles):

@@ -7,6 +7,10 @@
 //   s = sum_{p in column i+1} y[rowval[p]] * nzval[p] in ascending row order,
 //   then the erf-form CDF and weight of the dense loop.
 //
+// Factors whose entries fill a good part of their band run in the group loops
+// instead (dbgz_band_loop below: loop_f64_kernels.cuh in FP64,
+// loop_w32_kernels.cuh in FP32); this one walks the entries and takes the rest.
+//
 // Work decomposition: one thread per sample, 128 samples per CTA, several
 // CTAs per SM (no tensor cores: the dot has at most `bandwidth` terms).  The
 // y history a sample needs is the last W = bandwidth + 1 values; it lives in

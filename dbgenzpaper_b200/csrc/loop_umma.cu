@@ -917,39 +917,32 @@ int launch_umma(dbgz_problem *p, const PassArgs &pa, double *partials, int64_t n
   return DBGZ_OK;
 }
 
+// Batches: TF32 only (a split-BF16 batch runs in the warp-level loop).
+constexpr int kBatchMode = DBGZ_PREC_FP32_TF32;
+
 // U^T panels of many problems: problems blockIdx.y + i gridDim.y, factor at
-// M + off2[k] (d x d), panel at byte offset pan[k] of out0/out1 with leading
+// M + off2[k] (d x d), panel at byte offset pan[k] of out with leading
 // dimension ldU[k] (rows t = 0..d-1).
-template <int MODE>
 __global__ void k_make_ut_batch(const double *M, int64_t n, const int64_t *dims, const int64_t *off2,
-                                const int64_t *ldU, const int64_t *pan, char *out0, char *out1) {
+                                const int64_t *ldU, const int64_t *pan, char *out) {
   for (int64_t k = blockIdx.y; k < n; k += gridDim.y) {
   const int64_t d = dims[k], ld = ldU[k];
   const double *U = M + off2[k];
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < d * ld; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t = e / ld, l = e - t * ld;
     const double u = (l < t) ? U[t * d + l] : 0.0;
-    if (MODE == DBGZ_PREC_FP32_SPLIT_BF16) {
-      const __nv_bfloat16 h = __double2bfloat16(u);
-      const __nv_bfloat16 lo = __double2bfloat16(u - (double)__bfloat162float(h));
-      reinterpret_cast<__nv_bfloat16 *>(out0 + pan[k])[e] = h;
-      reinterpret_cast<__nv_bfloat16 *>(out1 + pan[k])[e] = lo;
-    } else {
-      reinterpret_cast<uint32_t *>(out0 + pan[k])[e] = to_tf32((float)u);
-    }
+    reinterpret_cast<uint32_t *>(out + pan[k])[e] = to_tf32((float)u);
   }
   }
 }
 
-template <int MODE, int GEN>
-auto batch_kernel() {
-  return k_genz_umma<MODE, pol::Forward<float, GEN, false>, true>;
+auto batch_kernel(int qmc_type) {
+  return qmc_type == DBGZ_QMC_SOBOL ? k_genz_umma<kBatchMode, pol::Forward<float, DBGZ_QMC_SOBOL, false>, true>
+                                    : k_genz_umma<kBatchMode, pol::Forward<float, DBGZ_QMC_RICHTMYER, false>, true>;
 }
 
-template <int MODE>
 int setup_umma_batch(dbgz_ctx *ctx, const UmmaBatchArgs &A, UmmaBatchPlan *B) {
-  using F = Fmt<MODE>;
-  using SM = Smem<MODE>;
+  using F = Fmt<kBatchMode>;
   const int Pw = 256;
   const int64_t nsel = (int64_t)A.probs.size();
   // panels and per-problem tables
@@ -971,15 +964,14 @@ int setup_umma_batch(dbgz_ctx *ctx, const UmmaBatchArgs &A, UmmaBatchPlan *B) {
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t szTab = al(8 * (size_t)nsel);
   const size_t szDesc = al(sizeof(UmmaProb) * (size_t)nsel), szItems = al(4 * (size_t)n_items);
-  DBGZ_TRY(dbgz_ensure(ctx, B->buf, al(pan_bytes) * F::NPART + 4 * szTab + szDesc + 2 * szItems + 1024));
+  DBGZ_TRY(dbgz_ensure(ctx, B->buf, al(pan_bytes) + 4 * szTab + szDesc + 2 * szItems + 1024));
   char *base = (char *)B->buf.p;
   auto take = [&](size_t b) {
     char *r = base;
     base += al(b);
     return r;
   };
-  B->pan0 = take(pan_bytes);
-  B->pan1 = F::NPART > 1 ? take(pan_bytes) : nullptr;
+  B->pan = take(pan_bytes);
   B->d_dims = (int64_t *)take(szTab);
   B->d_off2 = (int64_t *)take(szTab);
   B->d_ld = (int64_t *)take(szTab);
@@ -996,9 +988,7 @@ int setup_umma_batch(dbgz_ctx *ctx, const UmmaBatchArgs &A, UmmaBatchPlan *B) {
     const int64_t k = A.probs[i];
     UmmaProb &D = hd[i];
     std::memset(&D, 0, sizeof(D));
-    DBGZ_TRY(encode_2d<MODE>(ctx, &D.tm_u[0], B->pan0 + pan[i], (uint64_t)ld[i], (uint64_t)dims[i], 64));
-    if (F::NPART > 1)
-      DBGZ_TRY(encode_2d<MODE>(ctx, &D.tm_u[1], B->pan1 + pan[i], (uint64_t)ld[i], (uint64_t)dims[i], 64));
+    DBGZ_TRY(encode_2d<kBatchMode>(ctx, &D.tm_u[0], B->pan + pan[i], (uint64_t)ld[i], (uint64_t)dims[i], 64));
     D.d = dims[i];
     D.nY = dims[i] - 1;
     D.m = A.m;
@@ -1038,9 +1028,8 @@ int setup_umma_batch(dbgz_ctx *ctx, const UmmaBatchArgs &A, UmmaBatchPlan *B) {
   DBGZ_CUDA_TRY(ctx, cudaMemcpyAsync(B->d_itile, itl.data(), 4 * n_items, cudaMemcpyHostToDevice, st));
   DBGZ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   // kernel configuration (attributes set here, outside any stream capture)
-  const int smem = umma_smem_bytes<MODE>(Pw, A.qmc_type == DBGZ_QMC_SOBOL);
-  auto kern = A.qmc_type == DBGZ_QMC_SOBOL ? batch_kernel<MODE, DBGZ_QMC_SOBOL>()
-                                           : batch_kernel<MODE, DBGZ_QMC_RICHTMYER>();
+  const int smem = umma_smem_bytes<kBatchMode>(Pw, A.qmc_type == DBGZ_QMC_SOBOL);
+  auto kern = batch_kernel(A.qmc_type);
   DBGZ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   DBGZ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   cudaFuncAttributes fa;
@@ -1056,12 +1045,11 @@ int setup_umma_batch(dbgz_ctx *ctx, const UmmaBatchArgs &A, UmmaBatchPlan *B) {
   return DBGZ_OK;
 }
 
-template <int MODE>
 int enqueue_umma_batch(UmmaBatchPlan *B) {
   dbgz_ctx *ctx = B->ctx;
   cudaStream_t st = ctx->stream;
-  k_make_ut_batch<MODE><<<dim3(8, (unsigned)std::min<int64_t>(B->nsel, 65535)), 256, 0, st>>>(
-      B->dM, B->nsel, B->d_dims, B->d_off2, B->d_ld, B->d_pan, B->pan0, B->pan1);
+  k_make_ut_batch<<<dim3(8, (unsigned)std::min<int64_t>(B->nsel, 65535)), 256, 0, st>>>(
+      B->dM, B->nsel, B->d_dims, B->d_off2, B->d_ld, B->d_pan, B->pan);
   dbgz_count_launch(ctx);
   UmmaParams P{};
   P.P = 256;
@@ -1073,9 +1061,7 @@ int enqueue_umma_batch(UmmaBatchPlan *B) {
   P.item_prob = B->d_iprob;
   P.item_tile = B->d_itile;
   DBGZ_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), st));
-  auto kern = B->qmc_type == DBGZ_QMC_SOBOL ? batch_kernel<MODE, DBGZ_QMC_SOBOL>()
-                                            : batch_kernel<MODE, DBGZ_QMC_RICHTMYER>();
-  kern<<<(unsigned)B->grid, NT, B->smem, st>>>(P);
+  batch_kernel(B->qmc_type)<<<(unsigned)B->grid, NT, B->smem, st>>>(P);
   dbgz_count_launch(ctx);
   DBGZ_CUDA_TRY(ctx, cudaGetLastError());
   return DBGZ_OK;
@@ -1083,15 +1069,13 @@ int enqueue_umma_batch(UmmaBatchPlan *B) {
 
 }  // namespace
 
-int dbgz_umma_batch_setup(dbgz_ctx *ctx, int precision, const UmmaBatchArgs &A, UmmaBatchPlan **out) {
+int dbgz_umma_batch_setup(dbgz_ctx *ctx, const UmmaBatchArgs &A, UmmaBatchPlan **out) {
   *out = nullptr;
   if (A.probs.empty()) return DBGZ_OK;
   UmmaBatchPlan *B = new UmmaBatchPlan;
   B->ctx = ctx;
-  B->mode = precision;
   B->qmc_type = A.qmc_type;
-  const int rc = precision == DBGZ_PREC_FP32_SPLIT_BF16 ? setup_umma_batch<DBGZ_PREC_FP32_SPLIT_BF16>(ctx, A, B)
-                                                        : setup_umma_batch<DBGZ_PREC_FP32_TF32>(ctx, A, B);
+  const int rc = setup_umma_batch(ctx, A, B);
   if (rc != DBGZ_OK) {
     dbgz_umma_batch_free(B);
     return rc;
@@ -1100,11 +1084,7 @@ int dbgz_umma_batch_setup(dbgz_ctx *ctx, int precision, const UmmaBatchArgs &A, 
   return DBGZ_OK;
 }
 
-int dbgz_umma_batch_enqueue(UmmaBatchPlan *B) {
-  if (!B) return DBGZ_OK;
-  return B->mode == DBGZ_PREC_FP32_SPLIT_BF16 ? enqueue_umma_batch<DBGZ_PREC_FP32_SPLIT_BF16>(B)
-                                             : enqueue_umma_batch<DBGZ_PREC_FP32_TF32>(B);
-}
+int dbgz_umma_batch_enqueue(UmmaBatchPlan *B) { return B ? enqueue_umma_batch(B) : DBGZ_OK; }
 
 void dbgz_umma_batch_free(UmmaBatchPlan *B) {
   if (!B) return;

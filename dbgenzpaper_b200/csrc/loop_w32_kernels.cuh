@@ -6,7 +6,7 @@
 // in one dependent chain of some 330 cycles, so a scheduler needs four or more
 // warps of samples.  The tcgen05 loop (loop_umma.cu) holds two: its partial
 // sums take 256 TMEM columns and 32 registers a sample.  Here a warp keeps the
-// sums of 64 targets in 8 KB of shared memory and 8 of them in registers, so
+// sums of 32 targets in 4 KB of shared memory and 8 of them in registers, so
 // 16 warps fit on an SM, and mma.m16n8k16 (8 cycles of a scheduler, in the
 // shadow of the other warps' steps) feeds them without a round trip to
 // another warp.  The larger the dimension, the more the contraction weighs:
@@ -16,7 +16,7 @@
 // One CTA = one tile of 128 samples = four warps of 32.  y-indices run in
 // groups of G, each in chunks of 8:
 //   * group start: S[32 x G] = Y[:, k0 .. g0) U[k0 .. g0, targets], Y from the
-//     CTA's workspace and U^T panels through a three-stage cp.async ring that
+//     CTA's workspace and U^T panels through a two-stage cp.async ring that
 //     lies in the S buffer (idle then).  Banded factors: k0 is the first
 //     y-index within the band of the group, else 0;
 //   * chunk: its sums + the group's own earlier chunks by mma (a chunk's y's
@@ -25,8 +25,8 @@
 // The tensor unit truncates as it accumulates, so the products of high parts
 // have accumulators of their own: their sum is truncated once per 16 y-indices,
 // not once per product (relative error of P, batch of d 16..256: 4.7e-6 with
-// one accumulator).  Operands are NPART BF16 parts: 2 (hi hi + hi lo + lo hi: the split-BF16
-// mode) or 3 (six products, about 2^-24: FP32 operands' accuracy, for the
+// one accumulator).  Operands are NPART BF16 parts: 2 (hi hi + hi lo + lo hi:
+// the split-BF16 mode) or 3 (six products, about 2^-24: FP32 operands' accuracy, for the
 // banded loop).  Warps meet once per chunk of the ring and per 32 dimensions
 // (their staged constants, copied one block ahead).
 #pragma once
@@ -43,13 +43,8 @@ constexpr int TS = 128, NT = 128;
 constexpr int SB = 32;  // dimensions per staged block
 constexpr int CH = 8;   // y-indices per chunk
 constexpr int KC = 16;  // y-indices per ring stage
-// Stages of the ring and points formed ahead of the steps, by group size
-// (measured beside the launch rules)
-template <int G>
-struct Cfg {
-  static constexpr int NST = G == 32 ? 2 : 3;
-  static constexpr int kAhead = G == 32 ? 1 : 8;
-};
+constexpr int NST = 2;     // stages of the ring
+constexpr int kAhead = 1;  // points formed ahead of the steps
 
 // One problem's operands and constants.
 struct Prob {
@@ -89,7 +84,6 @@ struct Stage {
 };
 template <int NPART, int G>
 struct Smem {
-  static constexpr int NST = Cfg<G>::NST;
   static constexpr int SLOT = NPART * 512 > 1024 ? NPART * 512 : 1024;  // a chunk's sums, then its y's
   struct Ring {
     unsigned char y[NST][4][KC / CH][NPART][512];
@@ -181,7 +175,6 @@ template <int NPART, int G, typename Policy>
 __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io, Smem<NPART, G> &sm,
                                      unsigned char *Yw, int64_t tile_id) {
   using SM = Smem<NPART, G>;
-  constexpr int NST = Cfg<G>::NST, kAhead = Cfg<G>::kAhead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int fr = lane >> 2, fk = lane & 3;
   const int64_t d = P.d, nY = d - 1;
