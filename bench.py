@@ -42,14 +42,14 @@ METRIC = "d=1000 MVN P time at |err|<=1e-5 vs FP64: mixed-prec vs FP64 GPU; grad
 UNIT = "ms"
 MIXED = "fp32_split_bf16"   # mixed-precision mode of the headline number
 # DRAM bytes of one 2^21-sample launch of the split-BF16 loop at d=1000 (ncu capture of a
-# 131,072-sample launch: 0.239 GB read + 0.328 GB written, scaled by the sample count)
-TRAFFIC_PER_LAUNCH = 16 * (239.36e6 + 328.14e6)
+# 131,072-sample launch: 0.229 GB read + 0.326 GB written, scaled by the sample count)
+TRAFFIC_PER_LAUNCH = 16 * (229.39e6 + 325.92e6)
 # warp instructions of one split-BF16 loop launch at d = 1000 per sample (ncu
-# smsp__inst_executed.sum of a 131,072-sample launch: 6.788e8), and its
+# smsp__inst_executed.sum of a 131,072-sample launch: 5.976e8), and its
 # XU (special-function) pipe share; the issue roofline below scales it to the
 # timed launch
-INST_PER_SAMPLE = 6.788e8 / 131072
-XU_PIPE_PCT = 15.4
+INST_PER_SAMPLE = 5.976e8 / 131072
+XU_PIPE_PCT = 17.7
 ISSUE_PROFILE = "ncu --set full of the split-BF16 loop at d=1000, 8192 points x 16 shifts (profiles/)"
 
 
@@ -420,14 +420,15 @@ def run_c5(args, emit=True):
     (P64, e64, _), out["fp64_ms"] = timed(lambda: D.qmc_pnorm(Q, precision=L.PREC_FP64), max(1, args.steps // 2))
     g, out["fp32_grad_ms"] = timed(lambda: D.qmc_pnorm_grad(Q, precision=L.PREC_FP32_SIMT), max(1, args.steps // 2))
     lib.dbgz_get_profile(ctx.handle, C.byref(prof))
-    # stored forward state of the gradient call: dimension checkpoints every
-    # 256 dimensions (the band's last values and the recursion state) and one
-    # segment's recomputed rows, against y, s, dc of every sample-variable
+    # stored forward state of the gradient call at the default checkpoint
+    # setting (which the CSC loop heeds; a factor that fills its band stores
+    # the whole state, in sample chunks within the state budget), against
+    # y, s, dc of every sample-variable
     out["grad_state"] = {"checkpoint_every_dims": 256, "bytes": int(prof.grad_state_bytes),
                          "sample_chunks": int(prof.grad_chunks),
                          "full_state_bytes": int(w.m * w.n_reps * 3 * 4 * w.d)}
     out["grad_state"]["fraction_of_full"] = out["grad_state"]["bytes"] / out["grad_state"]["full_state_bytes"]
-    # the alternative: every sample's forward state stored, in sample chunks
+    # checkpoints off: every sample's forward state stored, in sample chunks
     # within the context's state budget (no recomputation)
     ctx.set_grad_checkpoints(0)
     g0, out["fp32_grad_full_state_ms"] = timed(lambda: D.qmc_pnorm_grad(Q, precision=L.PREC_FP32_SIMT),

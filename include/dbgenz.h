@@ -117,12 +117,15 @@ int dbgz_release_cached(dbgz_ctx *ctx, uint64_t *freed_bytes);
  * counts run the forward and adjoint passes in chunks of whole 128-sample
  * tiles (default 48 GiB).  No reference counterpart. */
 int dbgz_set_state_budget(dbgz_ctx *ctx, uint64_t bytes);
-/* Banded (QMCDataSparse) gradients keep, instead of every sample's forward
+/* Gradients of sparse (QMCDataSparse) factors with few entries for their
+ * bandwidth, which take the CSC loop, keep, instead of every sample's forward
  * state, a checkpoint every `segment` dimensions (the band's recent values
  * and the recursion state) and recompute each segment's state from its
  * checkpoint just before the adjoint sweeps it (default 256; 0 stores the
  * whole forward state as the dense path does).  The results are the same
- * bits either way.  No reference counterpart. */
+ * bits either way.  Factors that fill their band store the whole state within
+ * the state budget (faster there), whatever the setting.  No reference
+ * counterpart. */
 int dbgz_set_grad_checkpoints(dbgz_ctx *ctx, int64_t segment);
 const char *dbgz_last_error(const dbgz_ctx *ctx);
 
@@ -250,7 +253,7 @@ int dbgz_pnorm_grad(dbgz_problem *p, int precision, double *result, double *err,
  * column-major, symmetric) is the gradient for symmetric perturbations:
  * dP = sum_ij dP_dSigma[i,j] E[i,j] for symmetric E, so that for
  * Sigma = B B' + diag(psi), dP/dB = 2 dP_dSigma B.  FP64 throughout
- * (cuBLAS TRMM/TRSM/GEMM on the context's stream). */
+ * (this library's own kernels on the context's stream). */
 int dbgz_problem_sigma_adjoint(dbgz_problem *p, const double *dP_dU, const double *dP_da,
                                const double *dP_db, double *dP_dSigma);
 /* dbgz_pnorm_grad followed by dbgz_problem_sigma_adjoint with the factor
