@@ -1,7 +1,7 @@
 """The sample loops, their dispatch rules and the pivoted factorisation at the
 sizes where tiles, groups, chunks and rings end (needs a B200).
 
-Bars, as elsewhere: FP64 replicate means within 1e-12 relative of the checker;
+Bars, as elsewhere: FP64 replicate means within 1e-12 relative of the oracle;
 FP32 probabilities within 5e-6 + 2e-5 P of FP64 on the same points; FP32
 gradients within 2e-3 of FP64 in norm; FP64 gradients against a central
 difference of step 1e-6 along all upper bounds (rounding 1e-16 / 1e-6,
@@ -30,7 +30,7 @@ def _points(qmc, n, rng):
     return {"ushifts": rng.integers(0, 2**64, size=(n - 1, R), dtype=np.uint64)}
 
 
-def _checker(D, oracle, Q, qmc, pts, m, sparse):
+def _oracle(D, oracle, Q, qmc, pts, m, sparse):
     kw = dict(m=m, n_reps=R, max_pts=m, max_abs_err=0.0, sparse=sparse)
     if qmc == "Richtmyer":
         kw["shifts"] = pts["shifts"]
@@ -60,7 +60,7 @@ def test_dense_loops_at_group_edges(D, oracle, n, qmc):
     pts = _points(qmc, n, rng)
     Q = D.QMCData(S, a, b, _opts(D, 200), qmc_type=qmc, **pts)
     r64 = D.qmc_pnorm(Q, precision=L.PREC_FP64, return_reps=True)
-    rc = _checker(D, oracle, Q, qmc, pts, 200, False)
+    rc = _oracle(D, oracle, Q, qmc, pts, 200, False)
     np.testing.assert_allclose(r64[3], rc[3], rtol=1e-12)
     for prec in (L.PREC_FP32_SPLIT_BF16, L.PREC_FP32_SIMT):
         Q.close()
@@ -128,7 +128,7 @@ def test_band_loops_at_group_and_ring_edges(D, oracle, n, band, qmc):
     pts = _points(qmc, n, rng)
     Q = _band_data(D, n, band, qmc, pts, a, b)
     P, _, _, reps = D.qmc_pnorm(Q, precision=L.PREC_FP64, return_reps=True)
-    rc = _checker(D, oracle, Q, qmc, pts, 200, True)
+    rc = _oracle(D, oracle, Q, qmc, pts, 200, True)
     np.testing.assert_allclose(reps, rc[3], rtol=1e-12, atol=1e-300)
     Q.close()
     Q = _band_data(D, n, band, qmc, pts, a, b)
@@ -166,7 +166,7 @@ def test_few_entries_in_a_wide_band(D, oracle, n, dist, qmc):
 
     Q = data(b)
     P, _, _, reps = D.qmc_pnorm(Q, precision=L.PREC_FP64, return_reps=True)
-    rc = _checker(D, oracle, Q, qmc, pts, 200, True)
+    rc = _oracle(D, oracle, Q, qmc, pts, 200, True)
     np.testing.assert_allclose(reps, rc[3], rtol=1e-12, atol=1e-300)
     Q.close()
     Q = data(b)
