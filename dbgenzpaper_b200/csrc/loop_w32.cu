@@ -27,10 +27,7 @@ __global__ void k_w32_ops_batch(const OpsProb *probs, int64_t n) {
       P.u0[e] = __bfloat16_as_ushort(h);
       P.u1[e] = __bfloat16_as_ushort(__double2bfloat16(u - (double)__bfloat162float(h)));
     }
-    for (int64_t e = e0; e < P.tri_n; e += step) {
-      const int64_t c = e >> 6, kk = (e >> 3) & 7, j = e & 7, l = 8 * c + kk, t = 8 * c + j + 1;
-      P.tri[e] = kk <= j && t < P.d ? (float)P.U[t * P.d + l] : 0.f;
-    }
+    for (int64_t e = e0; e < P.tri_n; e += step) P.tri[e] = w32::tri_value(P.U, P.d, e);
   }
 }
 
@@ -61,7 +58,7 @@ int dbgz_w32_batch_setup(dbgz_ctx *ctx, const UmmaBatchArgs &A, W32BatchPlan **o
     return rc;
   };
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-  // operands of problem i at base + off[i]: two panels, then the triangles
+  // operands of problem i at base + off[i]: two panels, then the groups' FP32 coefficients
   std::vector<size_t> off(nsel);
   size_t bytes = 0;
   int64_t slot = 0;

@@ -9,7 +9,7 @@
 namespace {
 
 // U^T panels in NPART BF16 parts (rows t = 1 .. d - 1 of ld entries from the
-// first y-index that reaches the row's group) and the chunk triangles.
+// first y-index that reaches the row's group) and the groups' FP32 coefficients.
 template <int NPART, int G>
 __global__ void k_w32_panels(const double *U, int64_t d, int64_t ld, int64_t band, uint16_t *u0, uint16_t *u1,
                              uint16_t *u2) {
@@ -31,9 +31,7 @@ __global__ void k_w32_panels(const double *U, int64_t d, int64_t ld, int64_t ban
 __global__ void k_w32_tri(const double *U, int64_t d, int64_t n, float *tri) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const int64_t c = e >> 6, k = (e >> 3) & 7, j = e & 7;
-  const int64_t l = 8 * c + k, t = 8 * c + j + 1;
-  tri[e] = k <= j && t < d ? (float)U[t * d + l] : 0.f;
+  tri[e] = w32::tri_value(U, d, e);
 }
 
 template <int NPART, int G>
@@ -43,7 +41,7 @@ struct W32Layout {
     const int64_t nY = d - 1;
     ld = band > 0 ? (band + 15) / 16 * 16 + 16 + G : (nY + 63) / 64 * 64;
     rows_bytes = (d * ld * 2 + 255) / 256 * 256;
-    tri_n = (nY + w32::SB - 1) / w32::SB * w32::SB * w32::CH;
+    tri_n = (nY + w32::SB - 1) / w32::SB * w32::kTri;
     ring_chunks = ld / w32::CH;
     slot = ring_chunks * 4 * NPART * 512;
   }

@@ -19,16 +19,22 @@
 //     CTA's workspace and U^T panels through a two-stage cp.async ring that
 //     lies in the S buffer (idle then).  Banded factors: k0 is the first
 //     y-index within the band of the group, else 0;
-//   * chunk: its sums + the group's own earlier chunks by mma (a chunk's y's
-//     take the place of the sums they consumed), 8 sequential steps with the
-//     chunk's triangle as FMAs in registers, the y's back as BF16 parts.
+//   * chunk: its sums + the group's own earlier chunks and the chunk's triangle
+//     as FP32 FMAs on FP32 y's and coefficients, as the tcgen05 loop does within
+//     its blocks of 32 (a chunk's y's take the place of the sums they consumed);
+//     the y's that a later group reads go to the workspace as BF16 parts.
+//     (With the earlier chunks as BF16 parts too, rms error of the shifts' means
+//     against FP64, split BF16: 2.1e-7 at d = 20, 1.9e-7 at 33, geometric mean
+//     over d = 8..380 4.3e-7; as FP32 0.8e-7, 0.7e-7, 3.4e-7.  Time with the parts and now: batch of
+//     256 problems 20.50 / 20.45 ms, banded d = 4000 pass 10.46 / 10.64, gradient
+//     7.81 / 7.78.)
 // The tensor unit truncates as it accumulates, so the products of high parts
 // have accumulators of their own: their sum is truncated once per 16 y-indices,
 // not once per product (relative error of P, batch of d 16..256: 4.7e-6 with
 // one accumulator).  Operands are NPART BF16 parts: 2 (hi hi + hi lo + lo hi:
 // the split-BF16 mode) or 3 (six products, about 2^-24: FP32 operands' accuracy, for the
-// banded loop).  Warps meet once per chunk of the ring and per 32 dimensions
-// (their staged constants, copied one block ahead).
+// banded loop), from one group to the later ones.  Warps meet once per chunk of
+// the ring and per 32 dimensions (their staged constants, copied one block ahead).
 #pragma once
 #include <type_traits>
 
@@ -42,6 +48,8 @@ namespace w32 {
 constexpr int TS = 128, NT = 128;
 constexpr int SB = 32;  // dimensions per staged block
 constexpr int CH = 8;   // y-indices per chunk
+constexpr int kTri = 10 * CH * CH;  // FP32 coefficients of a group: its 10 blocks of 8 x 8
+__host__ __device__ constexpr int tri_at(int q, int c) { return (q * (q + 1) / 2 + c) * CH * CH; }
 constexpr int KC = 16;  // y-indices per ring stage
 constexpr int NST = 2;     // stages of the ring
 constexpr int kAhead = 1;  // points formed ahead of the steps
@@ -51,7 +59,9 @@ struct Prob {
   int64_t d, m, tiles_per_shift;
   dbgz::GenParams gen;
   const TargetParams32 *tgt;
-  // tri[(l / 8) * 64 + k * 8 + j] = U[8 c + k, target of step 8 c + j], k <= j
+  // per group of 32 y-indices kTri floats: block (q, c), c <= q < 4, at
+  // tri_at(q, c): [k * 8 + j] = U[y-index 8 c + k, target of step 8 q + j] (0
+  // below the diagonal)
   const float *tri;
   // U^T panels: part p of U[l, t] at u[p][t * ld + l - lofs(group of t)]
   const uint16_t *u[3];
@@ -77,14 +87,24 @@ __host__ __device__ inline int64_t first_k(int64_t g0, int64_t band) {
   return k > 0 ? k / KC * KC : 0;
 }
 
+// element e of Prob::tri for the factor U (d x d, column-major)
+__device__ __forceinline__ float tri_value(const double *U, int64_t d, int64_t e) {
+  const int64_t g = e / kTri;
+  const int r = (int)(e - g * kTri), blk = r >> 6, k = (r >> 3) & 7, j = r & 7;
+  const int q = blk >= 6 ? 3 : blk >= 3 ? 2 : blk >= 1 ? 1 : 0, c = blk - q * (q + 1) / 2;
+  const int64_t l = SB * g + 8 * c + k, t = SB * g + 8 * q + j + 1;
+  return l < t && t < d ? (float)U[t * d + l] : 0.f;
+}
+
 struct Stage {
   pol::Staged<float> sg;
-  float tri[SB / CH][CH][CH];
+  float tri[kTri];
   uint32_t sob[SB][dbgz::kSobolRow];
 };
 template <int NPART, int G>
 struct Smem {
-  static constexpr int SLOT = NPART * 512 > 1024 ? NPART * 512 : 1024;  // a chunk's sums, then its y's
+  static_assert(G == SB, "a staged block holds the coefficients of one group");
+  static constexpr int SLOT = 1024;  // a chunk's sums, then its y's: 8 floats a sample
   struct Ring {
     unsigned char y[NST][4][KC / CH][NPART][512];
     unsigned char u[NST][NPART][2][G][16];  // [part][k half][target][8 BF16]
@@ -113,11 +133,6 @@ __device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uin
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(b0));
-}
 // The products of the parts: every (i, j) with i + j < NPART.
 template <int NPART, typename F>
 __device__ __forceinline__ void products(F &&f) {
@@ -134,17 +149,27 @@ __device__ __forceinline__ void products(F &&f) {
 __device__ __forceinline__ uint32_t soff(int t, int r) {
   return (uint32_t)(r * 32 + ((((t >> 2) ^ (r >> 2)) & 1) << 4) + (t & 2) * 4);
 }
-__device__ __forceinline__ void lds2(float &x, float &y, uint32_t a) {
-  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(x), "=f"(y) : "r"(a) : "memory");
-}
 __device__ __forceinline__ void sts2(uint32_t a, float x, float y) {
   asm volatile("st.shared.v2.f32 [%0], {%1,%2};" ::"r"(a), "f"(x), "f"(y) : "memory");
 }
 __device__ __forceinline__ void lds4(float *x, uint32_t a) {
   asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(a) : "memory");
 }
-__device__ __forceinline__ void sts4(uint32_t a, const uint32_t (&w)[4]) {
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+__device__ __forceinline__ void sts4(uint32_t a, const float *x) {
+  asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]) : "memory");
+}
+
+// two FP32 values in a 64-bit register; c += a b for both, each rounded as fmaf
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &x, float &y) {
+  asm("mov.b64 {%0,%1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ void fma2(uint64_t &c, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
 // x as BF16 parts of 8 values: word e of part p holds values 2e, 2e + 1
@@ -201,7 +226,7 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
     Stage &st = sm.stg[b];
     const int nb = (int)(nY - lb < SB ? nY - lb : SB);
     pl.stage_async(st.sg, P.tgt, tid, lb, nb);
-    if (tid < SB * CH / 4) cp16(saddr(&st.tri[0][0][0] + 4 * tid), P.tri + lb * CH + 4 * tid);
+    for (int e = tid; e < kTri / 4; e += NT) cp16(saddr(st.tri + 4 * e), P.tri + lb / SB * kTri + 4 * e);
     pol::cp_async_commit();
     if constexpr (Policy::kSobolTable)
       if (sob_staged)
@@ -332,68 +357,39 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
         const int nv = nb - i0;        // valid steps (8 or more: all)
         const uint32_t Sq = Sa + q * SM::SLOT;
         float s[8];
-        if (q > 0) {
-          // the group's earlier chunks, two at a time
-          float c[2][4], cs[2][4];
-#pragma unroll
-          for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              cs[mi][2 * h] = cs[mi][2 * h + 1] = 0.f;
-              c[mi][2 * h] = c[mi][2 * h + 1] = 0.f;
-              if (g0 > 0) lds2(c[mi][2 * h], c[mi][2 * h + 1], Sq + sf + mi * 512 + h * 256);
-            }
-          const int64_t t = g0 + CH * q + 1 + fr;
-          const int64_t uo = (t < d ? t : d - 1) * P.ld + (g0 - lofs) + 2 * fk;
-          const uint32_t *ub[NPART];
-#pragma unroll
-          for (int p = 0; p < NPART; ++p) ub[p] = reinterpret_cast<const uint32_t *>(P.u[p] + uo);
-          const uint32_t la = Sa + lm_ch * SM::SLOT + lm_row * 16;
-#pragma unroll
-          for (int cc = 0; cc < G / CH; cc += 2)
-            if (cc + 2 <= q) {
-              uint32_t b[NPART][2];
-#pragma unroll
-              for (int p = 0; p < NPART; ++p) {
-                b[p][0] = __ldg(ub[p] + cc * (CH / 2));
-                b[p][1] = __ldg(ub[p] + cc * (CH / 2) + CH / 2);
-              }
-#pragma unroll
-              for (int mi = 0; mi < 2; ++mi) {
-                uint32_t a[NPART][4];
-#pragma unroll
-                for (int p = 0; p < NPART; ++p) ldsm4(a[p], la + cc * SM::SLOT + p * 512 + mi * 256);
-                products<NPART>(
-                    [&](int i, int jj) { mma16(i + jj > 0 ? cs[mi] : c[mi], a[i], b[jj][0], b[jj][1]); });
-              }
-            }
-          if (q & 1) {
-            uint32_t b[NPART], a[NPART][4];  // a: samples 0-7, 8-15, 16-23, 24-31 of one chunk
-#pragma unroll
-            for (int p = 0; p < NPART; ++p) b[p] = __ldg(ub[p] + (q - 1) * (CH / 2));
-#pragma unroll
-            for (int p = 0; p < NPART; ++p) ldsm4(a[p], Sq - SM::SLOT + p * 512 + lane * 16);
-            products<NPART>([&](int i, int jj) {
-#pragma unroll
-              for (int mi = 0; mi < 2; ++mi) mma8(i + jj > 0 ? cs[mi] : c[mi], a[i][2 * mi], a[i][2 * mi + 1], b[jj]);
-            });
-          }
-          __syncwarp();  // every lane has read its part of the chunk's sums
-#pragma unroll
-          for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-              sts2(Sq + sf + mi * 512 + h * 256, c[mi][2 * h] + cs[mi][2 * h], c[mi][2 * h + 1] + cs[mi][2 * h + 1]);
-          __syncwarp();
-        }
-        if (g0 > 0 || q > 0) {
+        // (a sample's sums and y's in S are its own lane's)
+        if (g0 > 0) {
           lds4(s, Sq + s_lo);
           lds4(s + 4, Sq + s_hi);
         } else {
 #pragma unroll
           for (int t = 0; t < 8; ++t) s[t] = 0.f;
         }
-        __syncwarp();  // the sums are read: the y's may take their place
+        // the group's earlier chunks (paired FMAs: half the issue slots, banded
+        // pass 10.70 -> 10.64 ms)
+        if (q > 0) {
+          uint64_t s2[4];
+#pragma unroll
+          for (int t = 0; t < 4; ++t) s2[t] = pack2(s[2 * t], s[2 * t + 1]);
+#pragma unroll 1
+          for (int c = 0; c < q; ++c) {
+            float ye[8];
+            lds4(ye, Sa + c * SM::SLOT + s_lo);
+            lds4(ye + 4, Sa + c * SM::SLOT + s_hi);
+            const ulonglong2 *ur = reinterpret_cast<const ulonglong2 *>(st.tri + tri_at(q, c));
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const uint64_t y2 = pack2(ye[k], ye[k]);
+              const ulonglong2 u0 = ur[2 * k], u1 = ur[2 * k + 1];
+              fma2(s2[0], y2, u0.x);
+              fma2(s2[1], y2, u0.y);
+              fma2(s2[2], y2, u1.x);
+              fma2(s2[3], y2, u1.y);
+            }
+          }
+#pragma unroll
+          for (int t = 0; t < 4; ++t) unpack2(s2[t], s[2 * t], s[2 * t + 1]);
+        }
         float ys[8];
         const int64_t l0 = lb + i0;
         pl.chunk_begin(l0, nv);
@@ -422,7 +418,7 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
                 y = pl.emit_k(st.sg, li, l, k, sob_x(k));
               else
                 y = pl.emit_k_at(st.sg, li, l, k, pt[k]);
-              const float4 *ur = reinterpret_cast<const float4 *>(&st.tri[i0 / CH][k][0]);
+              const float4 *ur = reinterpret_cast<const float4 *>(st.tri + tri_at(q, q) + k * CH);
               const float4 u0 = ur[0], u1 = ur[1];
               const float uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
 #pragma unroll
@@ -460,16 +456,19 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
         }
         pl.chunk_end(l0, nv);
         if constexpr (Policy::kDeferTail) pl.tail_repair(st.sg, s, i0, l0);
-        uint32_t w[NPART][4];
-        split8<NPART>(ys, w);
+        if (q + 1 < nt) {
+          sts4(Sq + s_lo, ys);
+          sts4(Sq + s_hi, ys + 4);
+        }
+        if (keep) {
+          uint32_t w[NPART][4];
+          split8<NPART>(ys, w);
 #pragma unroll
-        for (int p = 0; p < NPART; ++p) {
-          sts4(Sq + p * 512 + lane * 16, w[p]);
-          if (keep) *reinterpret_cast<uint4 *>(yout + p * 512) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+          for (int p = 0; p < NPART; ++p)
+            *reinterpret_cast<uint4 *>(yout + p * 512) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
         }
         yout += 4 * NPART * 512;
         if (P.band > 0 && yout == yend) yout -= P.ring_chunks * (4 * NPART * 512);
-        __syncwarp();
       }
       // the next block's constants have landed, and this block's are read
       pol::cp_async_wait_all();
