@@ -83,7 +83,9 @@ class Context:
     def set_grad_checkpoints(self, segment: int) -> None:
         """Banded gradients: a checkpoint every `segment` dimensions, each
         segment recomputed from its checkpoint before the adjoint sweeps it
-        (default 256; 0 stores the whole forward state).  Same results."""
+        (0 stores the whole forward state), the same bits for every setting.
+        Without a call, factors that fill their band store the whole state
+        within the state budget in a faster loop, others take segments of 256."""
         L.check(self._lib.dbgz_set_grad_checkpoints(self.handle, int(segment)), self.handle)
 
     def close(self):

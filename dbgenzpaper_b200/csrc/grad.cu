@@ -119,12 +119,15 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   // to the next segment.  The same kernels and arithmetic as storing
   // everything: the same bits, with the stored state of K = ceil((d-1)/seg)
   // checkpoints instead of d rows.
-  // Problems that run in the loops that treat the band as dense
+  // Checkpoints are the CSC loop's.  Where the caller has not asked for them,
+  // problems that run in the loops that treat the band as dense
   // (dbgz_band_loop) store the state of every variable and bound it by chunks of
-  // samples alone, whatever the checkpoint setting: no recomputation (the
-  // setting applies to the CSC loop).
+  // samples alone: no recomputation.  A caller's setting, 0 too, is kept for
+  // every factor, all in the CSC loop, so that every setting gives the same bits.
   if (sparse && !p->csc_colptr.p) DBGZ_TRY(dbgz_build_csc(p));
-  const int64_t seg = sparse && !dbgz_band_loop(p, true) ? ctx->grad_ckpt_seg : 0;
+  const bool ckpt_set = ctx->grad_ckpt_seg >= 0;
+  const bool csc = sparse && (ckpt_set || !dbgz_band_loop(p, true));
+  const int64_t seg = !csc ? 0 : ckpt_set ? ctx->grad_ckpt_seg : kDefaultCkptSeg;
   const int64_t nY = d - 1, K = seg > 0 ? (nY + seg - 1) / seg : 0;
   const bool ckpt = seg > 0 && K >= 1;
   int64_t Wf = 0, Wb = 0;  // ring sizes of the forward and adjoint banded loops
@@ -215,6 +218,7 @@ static int grad_impl(dbgz_problem *p, int precision, double *result, double *err
   pa.c1 = p->c1;
   pa.dc1 = p->dc1;
   pa.gen_base = p->gen_base;
+  pa.csc = csc;
   pa.grad = ga;
   const bool tensor = !sparse && (precision == DBGZ_PREC_FP32_TF32 || precision == DBGZ_PREC_FP32_SPLIT_BF16);
   auto run = [&](int kind, int64_t t0, int64_t t1) -> int {

@@ -45,6 +45,8 @@ struct BatchTuning {
   int32_t item_dims[kBatchMaxD + 1] = {};
 };
 
+constexpr int64_t kDefaultCkptSeg = 256;
+
 struct dbgz_ctx {
   int device = 0;
   int num_sms = 0;
@@ -66,8 +68,10 @@ struct dbgz_ctx {
   int64_t live_problems = 0;  // problems created on this context and not yet freed
   size_t state_budget = size_t(48) << 30;  // bytes of stored forward state a gradient call may hold
   // banded gradients: dimensions per checkpoint segment (0: store the whole
-  // forward state instead)
-  int64_t grad_ckpt_seg = 256;
+  // forward state instead), or -1: the caller has not set it, and a factor that
+  // fills its band runs in the band loops with the whole state, any other with
+  // segments of kDefaultCkptSeg
+  int64_t grad_ckpt_seg = -1;
   BatchTuning batch_tune[4][2];            // [precision][qmc_type]
 };
 
@@ -195,6 +199,7 @@ struct PassArgs {
   void *ck_ring = nullptr;
   double *ck_state = nullptr;
   int64_t ck_seg = 0, ck_N = 0;
+  bool csc = false;  // a banded gradient's passes: in the CSC loop, whatever the factor (grad.cu)
   int64_t io_row0 = 0, io_rows = 0;  // rows of the stored-state arrays (0: all d from row 0)
   int store_p = 0;
 };

@@ -432,8 +432,7 @@ bool dbgz_band_loop(const dbgz_problem *p, bool grad) {
 
 int dbgz_loop_sparse(dbgz_problem *p, const PassArgs &pa, int precision, double *partials, int64_t n_tiles) {
   if (!p->csc_colptr.p) DBGZ_TRY(dbgz_build_csc(p));
-  const bool segments = pa.i_begin != 0 || pa.i_end >= 0 || pa.ck_save || pa.ck_load || pa.store_p;
-  if (!segments && dbgz_band_loop(p, pa.kind == kLoopForwardStore || pa.kind == kLoopAdjoint))
+  if (!pa.csc && dbgz_band_loop(p, pa.kind == kLoopForwardStore || pa.kind == kLoopAdjoint))
     return precision == DBGZ_PREC_FP64 ? dbgz_loop_simt(p, pa, precision, partials, n_tiles)
                                        : dbgz_loop_w32_band(p, pa, partials, n_tiles);
   if (pa.kind == kLoopAdjoint && !p->cscb_colptr.p) {

@@ -117,15 +117,16 @@ int dbgz_release_cached(dbgz_ctx *ctx, uint64_t *freed_bytes);
  * counts run the forward and adjoint passes in chunks of whole 128-sample
  * tiles (default 48 GiB).  No reference counterpart. */
 int dbgz_set_state_budget(dbgz_ctx *ctx, uint64_t bytes);
-/* Gradients of sparse (QMCDataSparse) factors with few entries for their
- * bandwidth, which take the CSC loop, keep, instead of every sample's forward
- * state, a checkpoint every `segment` dimensions (the band's recent values
- * and the recursion state) and recompute each segment's state from its
- * checkpoint just before the adjoint sweeps it (default 256; 0 stores the
- * whole forward state as the dense path does).  The results are the same
- * bits either way.  Factors that fill their band store the whole state within
- * the state budget (faster there), whatever the setting.  No reference
- * counterpart. */
+/* Gradients of sparse (QMCDataSparse) factors keep, instead of every sample's
+ * forward state, a checkpoint every `segment` dimensions (the band's recent
+ * values and the recursion state) and recompute each segment's state from its
+ * checkpoint just before the adjoint sweeps it; 0 stores the whole forward
+ * state.  The results are the same bits for every setting.  All settings run in
+ * the CSC loop.  Without a call, factors with few entries for their bandwidth
+ * take segments of 256, and factors that fill their band run in a faster loop
+ * that stores the whole state within the state budget (d = 4000, bandwidth 64,
+ * 82k samples, FP32: 7.8 ms against 54 with segments of 256, 48 KB a sample
+ * against 8; the results agree to rounding).  No reference counterpart. */
 int dbgz_set_grad_checkpoints(dbgz_ctx *ctx, int64_t segment);
 const char *dbgz_last_error(const dbgz_ctx *ctx);
 

@@ -1,4 +1,8 @@
-"""What a call's route through the loops must keep (needs a B200)."""
+"""What a call's route through the loops must keep: the working precision of the
+conditioning sums, the checkpoint setting of banded gradients (needs a
+B200)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -40,3 +44,65 @@ def test_products_within_a_group_are_fp32(dbgz, n, qmc):
         lw[prec] = D.qmc_pnorm_logw(Q, precision=prec)[0]
         Q.close()
     assert np.abs(lw[L.PREC_FP32_SPLIT_BF16] - lw[L.PREC_FP32_SIMT]).max() <= 4e-6
+
+
+def _sparse_problem(D, n, offsets, seed, sobol, m=600, context=None):
+    # a factor with entries at the given distances above its diagonal
+    rng = np.random.default_rng(seed)
+    U = np.eye(n)
+    for o in offsets:
+        i = np.arange(n - o)
+        U[i, i + o] = rng.uniform(-0.6, 0.6, n - o) / np.sqrt(len(offsets))
+    S = W.correlation(U.T @ U)
+    b = rng.uniform(1.5, 3.5, n)
+    pts = _points("Sobol" if sobol else "Richtmyer", n, rng)
+    return D.QMCDataSparse(S, np.full(n, -np.inf), b, D.QMC_opts(m=m, n_reps=R, max_pts=m, max_abs_err=0.0),
+                           qmc_type="Sobol" if sobol else "Richtmyer", context=context, **pts)
+
+
+def _state(ctx):
+    prof = L.DbgzProfile()
+    L.check(L.lib().dbgz_get_profile(ctx.handle, C.byref(prof)), ctx.handle)
+    return int(prof.grad_state_bytes), int(prof.grad_chunks)
+
+
+# set_grad_checkpoints decides the state of any banded gradient, of factors that
+# fill their band (the first two) too.  Segments inside, equal to and longer than
+# the problem; same bits as the whole state, also with the samples in several
+# chunks.
+@pytest.mark.parametrize("prec", [L.PREC_FP64, L.PREC_FP32_SIMT])
+@pytest.mark.parametrize("n,offsets,seg,sobol", [(150, range(1, 7), 32, False), (300, range(1, 41), 64, True),
+                                                 (420, (1, 300), 5, False), (500, (1, 2, 310), 100, True),
+                                                 (420, (3, 290), 420, False), (300, (250,), 600, True)])
+def test_checkpoint_setting_bounds_the_state(dbgz, prec, n, offsets, seg, sobol):
+    D = dbgz
+    ctx = D.Context(0)
+    try:
+        L.lib().dbgz_set_profiling(ctx.handle, 1)
+        Q = _sparse_problem(D, n, offsets, n + seg, sobol, context=ctx)
+        default = D.qmc_pnorm_grad(Q, precision=prec)
+        ctx.set_grad_checkpoints(0)
+        full = D.qmc_pnorm_grad(Q, precision=prec)
+        state_full, _ = _state(ctx)
+        ctx.set_grad_checkpoints(seg)
+        ck = D.qmc_pnorm_grad(Q, precision=prec)
+        state_ck, chunks = _state(ctx)
+        assert chunks == 1
+        ctx.set_state_budget(1 << 20)  # several chunks of tiles
+        ckc = D.qmc_pnorm_grad(Q, precision=prec)
+        assert _state(ctx)[1] > 1
+        Q.close()
+        if 2 * seg < n and max(offsets) < 64:
+            assert state_ck < state_full
+        assert state_ck != state_full
+        assert ck[0] == full[0] and ck[1] == full[1] and ckc[0] == full[0]
+        assert np.array_equal(ck[3], full[3]) and np.array_equal(ck[4], full[4])
+        for x, y in zip(ckc[3:5], full[3:5]):
+            assert np.linalg.norm(x - y) <= 1e-11 * np.linalg.norm(y)
+        # the default may run in another loop: the bars of the other banded tests
+        tol = 1e-11 if prec == L.PREC_FP64 else 2e-3
+        assert abs(default[0] - full[0]) <= (1e-12 if prec == L.PREC_FP64 else 5e-6 + 2e-5 * full[0])
+        for x, y in zip(default[3:5], full[3:5]):
+            assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y)
+    finally:
+        ctx.close()
