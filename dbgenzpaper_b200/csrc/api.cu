@@ -602,7 +602,7 @@ int dbgz_pnorm(dbgz_problem *p, int precision, double *result, double *err, int6
     if (prof) cudaEventRecord(ctx->ev[2], ctx->stream);
     const bool sparse = p->structure == DBGZ_STRUCTURE_SPARSE;
     const bool tensor = !sparse && (precision == DBGZ_PREC_FP32_TF32 || precision == DBGZ_PREC_FP32_SPLIT_BF16);
-    const bool waits = tensor && dbgz_umma_waits(pa, precision);  // the loop has bounded waits: read its status
+    const bool waits = tensor && dbgz_umma_waits(p, pa, precision);  // the loop has bounded waits: read its status
     if (sparse)
       DBGZ_TRY(dbgz_loop_sparse(p, pa, precision, (double *)p->partials.p, n_tiles));
     else if (tensor)

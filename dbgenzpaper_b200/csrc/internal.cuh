@@ -206,7 +206,7 @@ struct PassArgs {
 int dbgz_loop_simt(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,
                    int64_t n_tiles);
 // whether dbgz_loop_umma runs the kernel with bounded waits (ctx->d_status)
-bool dbgz_umma_waits(const PassArgs &pa, int precision);
+bool dbgz_umma_waits(const dbgz_problem *p, const PassArgs &pa, int precision);
 int dbgz_loop_umma(dbgz_problem *p, const PassArgs &pa, int precision, double *partials,
                    int64_t n_tiles);
 // The warp-level FP32 loop: dense split-BF16, and banded (p->bandwidth).

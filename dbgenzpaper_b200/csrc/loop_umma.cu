@@ -1092,20 +1092,36 @@ void dbgz_umma_batch_free(UmmaBatchPlan *B) {
   delete B;
 }
 
-bool dbgz_umma_waits(const PassArgs &pa, int precision) {
-  // the warp-level loop's products run on mma.sync and grow with d; this one's
-  // do not show, but its steps have half the warps to hide their latency.
-  // Measured (split BF16, 5.2e5 samples, this loop / that one): forward 1.08
-  // to 1.13 at d = 300, 0.99 to 1.01 at 400, 0.89 to 0.93 at 450, 0.84 to 0.88
-  // at 500; with gradient, lattice 1.05 at 400, 0.98 at 450, Sobol 1.16 at 450,
-  // 1.03 to 1.05 at 560, 0.98 to 1.01 at 620
-  const bool plain = pa.kind == kLoopForward || pa.kind == kLoopLogWeight;
-  const int64_t warp_loop_max_d = plain ? 400 : pa.qmc_type == DBGZ_QMC_SOBOL ? 600 : 430;
-  return precision != DBGZ_PREC_FP32_SPLIT_BF16 || pa.d > warp_loop_max_d;
+bool dbgz_umma_waits(const dbgz_problem *p, const PassArgs &pa, int precision) {
+  // The warp-level loop's products run on mma.sync and grow with d; this one's
+  // do not show, but its steps have half the warps to hide their latency.  That
+  // one holds 4 tiles per SM at a time, this one 2, so the line depends on the
+  // pass's tiles per SM (t; of the whole pass, so that a gradient's sample
+  // chunks all take one loop).  Times of that loop over this one's, split BF16:
+  //                       t <= 2           4 < t <= 6       other t
+  //   forward          d = 225 0.97-1.00  300 0.93-1.06   400 0.85-1.02
+  //                        257 0.99-1.09  330 0.99-1.11   450 0.93-1.10
+  //                        400 1.16-1.24  365 1.03-1.15
+  //   gradient,            150 0.97-1.03  300 0.97-1.03   430 0.93-1.02
+  //   lattice              170 1.00-1.05  350 1.03-1.10   500 1.01-1.12
+  //                        430 1.29-1.30  430 1.12-1.17
+  //   gradient, Sobol      200 0.95-1.03  430 1.00-1.01   560 0.91-1.00
+  //                        257 1.05-1.08  500 1.07-1.09   600 0.95-1.07
+  //                        430 1.19-1.24
+  // (With the last column's lines for all t, small forward passes at d = 300..400
+  // were 1.1 times, gradients 1.2 times as slow as when this loop took them all.)
+  if (precision != DBGZ_PREC_FP32_SPLIT_BF16) return true;
+  const bool plain = pa.kind == kLoopForward || pa.kind == kLoopLogWeight, sobol = pa.qmc_type == DBGZ_QMC_SOBOL;
+  const int64_t tiles = (pa.m + TS - 1) / TS * pa.n_reps, sms = p->ctx->num_sms;
+  int64_t max_d;
+  if (tiles <= 2 * sms) max_d = plain ? 257 : sobol ? 200 : 170;
+  else if (tiles > 4 * sms && tiles <= 6 * sms) max_d = plain ? 300 : sobol ? 430 : 300;
+  else max_d = plain ? 400 : sobol ? 560 : 430;
+  return pa.d > max_d;
 }
 
 int dbgz_loop_umma(dbgz_problem *p, const PassArgs &pa, int precision, double *partials, int64_t n_tiles) {
-  if (!dbgz_umma_waits(pa, precision)) return dbgz_loop_w32(p, pa, partials, n_tiles);
+  if (!dbgz_umma_waits(p, pa, precision)) return dbgz_loop_w32(p, pa, partials, n_tiles);
   if (precision == DBGZ_PREC_FP32_SPLIT_BF16)
     return launch_umma<DBGZ_PREC_FP32_SPLIT_BF16>(p, pa, partials, n_tiles);
   return launch_umma<DBGZ_PREC_FP32_TF32>(p, pa, partials, n_tiles);

@@ -1,6 +1,6 @@
 """What a call's route through the loops must keep: the working precision of the
-conditioning sums, the checkpoint setting of banded gradients (needs a
-B200)."""
+conditioning sums, the checkpoint setting of banded gradients, and the
+results either side of the loop-choice lines (needs a B200)."""
 import ctypes as C
 
 import numpy as np
@@ -104,5 +104,55 @@ def test_checkpoint_setting_bounds_the_state(dbgz, prec, n, offsets, seg, sobol)
         assert abs(default[0] - full[0]) <= (1e-12 if prec == L.PREC_FP64 else 5e-6 + 2e-5 * full[0])
         for x, y in zip(default[3:5], full[3:5]):
             assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y)
+    finally:
+        ctx.close()
+
+
+# either side of the lines between the warp-level and the tcgen05 loop, which
+# depend on the pass's tiles of 128 samples per SM (148): up to 2, more than 4 and up
+# to 6, and others.  Bars of the split-BF16 mode.
+@pytest.mark.parametrize("qmc,n,tiles,grad", [
+    ("Richtmyer", 257, 294, False), ("Sobol", 258, 294, False), ("Sobol", 300, 600, False),
+    ("Richtmyer", 301, 600, False), ("Richtmyer", 401, 300, False), ("Richtmyer", 170, 6, True),
+    ("Richtmyer", 171, 294, True), ("Sobol", 200, 294, True), ("Sobol", 201, 6, True), ("Richtmyer", 301, 600, True),
+    ("Sobol", 431, 600, True), ("Sobol", 560, 300, True), ("Sobol", 561, 300, True)])
+def test_split_bf16_at_the_lines_by_tiles(dbgz, qmc, n, tiles, grad):
+    D = dbgz
+    rng = np.random.default_rng(n)
+    S = W.correlation(W.rand_spd(n, 1.0, rng))
+    a, b = W.bounds_quarter(S)
+    pts = _points(qmc, n, rng)
+    m = 128 * tiles // R - 5
+    out = {}
+    for prec in (L.PREC_FP64, L.PREC_FP32_SPLIT_BF16):
+        Q = D.QMCData(S, a, b, D.QMC_opts(m=m, n_reps=R, max_pts=m, max_abs_err=0.0), qmc_type=qmc, **pts)
+        out[prec] = D.qmc_pnorm_grad(Q, precision=prec) if grad else D.qmc_pnorm(Q, precision=prec)
+        Q.close()
+    r64, r = out[L.PREC_FP64], out[L.PREC_FP32_SPLIT_BF16]
+    assert abs(r[0] - r64[0]) <= 5e-6 + 2e-5 * abs(r64[0])
+    for x, y in zip(r[3:6], r64[3:6]) if grad else ():
+        assert np.linalg.norm(x - y) <= 2e-3 * np.linalg.norm(y)
+
+
+# the line looks at the whole pass: sample chunks small enough for another one
+# give the same estimate to the last bit
+def test_sample_chunks_take_the_pass_s_loop(dbgz):
+    D = dbgz
+    n, m = 350, 12800  # 300 tiles
+    rng = np.random.default_rng(n)
+    S = W.correlation(W.rand_spd(n, 1.0, rng))
+    a, b = W.bounds_quarter(S)
+    ctx = D.Context(0)
+    try:
+        Q = D.QMCData(S, a, b, D.QMC_opts(m=m, n_reps=R, max_pts=m, max_abs_err=0.0), context=ctx,
+                      **_points("Richtmyer", n, rng))
+        one = D.qmc_pnorm_grad(Q, precision=L.PREC_FP32_SPLIT_BF16)
+        ctx.set_state_budget(100 << 20)
+        two = D.qmc_pnorm_grad(Q, precision=L.PREC_FP32_SPLIT_BF16)
+        chunks = _state(ctx)[1]
+        Q.close()
+        assert chunks > 1 and one[0] == two[0] and one[1] == two[1]
+        for x, y in zip(two[3:6], one[3:6]):
+            assert np.linalg.norm(x - y) <= 1e-6 * np.linalg.norm(y)
     finally:
         ctx.close()
