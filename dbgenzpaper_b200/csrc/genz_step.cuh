@@ -194,18 +194,6 @@ __device__ __forceinline__ void sobol_tent_f32(uint32_t X, int L, float &w, floa
   w1 = __uint2float_rn(half - dd) * sc;
 }
 
-// The same integer by one thread alone (loop over the set bits).
-__device__ __forceinline__ uint32_t sobol_int(const uint32_t *Vl, uint64_t idx) {
-  uint32_t g = (uint32_t)(idx ^ (idx >> 1));
-  uint32_t x = 0;
-  while (g) {
-    int k = __ffs(g) - 1;
-    x ^= __ldg(Vl + k);
-    g &= g - 1;
-  }
-  return x;
-}
-
 // ---------------------------------------------------------------- FP64 ---
 struct StepFp64 {
   using Tent = double;

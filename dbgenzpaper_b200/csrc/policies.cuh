@@ -231,18 +231,9 @@ struct Forward {
   __device__ __forceinline__ T emit_k_at(const Staged<T> &sg, int li, int64_t l, int, Point w) {
     return emit_next(sg, li, l, w);
   }
-  __device__ __forceinline__ T emit_k_fast_at(const Staged<T> &sg, int li, int64_t l, int, Point w) {
-    return emit_next(sg, li, l, w);
-  }
   // chunked form (8 steps whose per-sample inputs may be loaded up front)
   __device__ __forceinline__ void chunk_begin(int64_t, int) {}
   __device__ __forceinline__ void chunk_end(int64_t, int) {}
-  __device__ __forceinline__ T emit_k(const Staged<T> &sg, int li, int64_t l, int, uint32_t xs) {
-    return emit(sg, li, l, xs);
-  }
-  __device__ __forceinline__ T emit_k_fast(const Staged<T> &sg, int li, int64_t l, int k, uint32_t xs) {
-    return emit_k(sg, li, l, k, xs);
-  }
   __device__ __forceinline__ void consume(const Staged<T> &sg, T s, int li, int64_t l) {
     const auto tg = sg.tg[li];
     st.cdf(s, tg.a, tg.b, tg.inv_u, cdf_form);
@@ -313,7 +304,7 @@ template <typename T, int GEN>
 struct Adjoint {
   static constexpr bool kPlain = false;
   static constexpr bool kDeferTail = false;
-  // the loop may run a chunk with emit_k_fast (no per-step vote) and redo it
+  // the loop runs a chunk with emit_k_fast_at (no per-step vote) and redoes it
   // with emit_k when some lane's FP32 terms left FP32 range (bad)
   static constexpr bool kChunkRedo = sizeof(T) == 4;
   bool bad;
@@ -650,11 +641,6 @@ struct Adjoint {
   // any case, `bad` set where they are not finite; the loop then redoes the
   // chunk with emit_k from the chunk's saved state, which gives exactly what
   // emit_k alone would have given
-  __device__ __forceinline__ T emit_k_fast(const Staged<T> &sg, int li, int64_t l, int kk, uint32_t xs) {
-    const int64_t t = d - 1 - l;
-    const bool has_u = t <= d - 2;
-    return emit_k_fast_at(sg, li, l, kk, has_u ? point_w32(sg, li, t, xs, gen.sobol_staged != 0) : 0.0f);
-  }
   __device__ __forceinline__ T emit_k_fast_at(const Staged<T> &sg, int li, int64_t l, int kk, Point w) {
     const int64_t t = d - 1 - l;
     const bool has_u = t <= d - 2;
