@@ -412,12 +412,12 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
             if (!decltype(checked)::value || k < nv) {
               const int64_t l = l0 + k;
               if (k + kAhead < 8) pt[k + kAhead] = point(k + kAhead);
-              if constexpr (decltype(fast)::value)
-                y = pl.emit_k_fast_at(st.sg, li, l, k, pt[k]);
-              else if constexpr (chunk_redo<Policy>::value)
-                y = pl.emit_k(st.sg, li, l, k, sob_x(k));
-              else
+              if constexpr (Policy::kDeferTail)
                 y = pl.emit_k_at(st.sg, li, l, k, pt[k]);
+              else if constexpr (decltype(fast)::value)
+                y = pl.emit_k_fast_at(st.sg, li, l, k, pt[k]);
+              else
+                y = pl.emit_k(st.sg, li, l, k, sob_x(k));
               const float4 *ur = reinterpret_cast<const float4 *>(st.tri + tri_at(q, q) + k * CH);
               const float4 u0 = ur[0], u1 = ur[1];
               const float uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
