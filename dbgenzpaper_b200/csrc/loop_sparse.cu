@@ -86,11 +86,13 @@ __global__ void __launch_bounds__(TS) k_genz_sparse(const SparseParams<T> P) {
   // layout: [staged entries x cap][colptr of block (CB+1)][ring].  The staged
   // entries are (slot offset, value) pairs, read by one load each, or -- in
   // the FP32 forward pass without stored state -- two arrays of offsets and
-  // values (measured on the banded d = 10^4, bandwidth 64, 2^18 x 10 Sobol
-  // workload: pairs 947 ms, arrays 863 ms for that pass; pairs
-  // faster for the FP64 pass, 1552 against 1588 ms, and the FP32 gradient,
-  // 1744 against 2002 ms)
+  // values.  Pairs / arrays, d = 2000, 2^13 x 10 Sobol points: that pass 3.12 / 2.94
+  // ms with one entry a column at distance 400, 1.52 / 1.35 at distance 1, 1.62 /
+  // 1.47 with three; the FP32 gradient 9.10 / 9.36, 4.16 / 4.29, 4.37 / 4.50, and
+  // 16.9 / 19.5 with 64 (on lattice points arrays gain 3 to 4%, not told apart).
+  // The FP64 dot reads pairs only.
   constexpr bool kPairs = sizeof(T) == 8 || !Policy::kPlain;
+  static_assert(sizeof(T) != 8 || kPairs, "the FP64 dot reads the pairs");
   SlotVal<T> *sent = reinterpret_cast<SlotVal<T> *>(smem_raw);
   int32_t *soff = reinterpret_cast<int32_t *>(smem_raw);
   T *sval = reinterpret_cast<T *>(smem_raw + ((sizeof(int32_t) * P.max_block_nnz + 15) & ~size_t(15)));
@@ -319,11 +321,10 @@ static int launch_sparse(dbgz_problem *p, const PassArgs &pa, double *partials, 
   P.gen.gen_base = pa.gen_base;
   P.gen.gen_base_dev = pa.gen_base_dev;
   P.gen.sobol_first = pa.sobol_first;
-  // staged Sobol integers; not in the FP32 pass that keeps its state (measured
-  // on the banded d = 10^4, bandwidth 64 workload at 2^14 x 10 Sobol points: the
-  // gradient call 125.1 ms without, 136.9 ms with them)
-  P.gen.sobol_staged =
-      pa.qmc_type == DBGZ_QMC_SOBOL && !(sizeof(T) == 4 && pa.kind == kLoopForwardStore);
+  // (FP32 gradient without / with them in the pass that keeps the state, d = 2000,
+  // 2^13 x 10 points: 10.1 / 9.1 ms with one entry a column at distance 400, 5.0 /
+  // 4.4 with three, 18.1 / 16.9 with 64)
+  P.gen.sobol_staged = pa.qmc_type == DBGZ_QMC_SOBOL;
   P.gen.q = (const double *)p->q.p;
   P.gen.shift64 = (const double *)p->shifts.p;
   P.gen.shift32 = (const float *)p->shifts32.p;
