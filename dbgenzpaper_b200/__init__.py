@@ -271,7 +271,8 @@ class QMCData:
 
 class QMCDataSparse(QMCData):
     """QMCDataSparse (src/qmc.jl:225-282): classic (unpivoted) Cholesky and
-    the loop over the strict-upper CSC of U.  Default generator: Sobol."""
+    the loop over the band of U, or over its strict-upper CSC where it has few
+    entries for its bandwidth.  Default generator: Sobol."""
 
     _structure = L.STRUCTURE_SPARSE
     _default_type = "Sobol"

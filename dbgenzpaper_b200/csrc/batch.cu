@@ -14,11 +14,13 @@
 //      (16 warps an SM hide the step's latency; 20.5 against 38.4 ms of the
 //      tcgen05 loop at 256 problems of d = 16..256, 6.6e4 samples each), TF32
 //      the tcgen05 loop for d <= 257, both with the SIMT kernel for larger d.
-//      Persistent CTAs take work items (a run of tiles of one problem, about
-//      the same number of tile-dimensions per item, largest problems first)
-//      from a global counter;
-//   3. k_finalize_batch: per (problem, shift) sums of the tile sums in tile
-//      order (the one-problem finalize, so results agree bit for bit).
+//      Without a tuning table the tensor precisions start at d = 25, smaller
+//      problems run in the SIMT kernel (kDefaultTensorMinD below).  Persistent
+//      CTAs take work items (a tile, or a run of tiles of one problem of about
+//      the same number of tile-dimensions, largest problems first) from a global
+//      counter;
+//   3. k_finalize_batch: the tile sums of each (problem, shift) by one warp, as
+//      the one-problem finalize adds them.
 // Limits: 2 <= d <= min(512, chol_block_size2) (one Cholesky panel), one
 // pass (n_pts = m), erf-form CDF.
 #include <algorithm>
@@ -207,10 +209,13 @@ int batch_grid(dbgz_ctx *ctx, int GEN, int64_t *grid) {
 }
 
 
-// Default choices before (or without) dbgz_batch_autotune: the tensor-core
-// loop from d = 25 in the tensor-core precisions (below that the SIMT loop
-// is as fast or faster: measured on B200, 2^14 points x 8 shifts), SIMT work
-// items of about 1024 tile-dimensions.
+// Default choices before (or without) dbgz_batch_autotune, which dbgenz.h
+// states: the tensor-core precisions' own loop from d = 25, SIMT work items of
+// about 1024 tile-dimensions.  At 25 the tcgen05 loop, which both modes ran in
+// when the line was drawn and TF32 still does, passed the SIMT loop.  Split
+// BF16's warp-level loop is faster at every d (a run of 256 problems of one d,
+// 2^13 Sobol points x 8, SIMT / it: d = 8 3.2 / 1.0 ms, 16 4.6 / 1.8, 24 6.8 / 2.5;
+// d = 16..256 mixed 21.1 / 20.6), so its tuned table starts at d = 2.
 constexpr int64_t kDefaultItemDims = 1024;
 constexpr int64_t kDefaultTensorMinD = 25;
 

@@ -14,10 +14,13 @@
 // concurrently (one chain per output element), never from splitting a
 // chain.
 //
-// Layout: M is d x d column-major in HBM (8 MB at d = 1000, L2 resident);
-// a sequential pivot step runs in one CTA (latency-bound: scores, argmin,
-// swaps, row update), the trailing Schur updates and triangular solves run
-// on the whole GPU.
+// Layout: M is d x d column-major in HBM (8 MB at d = 1000, L2 resident).
+// The Genz order's pivots of a block run in a cluster of CTAs, 64 candidates
+// each (panels of at most 512 candidates, blocks of at most 64 pivots;
+// latency-bound: scores, argmin, row update), and its swaps reach M as one
+// permutation by the whole GPU; larger panels or blocks, and the diagonal
+// pivots of cholesky_rowmax!, run in one CTA.  The trailing Schur updates and
+// triangular solves run on the whole GPU.
 #include "internal.cuh"
 #include "detmath.h"
 #include "chol_dev.cuh"

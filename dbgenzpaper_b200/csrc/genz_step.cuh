@@ -14,9 +14,12 @@
 //   p  *= dc
 //
 // Two numerics are provided:
-//  * StepFp64: the reference's Float64 arithmetic (erf form or erfc form of
-//    the CDF, the clamp to [-9, 9] in erf units, the same fma pattern), with
-//    the table-based erf and inverse erf of normal64.cuh.
+//  * StepFp64: the reference's Float64 expressions (erf form or erfc form of
+//    the CDF, the clamp to [-9, 9] in erf units, the same fma pattern).  In the
+//    erf form erf and inverse erf are normal64.cuh's, by a table: erf to an
+//    absolute 1.2e-16 (not relative: only 1 + erf and its differences are used;
+//    the CDF's largest error is 1.1e-16, with CUDA's erf 0.9e-16), the inverse an FP32
+//    start and one third-order correction.
 //  * StepFp32: FP32 arithmetic kept close to the FP64 result where the
 //    reference's Float32 loop loses digits (tail masses from normal32.cuh,
 //    relative error < 3e-6 where they are above 1e-10; Phi^-1 of the smaller

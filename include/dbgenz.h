@@ -51,7 +51,9 @@ typedef enum dbgz_qmc_type {
 
 typedef enum dbgz_structure {
   DBGZ_STRUCTURE_DENSE = 0,  /* QMCData:       cholesky_genz!, dense loop  */
-  DBGZ_STRUCTURE_SPARSE = 1  /* QMCDataSparse: cholesky_classic!, CSC loop */
+  DBGZ_STRUCTURE_SPARSE = 1  /* QMCDataSparse: cholesky_classic!, loops over
+                                the factor's band, or its CSC entries where
+                                they are few for the bandwidth */
 } dbgz_structure;
 
 typedef enum dbgz_cdf_form {
@@ -67,10 +69,16 @@ typedef enum dbgz_precision {
    * with TF32 operands accumulated in FP32. */
   DBGZ_PREC_FP32_TF32 = 1,
   /* As above with the contraction as three BF16 products (hi*hi + hi*lo +
-   * lo*hi of the split operands) accumulated in FP32. */
+   * lo*hi of the split operands) accumulated in FP32, on tcgen05 or, for
+   * smaller dimensions, warp-level tensor instructions; within 32 consecutive
+   * variables, FP32 FMAs. */
   DBGZ_PREC_FP32_SPLIT_BF16 = 2,
   /* FP32 numerics of the two modes above with the contraction on CUDA
-   * cores (no tensor cores); an ablation of the tensor-core choice. */
+   * cores (no tensor cores); an ablation of the tensor-core choice.  Sparse
+   * (banded) problems run alike in all FP32 modes: FP32 FMAs within 32
+   * consecutive variables and, from further away in the band, six products of
+   * three BF16 parts (FP32's 24 bits) accumulated in FP32 on warp-level tensor
+   * instructions; FP32 FMAs throughout in the CSC loop. */
   DBGZ_PREC_FP32_SIMT = 3
 } dbgz_precision;
 
@@ -309,11 +317,11 @@ int dbgz_pnorm_pass_noalloc(int64_t d, const double *U, const double *a, const d
  * bounds one after another, shifts (Richtmyer) or ushifts (Sobol) the
  * (d_k - 1) x n_reps blocks one after another; sobol_dirnums is one table
  * for the largest d - 1 (NULL: the library's own) and sobol_first the
- * first Sobol index (as in dbgz_prepare).  precision: DBGZ_PREC_FP64 (FP64
- * SIMT loop), DBGZ_PREC_FP32_SIMT, or a tensor-core mode: problems with
- * d - 1 <= 256 then run in the batched tcgen05 loop and the others in the
- * FP32 SIMT loop, as the context's tuning table (dbgz_batch_autotune) or the
- * default (tensor-core loop from d = 25) says.  Inputs are checked on the
+ * first Sobol index (as in dbgz_prepare).  precision: DBGZ_PREC_FP64,
+ * DBGZ_PREC_FP32_SIMT, or a tensor-core mode: problems with d - 1 <= 256 then
+ * run in the mode's batched loop (TF32: tcgen05, split BF16: warp-level tensor
+ * instructions) and the others in the FP32 SIMT loop, as the context's tuning
+ * table (dbgz_batch_autotune) or the default (the mode's loop from d = 25) says.  Inputs are checked on the
  * device (non-finite Sigma, NaN bounds or a > b: DBGZ_ERR_NONFINITE_INPUT;
  * Richtmyer shifts outside [0,1]: DBGZ_ERR_INVALID_ARGUMENT).  results
  * and errs (may be NULL) receive P and 3 SEM per problem, ranks (may be
