@@ -26,8 +26,8 @@
 //     (With the earlier chunks as BF16 parts too, rms error of the shifts' means
 //     against FP64, split BF16: 2.1e-7 at d = 20, 1.9e-7 at 33, geometric mean
 //     over d = 8..380 4.3e-7; as FP32 0.8e-7, 0.7e-7, 3.4e-7.  Time with the parts and now: batch of
-//     256 problems 20.50 / 20.45 ms, banded d = 4000 pass 10.46 / 10.64, gradient
-//     7.81 / 7.78.)
+//     256 problems 20.50 / 20.27 ms, banded d = 4000 pass 10.46 / 10.52, gradient
+//     7.81 / 7.70.)
 // The tensor unit truncates as it accumulates, so the products of high parts
 // have accumulators of their own: their sum is truncated once per 16 y-indices,
 // not once per product (relative error of P, batch of d 16..256: 4.7e-6 with
@@ -365,28 +365,29 @@ __device__ __forceinline__ void tile(const Prob &P, const pol::GradIO<float> &io
 #pragma unroll
           for (int t = 0; t < 8; ++t) s[t] = 0.f;
         }
-        // the group's earlier chunks (paired FMAs: half the issue slots, banded
-        // pass 10.70 -> 10.64 ms)
+        // the group's earlier chunks (paired FMAs: half the issue slots; a copy of the
+        // code per chunk: banded pass 10.66 -> 10.52 ms, batch 20.44 -> 20.27)
         if (q > 0) {
           uint64_t s2[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) s2[t] = pack2(s[2 * t], s[2 * t + 1]);
-#pragma unroll 1
-          for (int c = 0; c < q; ++c) {
-            float ye[8];
-            lds4(ye, Sa + c * SM::SLOT + s_lo);
-            lds4(ye + 4, Sa + c * SM::SLOT + s_hi);
-            const ulonglong2 *ur = reinterpret_cast<const ulonglong2 *>(st.tri + tri_at(q, c));
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const uint64_t y2 = pack2(ye[k], ye[k]);
-              const ulonglong2 u0 = ur[2 * k], u1 = ur[2 * k + 1];
-              fma2(s2[0], y2, u0.x);
-              fma2(s2[1], y2, u0.y);
-              fma2(s2[2], y2, u1.x);
-              fma2(s2[3], y2, u1.y);
+          for (int c = 0; c < G / CH - 1; ++c)
+            if (c < q) {
+              float ye[8];
+              lds4(ye, Sa + c * SM::SLOT + s_lo);
+              lds4(ye + 4, Sa + c * SM::SLOT + s_hi);
+              const ulonglong2 *ur = reinterpret_cast<const ulonglong2 *>(st.tri + tri_at(q, c));
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const uint64_t y2 = pack2(ye[k], ye[k]);
+                const ulonglong2 u0 = ur[2 * k], u1 = ur[2 * k + 1];
+                fma2(s2[0], y2, u0.x);
+                fma2(s2[1], y2, u0.y);
+                fma2(s2[2], y2, u1.x);
+                fma2(s2[3], y2, u1.y);
+              }
             }
-          }
 #pragma unroll
           for (int t = 0; t < 4; ++t) unpack2(s2[t], s[2 * t], s[2 * t + 1]);
         }
