@@ -11,7 +11,7 @@
 //      copy of U and the first dimension's CDF;
 //   2. the integration, by precision: FP64 f64::k_genz_f64_batch, FP32 SIMT
 //      simt::k_genz_simt_batch, split BF16 w32::k_genz_w32_batch for d <= 257
-//      (16 warps an SM hide the step's latency; 20.5 against 38.4 ms of the
+//      (16 warps an SM hide the step's latency; 20.3 against 38.4 ms of the
 //      tcgen05 loop at 256 problems of d = 16..256, 6.6e4 samples each), TF32
 //      the tcgen05 loop for d <= 257, both with the SIMT kernel for larger d.
 //      Without a tuning table the tensor precisions start at d = 25, smaller

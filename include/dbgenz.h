@@ -133,7 +133,7 @@ int dbgz_set_state_budget(dbgz_ctx *ctx, uint64_t bytes);
  * the CSC loop.  Without a call, factors with few entries for their bandwidth
  * take segments of 256, and factors that fill their band run in a faster loop
  * that stores the whole state within the state budget (d = 4000, bandwidth 64,
- * 82k samples, FP32: 7.8 ms against 52 with segments of 256, 48 KB a sample
+ * 82k samples, FP32: 7.7 ms against 52 with segments of 256, 48 KB a sample
  * against 8; the results agree to rounding).  No reference counterpart. */
 int dbgz_set_grad_checkpoints(dbgz_ctx *ctx, int64_t segment);
 const char *dbgz_last_error(const dbgz_ctx *ctx);
