@@ -10,7 +10,7 @@
 // 16 warps fit on an SM, and mma.m16n8k16 (8 cycles of a scheduler, in the
 // shadow of the other warps' steps) feeds them without a round trip to
 // another warp.  The larger the dimension, the more the contraction weighs:
-// mma.sync runs at about a quarter of tcgen05's rate (dbgz_loop_umma has
+// mma.sync runs at about a quarter of tcgen05's rate (dbgz_umma_waits has
 // the crossover).
 //
 // One CTA = one tile of 128 samples = four warps of 32.  y-indices run in
